@@ -373,16 +373,16 @@ void shg_keys_mt19937_64(uint64_t seed, uint64_t n, uint64_t *out);
 /* n distinct uint64 keys out[j] = remix(seed ^ (j * 0x9E3779B97F4A7C15)) (Stafford Mix13, a bijection),
  * filled by up to `threads` host threads: the per-request key sets of the serving stream. */
 void shg_keys_mix(uint64_t seed, uint64_t n, uint64_t *out, int threads);
-/* Integer-pipe peak of the split-search arithmetic (remix + 16-bit part thresholds, operands in
- * registers) on `device`, in evaluations per second: the roofline denominator of the searches. */
+/* Integer-pipe peak of the split search's quarter loop (staged keys in shared memory, every lane busy)
+ * on `device`, in evaluations per second: the roofline denominator of the searches. */
 int shg_int_peak(int device, uint64_t iters, double *evals_per_s, double *ms);
-/* Same for the inner loop of one search: 0 = split quarter-split moments (as shg_int_peak),
+/* Same for the inner loop of one search: 0 = quarter split (as shg_int_peak),
  * 1 = original leaf coverage (remix, two fastrange32 cells, half masks), 2 = bipartite raw seeds
  * (remix, fastrange64, mask), 3 / 4 / 5 = split compare-and-count against 1 / 2 / 3 part
  * thresholds (fanout-2 and uneven split nodes), 6 = bipartite candidate-scan mask pairs,
  * 7 = bipartite isolated-key pair filter, 8 = bipartite pseudoforest edges (union-find),
- * 9 / 10 / 11 / 12 = kinds 0 / 3 / 4 / 5 with the split kernel's pipe-split arithmetic
- * (tuning parameter split_arith 1), 13 / 14 / 15 = kinds 6 / 7 / 8 for bipartite leaves of more
+ * 9 / 10 / 11 / 12 = kinds 0 / 3 / 4 / 5 again (tuning parameter split_arith 1 runs the same
+ * loops), 13 / 14 / 15 = kinds 6 / 7 / 8 for bipartite leaves of more
  * than 64 keys (64-bit masks, 100-edge tests), 16 / 17 / 18 / 19 = kinds 0 / 3 / 4 / 5 under
  * SIMDShockHash's split hash (SIMDShockHash.hpp:762-766), 20 = kind 13 with the other form of the
  * mask test ((a | t) == full instead of (~t & ~a) == 0; the faster of 13 and 20 bounds the scan). */
@@ -391,7 +391,7 @@ int shg_int_peak_kind(int device, int kind, uint64_t iters, double *evals_per_s,
 /* Work counts of the engine's last RecSplit build beyond shg_result.work (measurement utility, no
  * counterpart in the reference; the weights of the search stages' roofline denominators). Writes
  * min(n, 13) values: [0..2] useful split evaluations of nodes comparing 1, 2 or 3 part thresholds
- * (fanout-2 and uneven nodes), [3] of quarter splits (moment sums), [4] split level launches,
+ * (fanout-2 and uneven nodes), [3] of quarter splits, [4] split level launches,
  * [5] bipartite leaves' candidate-scan mask-pair tests (for each raw seed, the earlier raw seeds
  * it is paired with), [6..7] zero; [8..12] the last ShockHash2Flat build's leaf search: hash
  * evaluations, candidate pairs, pairs left by the isolated-key filter, union-find edges,
@@ -402,8 +402,8 @@ shg_status shg_engine_last_work(const shg_engine *e, uint64_t *out, int n);
  * change speed only, never a result). variant is an shg_variant (SHG_SHOCKHASH_ROTATION shares
  * SHG_SHOCKHASH's entry) or 4 for ShockHash2Flat<k> with leaf_size = k. Names and ranges:
  *   split_seeds_per_lane 1, 2, 4; split_threads 128, 256, 512; split_round_div 1..64 (a round of
- *   seeds aims at 1/round_div of a split node's expected trials); split_arith 0, 1 (1: remix's
- *   shifts partly as multiply-highs, moving work from the integer to the multiply pipe);
+ *   seeds aims at 1/round_div of a split node's expected trials); split_arith 0, 1 (the same
+ *   arithmetic; kept for tables that set it);
  *   leaf_blocks_per_sm 0..16 (0 =
  *   as many as shared memory allows); leaf_min_blocks 4, 6, 8 (bipartite leaves up to 64 keys:
  *   register bound); sh1_seeds_per_lane 1, 2 (original leaves); queue_lag_rounds 0..64 (work-queue

@@ -235,7 +235,7 @@ def device_memory(device=0):
 
 def int_peak(device=0, iters=1 << 16, kind=0):
     """Measured evaluations/s of a search's inner-loop arithmetic with no memory traffic
-    (kind 0 = split quarter moments, 1 = original leaf coverage, 2 = bipartite raw seeds,
+    (kind 0 = quarter split, 1 = original leaf coverage, 2 = bipartite raw seeds,
     3 / 4 / 5 = split compare-and-count with 1 / 2 / 3 part thresholds)."""
     e, ms = ctypes.c_double(), ctypes.c_double()
     _check(lib().shg_int_peak_kind(device, kind, iters, ctypes.byref(e), ctypes.byref(ms)))
@@ -251,22 +251,12 @@ TUNING_FLAT = 4
 
 
 def split_peaks(device=0, iters=1 << 15, detail=None, simd=False):
-    """Measured evaluations/s of each split inner loop, keyed as SPLIT_KINDS: the faster of the two
-    arithmetic forms the split kernel can run (split_arith 0 and 1), so the ceiling holds for both.
-    `detail`, a dict, receives both forms' rates per kind. `simd`: the loops under SIMDShockHash's
-    split hash, which has one form."""
-    if simd:
-        out = {name: int_peak(device, iters, k)[0] for name, k in zip(SPLIT_KINDS, (17, 18, 19, 16))}
-        if detail is not None:
-            detail.update({name: {"simd": v} for name, v in out.items()})
-        return out
-    plain, pipes = (3, 4, 5, 0), (10, 11, 12, 9)
-    out = {}
-    for name, a, b in zip(SPLIT_KINDS, plain, pipes):
-        ra, rb = int_peak(device, iters, a)[0], int_peak(device, iters, b)[0]
-        out[name] = max(ra, rb)
-        if detail is not None:
-            detail[name] = {"arith_0": ra, "arith_1": rb}
+    """Measured evaluations/s of each split inner loop, keyed as SPLIT_KINDS. `detail`, a dict, receives
+    the same per kind under the name of the split hash. `simd`: the loops under SIMDShockHash's split hash."""
+    kinds = (17, 18, 19, 16) if simd else (3, 4, 5, 0)
+    out = {name: int_peak(device, iters, k)[0] for name, k in zip(SPLIT_KINDS, kinds)}
+    if detail is not None:
+        detail.update({name: {"simd" if simd else "remix": v} for name, v in out.items()})
     return out
 
 

@@ -1,10 +1,10 @@
 // Measurement utilities (not part of the reference's interface):
 //  * the seeded key generators the benchmark configurations name (std::mt19937_64), shared by the
 //    CPU and GPU runs so both build from the same keys;
-//  * the integer-pipe peaks of the searches: the arithmetic of each search kernel's dominant inner
-//    loop (split: remix to 16 bits, quarter-split part, moment sums; original leaf: remix, two
-//    fastrange32 cells, half masks; bipartite leaf: remix, fastrange64, mask), two seeds per lane,
-//    on register-resident operands with no memory traffic. Their evaluations per second are the
+//  * the integer-pipe peaks of the searches: each search kernel's dominant inner loop (split: the
+//    counting loops over staged keys; original leaf: remix, two fastrange32 cells, half masks;
+//    bipartite leaf: remix, fastrange64, mask), two seeds per lane, on operands in registers and
+//    shared memory. Their evaluations per second are the
 //    denominators of the search kernels' roofline fractions.
 #include <algorithm>
 #include <cstdint>
@@ -15,108 +15,42 @@
 #include "shg.h"
 #include "shg_common.cuh"
 #include "shg_internal.h"
+#include "shg_split.cuh"
 
 namespace {
 
 constexpr int kPeakThreads = 256;
 
-// The arithmetic of the split kernel's dominant loop (quarter splits): remix to 16 bits, part
-// p = r >> 14, moments sum p, sum p^2, sum p^3; two seeds per key pair.
-__global__ void __launch_bounds__(kPeakThreads) k_int_peak(uint64_t iters, uint32_t T0, uint32_t T1, uint32_t T2,
-                                                           unsigned long long *sink) {
+// The split kernel's own counting loops (shg_split.cuh) alone: 256 staged keys in shared memory,
+// lanes on consecutive seeds, two seeds per lane; the quarter split (NT = 4) or compare-and-count against
+// NT thresholds, under remix or SIMDShockHash's split hash. `iters` key reads per thread, rounded up to
+// whole rounds (the caller counts the rounded number).
+constexpr uint32_t kPeakKeys = 256;
+template <int NT, bool SIMD>
+__global__ void __launch_bounds__(kPeakThreads) k_int_peak_split(uint64_t iters, uint32_t T0, uint32_t T1, uint32_t T2,
+                                                                 unsigned long long *sink) {
+    __shared__ shg::SplitKey<SIMD> keys[kPeakKeys];
+    // low 30 bits zero: every seed of the run is within the keys' room
+    for (uint32_t i = threadIdx.x; i < kPeakKeys; i += blockDim.x)
+        keys[i] = shg::SplitKey<SIMD>::make(shg::remix(0x9E3779B97F4A7C15ULL * (i + 1) + blockIdx.x) & ~(uint64_t)(shg::kSeedSpan - 1));
+    __syncthreads();
     const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    uint64_t k0 = shg::remix(tid * 0x9E3779B97F4A7C15ULL), k1 = shg::remix(k0);
-    const uint64_t x0 = 0x643e521ddbd2be98ULL + tid;
-    uint32_t c0 = 0, c1 = 0, c2 = 0, d0 = 0, d1 = 0, d2 = 0;
-    for (uint64_t i = 0; i < iters; i++) {
-        const uint32_t p0 = shg::remix_low16(k0 + x0 + i) >> 14;
-        const uint32_t p1 = shg::remix_low16(k1 + x0 + i) >> 14;
-        const uint32_t q0 = p0 * p0, q1 = p1 * p1;
-        c0 += p0; c1 += q0; c2 += q0 * p0;
-        d0 += p1; d1 += q1; d2 += q1 * p1;
+    uint32_t seed = (threadIdx.x >> 5) * 64 + (threadIdx.x & 31), out = 0;
+    for (uint64_t done = 0; done < iters; done += kPeakKeys, seed = (seed + 512) & (shg::kSeedSpan / 2 - 1)) {
+        uint32_t c[2][3] = {};
+        if constexpr (NT == 4) shg::quarter_range<2, SIMD>(keys, 0, kPeakKeys, seed, c);
+        else shg::count_range<NT, 2, SIMD>(keys, 0, kPeakKeys, seed, T0, T1, T2, c);
+        for (int s = 0; s < 2; s++) out ^= c[s][0] ^ c[s][1] ^ c[s][2];
     }
-    sink[tid] = c0 ^ c1 ^ c2 ^ d0 ^ d1 ^ d2 ^ T0 ^ T1 ^ T2;  // every thread's result is stored: no loop can fold
+    sink[tid] = out;  // every thread's result is stored: no loop can fold
 }
-
-// The arithmetic of the split kernel's compare-and-count loop (fanout-2 and uneven nodes): remix to
-// 16 bits, one count per part threshold (NT of them); two seeds per key pair, as k_int_peak.
-template <int NT>
-__global__ void __launch_bounds__(kPeakThreads) k_int_peak_cmp(uint64_t iters, uint32_t T0, uint32_t T1, uint32_t T2,
-                                                               unsigned long long *sink) {
-    const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    uint64_t k0 = shg::remix(tid * 0x9E3779B97F4A7C15ULL), k1 = shg::remix(k0);
-    const uint64_t x0 = 0x643e521ddbd2be98ULL + tid;
-    const uint32_t T[3] = {T0, T1, T2};
-    uint32_t c[2][3] = {};
-    for (uint64_t i = 0; i < iters; i++) {
-        const uint32_t r0 = shg::remix_low16(k0 + x0 + i);
-        const uint32_t r1 = shg::remix_low16(k1 + x0 + i);
-#pragma unroll
-        for (int t = 0; t < NT; t++) {
-            c[0][t] += r0 < T[t];
-            c[1][t] += r1 < T[t];
-        }
+template <bool SIMD> void launch_peak_split(int nt, int blocks, uint64_t iters, unsigned long long *sink) {
+    switch (nt) {
+        case 1: k_int_peak_split<1, SIMD><<<blocks, kPeakThreads>>>(iters, 50331, 65536, 65536, sink); break;
+        case 2: k_int_peak_split<2, SIMD><<<blocks, kPeakThreads>>>(iters, 21846, 43691, 65536, sink); break;
+        case 3: k_int_peak_split<3, SIMD><<<blocks, kPeakThreads>>>(iters, 16384, 32768, 49152, sink); break;
+        default: k_int_peak_split<4, SIMD><<<blocks, kPeakThreads>>>(iters, 16384, 32768, 49152, sink); break;
     }
-    sink[tid] = c[0][0] ^ c[0][1] ^ c[0][2] ^ c[1][0] ^ c[1][1] ^ c[1][2];
-}
-
-// The same two loops with remix split between the integer and multiply pipes (the split kernel's
-// arithmetic option 1): quarter moments (NT = 4) or compare-and-count against NT thresholds.
-template <int NT>
-__global__ void __launch_bounds__(kPeakThreads) k_int_peak_pipes(uint64_t iters, uint32_t T0, uint32_t T1, uint32_t T2,
-                                                                 const shg::PipeK K, unsigned long long *sink) {
-    const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    uint64_t k0 = shg::remix(tid * 0x9E3779B97F4A7C15ULL), k1 = shg::remix(k0);
-    const uint64_t x0 = 0x643e521ddbd2be98ULL + tid;
-    const uint32_t T[3] = {T0, T1, T2};
-    uint32_t c[2][3] = {};
-    for (uint64_t i = 0; i < iters; i++) {
-        uint32_t a0, b0, a1, b1;
-        shg::remix_lo32_pipes(k0 + x0 + i, K, a0, b0);
-        shg::remix_lo32_pipes(k1 + x0 + i, K, a1, b1);
-        if (NT == 4) {
-            const uint32_t p0 = __umulhi((a0 ^ b0) & 0xC000u, K.c18), p1 = __umulhi((a1 ^ b1) & 0xC000u, K.c18);
-            const uint32_t q0 = p0 * p0, q1 = p1 * p1;
-            c[0][0] += p0; c[0][1] += q0; c[0][2] += q0 * p0;
-            c[1][0] += p1; c[1][1] += q1; c[1][2] += q1 * p1;
-        } else {
-            const uint32_t r0 = (a0 ^ b0) & 0xFFFFu, r1 = (a1 ^ b1) & 0xFFFFu;
-#pragma unroll
-            for (int t = 0; t < NT; t++) {
-                c[0][t] = shg::add_sign_bit(c[0][t], r0 - T[t], K.two);
-                c[1][t] = shg::add_sign_bit(c[1][t], r1 - T[t], K.two);
-            }
-        }
-    }
-    sink[tid] = c[0][0] ^ c[0][1] ^ c[0][2] ^ c[1][0] ^ c[1][1] ^ c[1][2];
-}
-
-// The split loops under SIMDShockHash's split hash (fmix32 of the xor-folded halves): quarter
-// moments (NT = 4) or compare-and-count against NT thresholds; two seeds per key pair.
-template <int NT>
-__global__ void __launch_bounds__(kPeakThreads) k_int_peak_simd(uint64_t iters, uint32_t T0, uint32_t T1, uint32_t T2,
-                                                                unsigned long long *sink) {
-    const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    uint64_t k0 = shg::remix(tid * 0x9E3779B97F4A7C15ULL), k1 = shg::remix(k0);
-    const uint64_t x0 = 0x643e521ddbd2be98ULL + tid;
-    const uint32_t T[3] = {T0, T1, T2};
-    uint32_t c[2][3] = {};
-    for (uint64_t i = 0; i < iters; i++) {
-        const uint32_t r0 = shg::simd_split_low16(k0 + x0 + i), r1 = shg::simd_split_low16(k1 + x0 + i);
-        if (NT == 4) {
-            const uint32_t p0 = r0 >> 14, p1 = r1 >> 14;
-            const uint32_t q0 = p0 * p0, q1 = p1 * p1;
-            c[0][0] += p0; c[0][1] += q0; c[0][2] += q0 * p0;
-            c[1][0] += p1; c[1][1] += q1; c[1][2] += q1 * p1;
-        } else {
-#pragma unroll
-            for (int t = 0; t < NT; t++) {
-                c[0][t] += r0 < T[t];
-                c[1][t] += r1 < T[t];
-            }
-        }
-    }
-    sink[tid] = c[0][0] ^ c[0][1] ^ c[0][2] ^ c[1][0] ^ c[1][1] ^ c[1][2];
 }
 
 // The original leaf search's coverage rounds as the leaf kernel runs them, alone: a leaf of h1 + h2
@@ -225,42 +159,13 @@ void shg_keys_mix(uint64_t seed, uint64_t n, uint64_t *out, int threads) {
     for (auto &th : pool) th.join();
 }
 
-// Integer-pipe peak: evaluations per second of the split search arithmetic on `device`.
-int shg_int_peak(int device, uint64_t iters, double *evals_per_s, double *ms_out) {
-    if (cudaSetDevice(device) != cudaSuccess) return SHG_ERR_CUDA;
-    cudaDeviceProp prop;
-    cudaGetDeviceProperties(&prop, device);
-    const int blocks = prop.multiProcessorCount * 8;
-    unsigned long long *sink;
-    if (cudaMalloc(&sink, (size_t)blocks * kPeakThreads * 8) != cudaSuccess) return SHG_ERR_OOM;  // one result per thread
-    cudaEvent_t a, b;
-    cudaEventCreate(&a);
-    cudaEventCreate(&b);
-    const uint32_t T0 = 16384, T1 = 32768, T2 = 49152;
-    k_int_peak<<<blocks, kPeakThreads>>>(iters / 16 + 1, T0, T1, T2, sink);  // warm-up
-    cudaEventRecord(a);
-    k_int_peak<<<blocks, kPeakThreads>>>(iters, T0, T1, T2, sink);
-    cudaEventRecord(b);
-    cudaEventSynchronize(b);
-    float ms = 0;
-    cudaEventElapsedTime(&ms, a, b);
-    cudaEventDestroy(a);
-    cudaEventDestroy(b);
-    cudaFree(sink);
-    if (cudaGetLastError() != cudaSuccess) return SHG_ERR_CUDA;
-    *evals_per_s = 2.0 * (double)iters * blocks * kPeakThreads / (ms * 1e-3);
-    if (ms_out) *ms_out = ms;
-    return SHG_OK;
-}
-
-// Integer-pipe peak of one search's inner loop (0 = split quarter moments, 1 = original leaf,
+// Integer-pipe peak of one search's inner loop (0 = quarter split, 1 = original leaf,
 // 2 = bipartite leaf hashing, 3..5 = split compare-and-count with 1..3 thresholds, 6..8 = bipartite
-// candidate scan, pair filter and pseudoforest edges, 9..12 = kinds 0 and 3..5 with the split
-// kernel's pipe-split arithmetic, 13..15 = kinds 6..8 for leaves of more than 64 keys, 16..19 = kinds
-// 0 and 3..5 under SIMDShockHash's split hash, 20 = kind 13 with the other form of the mask test).
+// candidate scan, pair filter and pseudoforest edges, 9..12 = the loops of kinds 0 and 3..5 again
+// (split_arith 1 runs the same ones), 13..15 = kinds 6..8 for leaves of more than 64 keys, 16..19 =
+// kinds 0 and 3..5 under SIMDShockHash's split hash, 20 = kind 13 with the other form of the mask test).
 int shg_int_peak_kind(int device, int kind, uint64_t iters, double *evals_per_s, double *ms_out) {
-    if (kind == 0) return shg_int_peak(device, iters, evals_per_s, ms_out);
-    if (kind < 1 || kind > 20) return SHG_ERR_ARG;
+    if (kind < 0 || kind > 20) return SHG_ERR_ARG;
     if (cudaSetDevice(device) != cudaSuccess) return SHG_ERR_CUDA;
     cudaDeviceProp prop;
     cudaGetDeviceProperties(&prop, device);
@@ -277,33 +182,20 @@ int shg_int_peak_kind(int device, int kind, uint64_t iters, double *evals_per_s,
             k_int_peak_sh1<<<blocks, kPeakThreads>>>(it, 20, 20, sink);
         else if (kind == 2)
             k_int_peak_sh2<<<blocks, kPeakThreads>>>(it, 32, sink);
-        else if (kind == 3)
-            k_int_peak_cmp<1><<<blocks, kPeakThreads>>>(it, 50331, 65536, 65536, sink);
-        else if (kind == 4)
-            k_int_peak_cmp<2><<<blocks, kPeakThreads>>>(it, 21846, 43691, 65536, sink);
-        else if (kind == 5)
-            k_int_peak_cmp<3><<<blocks, kPeakThreads>>>(it, 16384, 32768, 49152, sink);
+        else if (kind == 0 || kind == 9)
+            launch_peak_split<false>(4, blocks, it, sink);
+        else if (kind <= 5)
+            launch_peak_split<false>(kind - 2, blocks, it, sink);
         else if (kind <= 8)  // the bipartite leaf's scan, pair filter and pseudoforest loops (64 edges per iteration)
             shg::launch_sh2_op_peak(kind - 6, blocks, kind == 8 ? it / 64 + 1 : it, sink);
-        else if (kind == 16)
-            k_int_peak_simd<4><<<blocks, kPeakThreads>>>(it, 16384, 32768, 49152, sink);
-        else if (kind == 17)
-            k_int_peak_simd<1><<<blocks, kPeakThreads>>>(it, 50331, 65536, 65536, sink);
-        else if (kind == 18)
-            k_int_peak_simd<2><<<blocks, kPeakThreads>>>(it, 21846, 43691, 65536, sink);
-        else if (kind == 19)
-            k_int_peak_simd<3><<<blocks, kPeakThreads>>>(it, 16384, 32768, 49152, sink);
+        else if (kind <= 12)
+            launch_peak_split<false>(kind - 9, blocks, it, sink);
+        else if (kind >= 16 && kind <= 19)
+            launch_peak_split<true>(kind == 16 ? 4 : kind - 16, blocks, it, sink);
         else if (kind == 20)
             shg::launch_sh2_op_peak(6, blocks, it, sink);
-        else if (kind >= 13)  // the same for leaves of more than 64 keys (100 edges per iteration)
+        else  // 13..15: kinds 6..8 for leaves of more than 64 keys (100 edges per iteration)
             shg::launch_sh2_op_peak(kind - 10, blocks, kind == 15 ? it / 100 + 1 : it, sink);
-        else {  // 9: quarter moments, 10..12: 1..3 thresholds, with the split kernel's pipe-split arithmetic
-            const shg::PipeK K{4u, 32u, 1u << 18, 2u};
-            if (kind == 9) k_int_peak_pipes<4><<<blocks, kPeakThreads>>>(it, 16384, 32768, 49152, K, sink);
-            else if (kind == 10) k_int_peak_pipes<1><<<blocks, kPeakThreads>>>(it, 50331, 65536, 65536, K, sink);
-            else if (kind == 11) k_int_peak_pipes<2><<<blocks, kPeakThreads>>>(it, 21846, 43691, 65536, K, sink);
-            else k_int_peak_pipes<3><<<blocks, kPeakThreads>>>(it, 16384, 32768, 49152, K, sink);
-        }
         if (rep) cudaEventRecord(b);
     }
     cudaEventSynchronize(b);
@@ -325,10 +217,16 @@ int shg_int_peak_kind(int device, int kind, uint64_t iters, double *evals_per_s,
         per_iter = shg::sh2_op_peak_per_iter(6);
     } else if (kind == 1) {
         timed_iters = (iters + 39) / 40 * 40;  // whole rounds of the 40-key leaf
+    } else if (kind != 2) {
+        timed_iters = (iters + kPeakKeys - 1) / kPeakKeys * kPeakKeys;  // whole rounds of the split loops' keys
     }
     *evals_per_s = per_iter * (double)timed_iters * blocks * kPeakThreads / (ms * 1e-3);
     if (ms_out) *ms_out = ms;
     return SHG_OK;
+}
+
+int shg_int_peak(int device, uint64_t iters, double *evals_per_s, double *ms_out) {
+    return shg_int_peak_kind(device, 0, iters, evals_per_s, ms_out);
 }
 
 } // extern "C"

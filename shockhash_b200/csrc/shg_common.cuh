@@ -65,35 +65,75 @@ SHG_HD uint32_t fmix32(uint32_t z) {
 // halves lane by lane). Only the low 16 bits reach remap16.
 SHG_HD uint32_t simd_split_low16(uint64_t z) { return fmix32((uint32_t)(z >> 32) ^ (uint32_t)z) & 0xFFFFu; }
 
-#ifdef __CUDACC__
-// remix's low 32 bits with the work split between the integer and multiply pipes: the high words
-// of the two xor-shifts are taken as multiply-highs by the runtime constants K.four (4) and
-// K.thirtytwo (32), which the compiler cannot turn back into shifts, so that they run on the
-// multiply-add pipe next to the 64-bit products. Returns (lo, t): remix(z) = lo ^ t in the low 32
-// bits, left unmerged so that the caller folds its own mask into the same logic operation.
-struct PipeK {
-    uint32_t four, thirtytwo, c18, two;  // 4, 32, 2^18, 2 (kernel arguments)
+// ------------------------------------------------------------------ remix over consecutive seeds
+// The searches hash a key under seeds x0, x0 + 1, ...: z = (key + x0) + t for t = 0, 1, .... While the
+// low 30 bits of key + x0 plus t stay below 2^30, t changes only z's low 30 bits, so that
+//   * z >> 30 is the same word for every t: the first xor-shift is one 32-bit addition and one xor of
+//     the low half with a word of the key (`fold`), instead of a 64-bit addition, two shifts and two
+//     xors, and the high half z_hi ^ (z_hi >> 30) does not depend on t at all;
+//   * nor does the high half's term z_hi' * M1_lo of the first product, which is kept per key (`hc`,
+//     in the high word of the 64-bit addend of lo * M1_lo).
+// seed_room says how many values of t keep that true for a key; past it a search prepares its keys
+// again (seed_key of z + t), which happens about once in 2^30 / t seeds and key.
+constexpr uint64_t kRemixM1 = 0xbf58476d1ce4e5b9ULL, kRemixM2 = 0x94d049bb133111ebULL;
+constexpr uint32_t kM1Lo = (uint32_t)kRemixM1, kM1Hi = (uint32_t)(kRemixM1 >> 32);
+constexpr uint32_t kM2Lo = (uint32_t)kRemixM2, kM2Hi = (uint32_t)(kRemixM2 >> 32);
+// The inverse of an odd number modulo 2^32 (Newton's iteration: five steps from three right bits).
+constexpr uint32_t inverse32(uint32_t a) {
+    uint32_t x = a;
+    for (int i = 0; i < 5; i++) x *= 2 - a * x;
+    return x;
+}
+struct alignas(16) SeedKey {
+    uint32_t lo, fold;  // low halves of z and of z >> 30
+    uint64_t hc;        // (z_hi ^ (z_hi >> 30)) * M1_lo in the high word, 0 in the low one
 };
-__device__ __forceinline__ void remix_lo32_pipes(uint64_t z, const PipeK &K, uint32_t &lo4, uint32_t &t) {
-    uint32_t lo = (uint32_t)z, hi = (uint32_t)(z >> 32);
-    lo ^= __funnelshift_r(lo, hi, 30);  // z ^= z >> 30
-    hi ^= __umulhi(hi, K.four);
-    uint64_t w = (uint64_t)lo * 0x1ce4e5b9u;  // z *= 0xbf58476d1ce4e5b9
-    uint32_t lo2 = (uint32_t)w, hi2 = (uint32_t)(w >> 32) + lo * 0xbf58476du + hi * 0x1ce4e5b9u;
-    lo2 ^= __funnelshift_r(lo2, hi2, 27);  // z ^= z >> 27
-    hi2 ^= __umulhi(hi2, K.thirtytwo);
-    w = (uint64_t)lo2 * 0x133111ebu;  // z *= 0x94d049bb133111eb (bits 0..46 matter)
-    lo4 = (uint32_t)w;
-    const uint32_t hi4 = (uint32_t)(w >> 32) + lo2 * 0x94d049bbu + hi2 * 0x133111ebu;
-    t = __funnelshift_r(lo4, hi4, 31);  // z ^ (z >> 31)
+SHG_HD SeedKey seed_key(uint64_t z) {
+    const uint32_t hi = (uint32_t)(z >> 32);
+    return SeedKey{(uint32_t)z, (uint32_t)(z >> 30), (uint64_t)((hi ^ (hi >> 30)) * kM1Lo) << 32};
 }
-// c + (x >> 31) as one multiply-add-high (x * 2 >> 32), on the multiply-add pipe.
-__device__ __forceinline__ uint32_t add_sign_bit(uint32_t c, uint32_t x, uint32_t two) {
-    uint32_t d;
-    asm("mad.hi.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(x), "r"(two), "r"(c));
-    return d;
+// z back from its SeedKey (hi ^ (hi >> 30) is its own inverse: the top two bits stay as they are).
+SHG_HD uint64_t seed_key_z(const SeedKey &k) {
+    const uint32_t h = (uint32_t)(k.hc >> 32) * inverse32(kM1Lo);
+    return (uint64_t)(h ^ (h >> 30)) << 32 | k.lo;
 }
+constexpr uint32_t kSeedSpan = 1u << 30;
+// t < seed_room(z) keeps the SeedKey of z valid for z + t.
+SHG_HD uint32_t seed_room(uint64_t z) { return kSeedSpan - ((uint32_t)z & (kSeedSpan - 1)); }
+SHG_HD uint32_t funnel_r(uint32_t lo, uint32_t hi, int n) { return lo >> n | hi << (32 - n); }  // 0 < n < 32
+// remix(z + t) up to the second xor-shift: the two halves of the word that is multiplied by M2.
+SHG_HD void seed_mid(const SeedKey &k, uint32_t t, uint32_t &l2, uint32_t &h2) {
+    const uint32_t lo = (k.lo + t) ^ k.fold;
+    const uint64_t p = (uint64_t)lo * kM1Lo + k.hc;
+    const uint32_t l = (uint32_t)p, h = (uint32_t)(p >> 32) + lo * kM1Hi;
+    l2 = l ^ funnel_r(l, h, 27);
+    h2 = h ^ (h >> 27);
+}
+SHG_HD uint32_t mulhi32(uint32_t a, uint32_t b) {
+#ifdef __CUDA_ARCH__
+    return __umulhi(a, b);
+#else
+    return (uint32_t)(((uint64_t)a * b) >> 32);
 #endif
+}
+// Two words whose xor holds bits 14 and 15 of remix(z + t) at bits P - 1 and P (17 <= P <= 31) and
+// other bits elsewhere: bits 14, 15 and 45, 46 of the second product, with the shifts to position P
+// made part of its constants.
+template <int P> SHG_HD void seed_quarter_at(const SeedKey &k, uint32_t t, uint32_t &a, uint32_t &b) {
+    static_assert(P >= 17 && P <= 31, "bit position of the hash");
+    uint32_t l2, h2;
+    seed_mid(k, t, l2, h2);
+    a = l2 * (kM2Lo << (P - 15));
+    b = mulhi32(l2, kM2Lo) * (1u << (P - 14)) + l2 * (kM2Hi << (P - 14)) + h2 * (kM2Lo << (P - 14));
+}
+// The low 16 bits of remix(z + t) at bits 15..30, other bits below and 0 above.
+SHG_HD uint32_t seed_low16_at30(const SeedKey &k, uint32_t t) {
+    uint32_t l2, h2;
+    seed_mid(k, t, l2, h2);
+    const uint64_t p = (uint64_t)l2 * kM2Lo;
+    const uint32_t lo = (uint32_t)p, hi = (uint32_t)(p >> 32) + l2 * kM2Hi + h2 * kM2Lo;
+    return (l2 * (kM2Lo << 15) ^ funnel_r(lo, hi, 16)) & 0x7FFFFFFFu;
+}
 
 // Lemire range reduction. fastrange32 takes the low 32 bits of its argument
 // (TinyBinaryCuckooHashTable.h:140-141, SimdUtils.h:48-51).

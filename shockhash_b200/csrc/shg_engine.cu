@@ -572,8 +572,8 @@ shg_status build_batch(shg_engine *e, const shg_params *p, const uint64_t *d_fir
     auto split_range = [&](size_t lv, uint64_t a, uint64_t b, cudaStream_t st) {
         if (b <= a) return;
         launch_split_level(e->nodes.as<Node>(), d_ids + level_off[lv] + a, (uint32_t)(b - a), e->keys.as<uint64_t>(),
-                           e->codes.as<uint64_t>(), p->max_trials, &misc->err, &misc->work[0], misc->split_kind, tun.split,
-                           st);
+                           e->codes.as<uint64_t>(), p->max_trials, &misc->err, &misc->work[0], misc->split_kind,
+                           std::min<uint32_t>(maxsz, tab.level_max[lv]), tun.split, st);
         launches++;
     };
     auto leaf_range = [&](uint64_t a, uint64_t b, cudaStream_t st, int grid) {
@@ -592,7 +592,7 @@ shg_status build_batch(shg_engine *e, const shg_params *p, const uint64_t *d_fir
     };
     if (queue) {
         // one persistent launch over the staggered item order: split nodes and per-bucket leaf groups
-        const int qsmem = tree_queue_smem_per_block(tun.split.spl);
+        const int qsmem = tree_queue_smem_per_block(tun.split.spl, maxsz);
         int qbps = std::max(1, std::min(3, (228 * 1024) / (qsmem + 1024)));
         if (tun.leaf_bps > 0) qbps = std::min(qbps, tun.leaf_bps);
         const int qgrid = std::max(1, std::min<int>(e->sms * qbps, (int)std::max<uint64_t>(leaf_off + nb, 1)));
@@ -630,7 +630,8 @@ shg_status build_batch(shg_engine *e, const shg_params *p, const uint64_t *d_fir
                           offs_stride, (uint32_t)nlevels, e->qdone.as<uint32_t>(), e->keys.as<uint64_t>(),
                           e->codes.as<uint64_t>(), e->rib_bits.as<uint8_t>(), e->scratch.as<uint8_t>(), per_warp, smax, cmax,
                           p->max_trials, &misc->err, misc->work, misc->split_kind, misc->qctr, groups ? 0u : nleaves,
-                          e->acc.as<uint64_t>(), e->singles.as<uint64_t>(), q_out, (uint32_t)R, tun.split, qgrid, s);
+                          e->acc.as<uint64_t>(), e->singles.as<uint64_t>(), q_out, (uint32_t)R, maxsz, tun.split, qgrid,
+                          s);
         launches++;
         CU(cudaEventRecord(e->ev[3], s));  // the split stage's time covers the whole queue launch
     } else if (pipelined) {

@@ -96,6 +96,7 @@ struct ShapeTables {
     std::vector<uint32_t> node_off;  // [rows + 1]
     std::vector<uint16_t> singles;
     std::vector<uint32_t> single_off;  // [rows + 1]
+    uint16_t level_max[kMaxLevels] = {};  // keys of the largest split node of each level
 };
 void make_shape_tables(const Config &c, uint32_t rows, ShapeTables &t);
 
@@ -153,8 +154,8 @@ struct SplitTuning {
     int spl = 2;         // seeds per lane: 1, 2 or 4
     int threads = 256;   // threads per split block (one node per block): 128, 256 or 512
     int round_div = 8;   // warp groups make a round about 1/round_div of a node's expected trials (1..64)
-    int arith = 0;       // 0: remix as the compiler schedules it; 1: split between integer and multiply pipes;
-                         // kSplitArithSimd: SIMDShockHash's split hash (set by the engine, not by the table)
+    int arith = 0;       // 0 or 1: remix (one form serves both); kSplitArithSimd: SIMDShockHash's split hash
+                         // (set by the engine, not by the table)
 };
 constexpr int kSplitArithSimd = 2;
 struct Tuning {
@@ -168,10 +169,10 @@ struct Tuning {
 bool split_tuning_valid(int spl, int threads, int round_div, int arith);
 constexpr int kTuningFlat = 4;  // tuning-table variant key of ShockHash2Flat<k> (leaf size = k)
 // work[0] += useful evaluations; kind_work[k] += the same per inner loop (k = compared thresholds
-// - 1, or 3 for quarter-split moments)
+// - 1, or 3 for the quarter split). max_m: no node of the launch has more keys.
 void launch_split_level(const Node *nodes, const uint32_t *ids, uint32_t count, uint64_t *keys,
                         uint64_t *codes, uint64_t max_trials, uint32_t *err, unsigned long long *work,
-                        unsigned long long *kind_work, const SplitTuning &t, cudaStream_t s);
+                        unsigned long long *kind_work, uint32_t max_m, const SplitTuning &t, cudaStream_t s);
 int leaves_sh1_warps_per_block();
 // Inner-loop peaks of the bipartite leaf search (kind 0 scan, 1 pair filter, 2 pseudoforest edges),
 // 256-thread blocks; operations per thread and iteration from sh2_op_peak_per_iter.
@@ -191,7 +192,7 @@ struct QueueOut {
     uint8_t *bits;
 };
 int tree_queue_warps_per_block();
-int tree_queue_smem_per_block(int spl);
+int tree_queue_smem_per_block(int spl, uint32_t max_m);  // max_m: keys of the largest node
 // Time slots T of the staggered item order (nb + nlevels * lag); launch_queue_order writes the items
 // into seq[0 .. nsplit + buckets with leaves), with scratch cnt[T] and pos[T + 1] (pos[T]: the
 // item count). Without groups the sequence holds the split nodes only, and the queue kernel is
@@ -205,7 +206,7 @@ void launch_tree_queue(const Node *nodes, const uint32_t *ids, const uint32_t *s
                        uint64_t *codes, uint8_t *rib_bits, uint8_t *scratch, uint64_t per_warp, uint32_t smax, uint32_t cmax,
                        uint64_t max_trials, uint32_t *err, unsigned long long *work, unsigned long long *kind_work,
                        unsigned int *ctr, uint32_t nleaf_tail, const uint64_t *acc, const uint64_t *singles,
-                       const QueueOut *out, uint32_t nreq, const SplitTuning &t, int grid, cudaStream_t s);
+                       const QueueOut *out, uint32_t nreq, uint32_t max_m, const SplitTuning &t, int grid, cudaStream_t s);
 void launch_gr_bucket_bits(const Node *nodes, const uint32_t *bnb, uint64_t nb, const uint64_t *acc,
                            const uint64_t *codes, const uint32_t *memo_skip_bits, uint64_t *bucket_bits,
                            cudaStream_t s);

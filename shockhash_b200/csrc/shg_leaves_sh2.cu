@@ -1064,7 +1064,7 @@ __device__ __noinline__ void queue_leaf(const NodeLeaves &leaves, uint32_t li, c
     sh2_leaf<64, NodeLeaves, true, true>(leaves, li, keys, rib_bits, sm, g, uf, lane, smax, cmax, kQuadMinRecSplit, err, lw);
 }
 
-template <int SPL, int ARITH>
+template <int SPL>
 __global__ void __launch_bounds__(kQueueThreads, 3)
     k_tree_queue(const Node *__restrict__ nodes, const uint32_t *__restrict__ ids, const uint32_t *__restrict__ seq,
                  const uint32_t *__restrict__ nitems_p, uint32_t nsplit, const uint32_t *__restrict__ offs, uint64_t stride, uint32_t nlevels,
@@ -1073,11 +1073,11 @@ __global__ void __launch_bounds__(kQueueThreads, 3)
                  uint32_t cmax, uint64_t max_trials, uint32_t *__restrict__ err, unsigned long long *__restrict__ work,
                  unsigned long long *__restrict__ kind_work, unsigned int *__restrict__ ctr, uint32_t nleaf_tail,
                  const uint64_t *__restrict__ acc, const uint64_t *__restrict__ singles,
-                 const QueueOut *__restrict__ out, uint32_t nreq, int round_div, const PipeK K) {
+                 const QueueOut *__restrict__ out, uint32_t nreq, int round_div) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
     __shared__ uint32_t item, leaf_next;
     // the block's shared memory is one SplitSmem for a split node, one Sh2Smem per warp for leaves
-    SplitSmem<SPL, kQueueThreads> &ssm = *reinterpret_cast<SplitSmem<SPL, kQueueThreads> *>(smem_raw);
+    SplitSmem<SPL, kQueueThreads, false> &ssm = *reinterpret_cast<SplitSmem<SPL, kQueueThreads, false> *>(smem_raw);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     Sh2Smem<64> &sm = reinterpret_cast<Sh2Smem<64> *>(smem_raw)[warp];
     Sh2Global<64> g;
@@ -1099,8 +1099,8 @@ __global__ void __launch_bounds__(kQueueThreads, 3)
             if (threadIdx.x == 0 && !wait_done(&done[nd.bucket], splits_above(offs, stride, nd.bucket, nd.level), err))
                 atomicOr(err, kErrInternal);
             __syncthreads();
-            split_node<SPL, kQueueThreads, ARITH, true>(ssm, nd, id, keys, codes, max_trials, err, work, kind_work,
-                                                        round_div, K);
+            split_node<SPL, kQueueThreads, false, true>(ssm, nd, id, keys, codes, max_trials, err, work, kind_work,
+                                                        round_div);
             __threadfence();  // this thread's part of the partition before the bucket's counter moves
             __syncthreads();
             if (threadIdx.x == 0) atomicAdd(&done[nd.bucket], 1u);
@@ -1142,20 +1142,18 @@ __global__ void __launch_bounds__(kQueueThreads, 3)
         for (int k = 0; k < 5; k++) atomicAdd(&work[1 + k], w[k]);
 }
 
-template <int SPL, int ARITH>
+template <int SPL>
 void launch_queue_t(const Node *nodes, const uint32_t *ids, const uint32_t *seq, const uint32_t *nitems, uint32_t nsplit,
                     const uint32_t *offs, uint64_t stride, uint32_t nlevels, uint32_t *done, uint64_t *keys, uint64_t *codes,
                     uint8_t *rib_bits, uint8_t *scratch, uint64_t per_warp, uint32_t smax, uint32_t cmax,
                     uint64_t max_trials, uint32_t *err, unsigned long long *work, unsigned long long *kind_work,
                     unsigned int *ctr, uint32_t nleaf_tail, const uint64_t *acc, const uint64_t *singles,
-                    const QueueOut *out, uint32_t nreq, int round_div, int grid, cudaStream_t s) {
-    const size_t smem = std::max(sizeof(SplitSmem<SPL, kQueueThreads>), kQueueWarps * sizeof(Sh2Smem<64>));
-    cudaFuncSetAttribute(k_tree_queue<SPL, ARITH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    const PipeK K{4u, 32u, 1u << 18, 2u};
-    k_tree_queue<SPL, ARITH><<<grid, kQueueThreads, smem, s>>>(nodes, ids, seq, nitems, nsplit, offs, stride, nlevels, done,
-                                                               keys, codes, rib_bits, scratch, per_warp, smax, cmax,
-                                                               max_trials, err, work, kind_work, ctr, nleaf_tail, acc,
-                                                               singles, out, nreq, round_div, K);
+                    const QueueOut *out, uint32_t nreq, uint32_t max_m, int round_div, int grid, cudaStream_t s) {
+    const size_t smem = tree_queue_smem_per_block(SPL, max_m);
+    cudaFuncSetAttribute(k_tree_queue<SPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    k_tree_queue<SPL><<<grid, kQueueThreads, smem, s>>>(nodes, ids, seq, nitems, nsplit, offs, stride, nlevels, done, keys,
+                                                        codes, rib_bits, scratch, per_warp, smax, cmax, max_trials, err, work,
+                                                        kind_work, ctr, nleaf_tail, acc, singles, out, nreq, round_div);
 }
 
 } // namespace
@@ -1193,10 +1191,11 @@ void launch_leaves_sh2_ctr(const Node *nodes, const uint32_t *ids, uint32_t coun
 int sh2_smem_per_warp(int max_leaf) { return max_leaf <= 64 ? (int)sizeof(Sh2Smem<64>) : (int)sizeof(Sh2Smem<128>); }
 
 int tree_queue_warps_per_block() { return kQueueWarps; }
-int tree_queue_smem_per_block(int spl) {
+int tree_queue_smem_per_block(int spl, uint32_t max_m) {
     const size_t leaf = kQueueWarps * sizeof(Sh2Smem<64>);
-    const size_t split = spl == 1 ? sizeof(SplitSmem<1, kQueueThreads>)
-                                  : spl == 4 ? sizeof(SplitSmem<4, kQueueThreads>) : sizeof(SplitSmem<2, kQueueThreads>);
+    const size_t split = spl == 1   ? split_smem_bytes<1, kQueueThreads, false>(max_m)
+                         : spl == 4 ? split_smem_bytes<4, kQueueThreads, false>(max_m)
+                                    : split_smem_bytes<2, kQueueThreads, false>(max_m);
     return (int)std::max(leaf, split);
 }
 
@@ -1219,15 +1218,10 @@ void launch_tree_queue(const Node *nodes, const uint32_t *ids, const uint32_t *s
                        uint64_t *codes, uint8_t *rib_bits, uint8_t *scratch, uint64_t per_warp, uint32_t smax, uint32_t cmax,
                        uint64_t max_trials, uint32_t *err, unsigned long long *work, unsigned long long *kind_work,
                        unsigned int *ctr, uint32_t nleaf_tail, const uint64_t *acc, const uint64_t *singles,
-                       const QueueOut *out, uint32_t nreq, const SplitTuning &t, int grid, cudaStream_t s) {
-#define SHG_QUEUE_CASE(SPL, AR)                                                                                          \
-    if (t.spl == SPL && t.arith == AR)                                                                                  \
-        return launch_queue_t<SPL, AR>(nodes, ids, seq, nitems, nsplit, offs, stride, nlevels, done, keys, codes,        \
-                                       rib_bits, scratch, per_warp, smax, cmax, max_trials, err, work, kind_work, ctr,   \
-                                       nleaf_tail, acc, singles, out, nreq, t.round_div, grid, s);
-    SHG_QUEUE_CASE(1, 0) SHG_QUEUE_CASE(2, 0) SHG_QUEUE_CASE(4, 0) SHG_QUEUE_CASE(1, 1) SHG_QUEUE_CASE(2, 1)
-    SHG_QUEUE_CASE(4, 1)
-#undef SHG_QUEUE_CASE
+                       const QueueOut *out, uint32_t nreq, uint32_t max_m, const SplitTuning &t, int grid, cudaStream_t s) {
+    auto launch = t.spl == 1 ? launch_queue_t<1> : t.spl == 4 ? launch_queue_t<4> : launch_queue_t<2>;
+    launch(nodes, ids, seq, nitems, nsplit, offs, stride, nlevels, done, keys, codes, rib_bits, scratch, per_warp, smax, cmax,
+           max_trials, err, work, kind_work, ctr, nleaf_tail, acc, singles, out, nreq, max_m, t.round_div, grid, s);
 }
 
 // ------------------------------------------------------------------ inner-loop peaks

@@ -152,6 +152,7 @@ void make_shape_tables(const Config &c, uint32_t rows, ShapeTables &t) {
     t.cnt.assign((size_t)rows * t.ncol, 0);
     t.nodes.clear();
     t.singles.clear();
+    std::fill(t.level_max, t.level_max + kMaxLevels, (uint16_t)0);
     t.node_off.assign(rows + 1, 0);
     t.single_off.assign(rows + 1, 0);
     for (uint32_t m = 0; m < rows; m++) {
@@ -170,6 +171,7 @@ void make_shape_tables(const Config &c, uint32_t rows, ShapeTables &t) {
             n.unit = tn.unit;
             n.fixed_off = tn.fixed_off;
             n.seed = tn.seed;
+            if (tn.kind != kLeaf) t.level_max[tn.level] = std::max(t.level_max[tn.level], tn.m);
             const int col = tn.kind == kLeaf ? kColLeaves : kColLevel0 + tn.level;
             n.rank = (uint16_t)row[col]++;
             t.nodes.push_back(n);

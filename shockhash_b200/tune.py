@@ -35,8 +35,7 @@ from . import SHOCKHASH, SHOCKHASH2, SIMDSHOCKHASH, TUNING_FLAT, Engine, keys_mt
 HERE = os.path.dirname(os.path.abspath(__file__))
 TABLE = os.path.join(HERE, "tuning.tsv")
 
-SPLIT_CANDIDATES = {"split_arith": (0, 1), "split_seeds_per_lane": (1, 2, 4), "split_threads": (128, 256, 512),
-                    "split_round_div": (2, 4, 8, 16, 32)}
+SPLIT_CANDIDATES = {"split_seeds_per_lane": (1, 2, 4), "split_threads": (128, 256, 512), "split_round_div": (2, 4, 8, 16, 32)}
 LEAF_CANDIDATES = {
     SHOCKHASH2: {"leaf_blocks_per_sm": (3, 4, 5, 6, 7, 8), "leaf_min_blocks": (4, 6, 8)},
     SHOCKHASH: {"leaf_blocks_per_sm": (4, 6, 8, 12, 16), "sh1_seeds_per_lane": (1, 2)},
@@ -121,8 +120,6 @@ def tune_config(eng, variant, leaf, n, reps=3, min_gain=0.02, log=print):
         # the work-queue schedule (the default here): 256-thread blocks, at most 3 per SM
         split_c.pop("split_threads", None)
         leaf_c = {"leaf_blocks_per_sm": (1, 2, 3), "queue_lag_rounds": (0, 2, 4, 16, 32)}
-    if variant == SIMDSHOCKHASH:  # its split hash has one arithmetic form, chosen by the engine
-        split_c.pop("split_arith", None)
     if variant != TUNING_FLAT:
         params, _ = tu.descend(params, split_c, 0, min_gain)
     params, _ = tu.descend(params, leaf_c, 1, min_gain)
