@@ -15,6 +15,7 @@
 #include "shg.h"
 #include "shg_common.cuh"
 #include "shg_internal.h"
+#include "shg_sh1.cuh"
 #include "shg_split.cuh"
 
 namespace {
@@ -53,33 +54,23 @@ template <bool SIMD> void launch_peak_split(int nt, int blocks, uint64_t iters, 
     }
 }
 
-// The original leaf search's coverage rounds as the leaf kernel runs them, alone: a leaf of h1 + h2
-// keys in shared memory, lanes on consecutive seeds, two seeds per lane per key read (full 64-bit
-// remix, both cells by fastrange32 on its halves, one bit each into two 32-bit half masks), the
-// masks compared after each round; no pseudoforest tests. `iters` key reads per thread, rounded up
-// to whole rounds (the caller counts the rounded number).
+// The original leaf search's first sieve as the leaf kernel runs it, alone: a leaf of h1 + h2 staged keys
+// in shared memory, lanes on consecutive seeds, two seeds per lane per key read, the masks compared after
+// each round; no later sieves. `iters` key reads per thread, rounded up to whole rounds (the caller counts
+// the rounded number).
 __global__ void __launch_bounds__(kPeakThreads) k_int_peak_sh1(uint64_t iters, uint32_t h1, uint32_t h2,
                                                                unsigned long long *sink) {
-    __shared__ uint64_t keys[64];
-    for (int i = threadIdx.x; i < 64; i += blockDim.x) keys[i] = shg::remix(0x9E3779B97F4A7C15ULL * (i + 1) + blockIdx.x);
+    __shared__ shg::SeedKey keys[64];
+    for (int i = threadIdx.x; i < 64; i += blockDim.x)
+        keys[i] = shg::seed_key(shg::remix(0x9E3779B97F4A7C15ULL * (i + 1) + blockIdx.x) & ~(uint64_t)(shg::kSeedSpan - 1));
     __syncthreads();
-    const uint32_t m = h1 + h2, lane = threadIdx.x & 31;
-    const uint32_t all1 = (1u << h1) - 1, all2 = (1u << h2) - 1;
-    uint64_t base = 0x643e521ddbd2be98ULL + (blockIdx.x * (uint64_t)blockDim.x + (threadIdx.x & ~31u)) * 64 * iters;
-    uint32_t hits = 0;
-    for (uint64_t done = 0; done < iters; done += m, base += 64) {
-        uint32_t c1m[2] = {0, 0}, c2m[2] = {0, 0};
-        for (uint32_t k = 0; k < m; k++) {
-            const uint64_t key = keys[k];
+    const uint32_t m = h1 + h2, all2 = (1u << h2) - 1;
+    uint32_t at = (threadIdx.x >> 5) * 64 + (threadIdx.x & 31), hits = 0;
+    for (uint64_t done = 0; done < iters; done += m, at = (at + 512) & (shg::kSeedSpan / 2 - 1)) {
+        uint32_t mask[2] = {0, 0}, low[2] = {~0u, ~0u};
+        shg::sh1_half_masks<2>(keys, m, h2, at, mask, low);
 #pragma unroll
-            for (int t = 0; t < 2; t++) {
-                const uint64_t r = shg::remix(key + base + lane + 32 * t);
-                c1m[t] |= 1u << shg::fastrange32((uint32_t)r, h1);
-                c2m[t] |= 1u << shg::fastrange32((uint32_t)(r >> 32), h2);
-            }
-        }
-#pragma unroll
-        for (int t = 0; t < 2; t++) hits += c1m[t] == all1 && c2m[t] == all2;
+        for (int t = 0; t < 2; t++) hits += shg::sh1_half_passes(mask[t], low[t], all2, h2);
     }
     sink[blockIdx.x * (uint64_t)blockDim.x + threadIdx.x] = hits;
 }

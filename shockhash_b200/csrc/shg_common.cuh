@@ -126,6 +126,12 @@ template <int P> SHG_HD void seed_quarter_at(const SeedKey &k, uint32_t t, uint3
     a = l2 * (kM2Lo << (P - 15));
     b = mulhi32(l2, kM2Lo) * (1u << (P - 14)) + l2 * (kM2Hi << (P - 14)) + h2 * (kM2Lo << (P - 14));
 }
+// The high word of remix's second product for z + t: remix(z + t) >> 32 is hi ^ (hi >> 31).
+SHG_HD uint32_t seed_hi_product(const SeedKey &k, uint32_t t) {
+    uint32_t l2, h2;
+    seed_mid(k, t, l2, h2);
+    return mulhi32(l2, kM2Lo) + l2 * kM2Hi + h2 * kM2Lo;
+}
 // The low 16 bits of remix(z + t) at bits 15..30, other bits below and 0 above.
 SHG_HD uint32_t seed_low16_at30(const SeedKey &k, uint32_t t) {
     uint32_t l2, h2;

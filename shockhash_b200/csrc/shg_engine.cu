@@ -29,7 +29,7 @@ uint64_t sh2_scratch_bytes(uint32_t smax, uint32_t cmax, int max_leaf);
 void launch_leaves_sh1_ctr(const Node *nodes, const uint32_t *ids, uint32_t count, const uint64_t *keys, uint64_t *codes,
                            uint64_t *rib_keys, uint8_t *rib_bits, uint64_t max_trials, uint32_t *err,
                            unsigned long long *work, unsigned int *ctr, int grid, cudaStream_t s, uint32_t rot_leaf = 0,
-                           int spl = 2);
+                           int spl = 2, bool block = false);
 void launch_leaves_sh2_ctr(const Node *nodes, const uint32_t *ids, uint32_t count, const uint64_t *keys, uint64_t *codes,
                            uint8_t *rib_bits, uint8_t *scratch, uint64_t scratch_per_warp, uint32_t smax, uint32_t cmax,
                            uint32_t *err, unsigned long long *work, unsigned int *ctr, int grid, cudaStream_t s,
@@ -556,6 +556,7 @@ shg_status build_batch(shg_engine *e, const shg_params *p, const uint64_t *d_fir
     const uint32_t smax = maxm > 64 ? 16384 : 4096, cmax = maxm > 64 ? 16384 : 2048;
     const uint64_t per_warp = (sh2_scratch_bytes(smax, cmax, maxm) + 255) & ~255ull;
     int leaf_grid;
+    bool sh1_block = false;
     if (sh2) {
         const int per_block_smem = 4 * sh2_smem_per_warp(maxm);
         int blocks_per_sm = std::max(1, std::min(8, (228 * 1024) / (per_block_smem + 1024)));
@@ -567,7 +568,16 @@ shg_status build_batch(shg_engine *e, const shg_params *p, const uint64_t *d_fir
     } else {
         const int wpb = leaves_sh1_warps_per_block();
         const int bps = tun.leaf_bps > 0 ? tun.leaf_bps : 8;
-        leaf_grid = std::max(1, std::min<int>(e->sms * (pipelined ? std::max(1, bps / 2) : bps), (int)((nleaves + wpb - 1) / wpb)));
+        const int most = e->sms * (pipelined ? std::max(1, bps / 2) : bps);
+        // A block per leaf instead of a warp while the grid's warps would get few leaves each, measured
+        // against the seeds that a leaf takes (about 2^(g+1)): the longest of the last leaves sets the
+        // launch's end, and a block brings it down fourfold, but the block's warps wait for one another
+        // once per leaf. Leaf stage, warp / block: ShockHash<30>, 33 leaves 0.42 / 0.12 ms, 3,333 leaves
+        // 1.03 / 0.62, 10,000 leaves (2 per warp) 1.41 / 1.52, 33,333 leaves 3.38 / 4.70; ShockHash<40>,
+        // 2,500 leaves 18.1 / 6.5, 25,000 leaves (5 per warp) 49.2 / 43.6, 100,000 leaves 164 / 169.
+        const uint64_t trials = std::min(8192ull, 2ull << std::min(cfg.golomb((uint32_t)p->leaf_size), 20));
+        sh1_block = !is_rotation(p->variant) && (uint64_t)nleaves * 1024 <= (uint64_t)most * wpb * trials;
+        leaf_grid = std::max(1, std::min<int>(most, (int)(sh1_block ? nleaves : (nleaves + wpb - 1) / wpb)));
     }
     auto split_range = [&](size_t lv, uint64_t a, uint64_t b, cudaStream_t st) {
         if (b <= a) return;
@@ -587,7 +597,7 @@ shg_status build_batch(shg_engine *e, const shg_params *p, const uint64_t *d_fir
             launch_leaves_sh1_ctr(e->nodes.as<Node>(), d_ids + leaf_off + a, (uint32_t)(b - a), e->keys.as<uint64_t>(),
                                   e->codes.as<uint64_t>(), e->rib_keys.as<uint64_t>(), e->rib_bits.as<uint8_t>(), p->max_trials,
                                   &misc->err, misc->work, &misc->leaf_ctr, grid, st,
-                                  is_rotation(p->variant) ? (uint32_t)p->leaf_size : 0, tun.sh1_spl);
+                                  is_rotation(p->variant) ? (uint32_t)p->leaf_size : 0, tun.sh1_spl, sh1_block);
         launches++;
     };
     if (queue) {

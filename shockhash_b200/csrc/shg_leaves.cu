@@ -2,8 +2,10 @@
 //
 // Original ShockHash (ShockHash.h:404-434): lanes take consecutive seeds x (SPL per lane, x, x + 32,
 // ..., per round of 32 * SPL); a lane's seed passes
-// when the two candidate cells of all m keys cover all m cells (64-bit OR) and the cuckoo graph
-// (cells = vertices, keys = edges) is a pseudoforest. The pseudoforest test is a per-lane
+// when the two candidate cells of all m keys cover all m cells and the cuckoo graph
+// (cells = vertices, keys = edges) is a pseudoforest. Seeds go through three sieves in seed order:
+// the second-half cells of all keys cover their half (one key in 8 to 20 does, for leaves of 30 to 40
+// keys), both halves are covered, pseudoforest. The pseudoforest test is a per-lane
 // union-find with a cycle flag per root; the reference inserts into a cuckoo table instead, and
 // ordered cuckoo insertion succeeds exactly when the graph is a pseudoforest, so both accept the
 // same seeds. The coverage mask is kept as two 32-bit halves (first-half and second-half cells).
@@ -15,6 +17,7 @@
 #include <cuda_runtime.h>
 #include "shg_common.cuh"
 #include "shg_internal.h"
+#include "shg_sh1.cuh"
 
 namespace shg {
 
@@ -83,16 +86,28 @@ __device__ bool cuckoo_insert(int16_t *cell, uint8_t *xr, int e, uint32_t c1, ui
 }
 
 // ------------------------------------------------------------------ original ShockHash leaves
-// Seeds that pass the coverage test queue up (in seed order) until kSh1Drain of them wait, and are
-// then tested for the pseudoforest property side by side, one per lane: tested one round at a
-// time, a round's one or two passing seeds ran the union-find while the other lanes waited.
+// Seeds that pass a sieve queue up in seed order for the next one, so that each runs with its lanes
+// filled: the first sieve's survivors are tested for the full coverage 32 at a time (one per lane;
+// leaves of up to kSh1SmallLeaf keys, which expect fewer seeds than a round has, after every round),
+// and the full coverage's for the pseudoforest property side by side once kSh1Drain of them wait.
+//
+// What bounds it: the integer pipes, in the first sieve, which sees every seed. It therefore works on
+// staged keys (SeedKey, shg_common.cuh), looks at one half of the cells only (one range reduction, shift
+// and or per key instead of two), and takes the high word of remix without its last xor-shift: that
+// can change the lowest bit alone, so the cell is the same unless the product with the half's size
+// lies within one size of a multiple of 2^32. The smallest low word over the keys says whether one
+// does; such a seed (about 1 in 10^6) counts as passing, and the second sieve decides.
 #ifndef SHG_SH1_DRAIN
 #define SHG_SH1_DRAIN 4
 #endif
 constexpr uint32_t kSh1Drain = SHG_SH1_DRAIN;
-constexpr uint32_t kSh1Queue = kSh1Drain + 64;  // fewer than kSh1Drain wait, plus one round's 32 x SPL (SPL <= 2)
+constexpr uint32_t kSh1SmallLeaf = 16;
+constexpr uint32_t kSh1Half = 31 + 64;        // waiting for the full coverage: at most 31, plus one round's 32 x SPL (SPL <= 2)
+constexpr uint32_t kSh1Queue = kSh1Drain + 32;  // fewer than kSh1Drain wait, plus one batch of 32
 
 struct Sh1WarpSmem {
+    SeedKey staged[64];     // the keys under the first seed of the current span
+    uint64_t half[kSh1Half];  // seed offsets that cover the second half, ascending
     uint64_t q[kSh1Queue];  // coverage-passing seed offsets, ascending
     uint64_t keys[64];
     uint64_t fkeys[64];  // rotation fitting: even keys in order, odd keys from the back
@@ -222,7 +237,11 @@ __device__ bool rotation_leaf(Sh1WarpSmem &sm, uint16_t *cells, LaneUF &uf, int 
 }
 
 // SPL: seeds per lane and round (1 or 2; a tuning parameter, the same seed is found either way).
-template <int SPL>
+// BLOCK: the block's warps search a leaf together (not with rotation fitting): warp w takes the rounds w,
+// w + kLeafWarps, ..., on its own, and goes on until its next round begins past the smallest passing seed
+// any of them has found, so every smaller seed has been tried. One leaf then takes a quarter of the time,
+// and with it the launch's tail, in which the last leaves run alone.
+template <int SPL, bool BLOCK>
 __global__ void __launch_bounds__(kLeafWarps * 32) k_leaves_sh1(const Node *__restrict__ nodes, const uint32_t *__restrict__ ids,
                                                                 uint32_t count, const uint64_t *__restrict__ keys,
                                                                 uint64_t *__restrict__ codes, uint64_t *__restrict__ rib_keys,
@@ -234,10 +253,22 @@ __global__ void __launch_bounds__(kLeafWarps * 32) k_leaves_sh1(const Node *__re
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     Sh1WarpSmem &sm = wsm[warp];
     unsigned long long evals = 0;
+    __shared__ unsigned long long block_best;  // BLOCK: smallest passing seed offset of the leaf so far
+    __shared__ uint32_t block_leaf;
     for (;;) {
         uint32_t li = 0;
-        if (lane == 0) li = atomicAdd(next_leaf, 1u);
-        li = __shfl_sync(0xffffffffu, li, 0);
+        if constexpr (BLOCK) {
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                block_leaf = atomicAdd(next_leaf, 1u);
+                block_best = ~0ull;
+            }
+            __syncthreads();
+            li = block_leaf;
+        } else {
+            if (lane == 0) li = atomicAdd(next_leaf, 1u);
+            li = __shfl_sync(0xffffffffu, li, 0);
+        }
         if (li >= count) break;
         const uint32_t id = ids[li];
         const Node nd = nodes[id];
@@ -254,7 +285,7 @@ __global__ void __launch_bounds__(kLeafWarps * 32) k_leaves_sh1(const Node *__re
         uint64_t cap = 1ull << min(nd.g + 10, 40);
         if (max_trials && max_trials < cap) cap = max_trials;
         LaneUF uf{sm.uf, lane};
-        if (rot_leaf && m == rot_leaf) {
+        if (!BLOCK && rot_leaf && m == rot_leaf) {
             // ~2^(g+1) codes x * L + r are expected; the cap counts seeds x
             uint64_t cap_x = (1ull << min(nd.g + 10, 40)) / m + 1;
             if (max_trials && max_trials < cap_x) cap_x = max_trials;
@@ -307,38 +338,83 @@ __global__ void __launch_bounds__(kLeafWarps * 32) k_leaves_sh1(const Node *__re
             nq = 0;
             __syncwarp();  // the queue's slots are read before the next round refills them
         };
-        // SPL seeds per lane (x, x + 32, ...): one shared-memory key read feeds SPL evaluations.
-        for (uint64_t base = 0; base < cap && found == ~0ull; base += 32 * SPL) {
-            uint32_t c1m[SPL], c2m[SPL];
-#pragma unroll
-            for (int t = 0; t < SPL; t++) c1m[t] = c2m[t] = 0;
+        // the second sieve: the first n <= 32 waiting seeds, one per lane, against both halves
+        uint32_t nhalf = 0;
+        auto cover = [&](uint32_t n) {
+            const uint64_t off = (uint32_t)lane < n ? sm.half[lane] : 0;
+            uint32_t c1m = 0, c2m = 0;
             for (uint32_t k = 0; k < m; k++) {
-                const uint64_t key = sm.keys[k];
-#pragma unroll
-                for (int t = 0; t < SPL; t++) {
-                    const uint64_t r = remix(key + seed0 + base + lane + 32 * t);
-                    c1m[t] |= 1u << fastrange32((uint32_t)r, h1);
-                    c2m[t] |= 1u << fastrange32((uint32_t)(r >> 32), h2);
-                }
+                const uint64_t r = remix(sm.keys[k] + seed0 + off);
+                c1m |= 1u << fastrange32((uint32_t)r, h1);
+                c2m |= 1u << fastrange32((uint32_t)(r >> 32), h2);
             }
-            bool ok[SPL], any = false;
-#pragma unroll
-            for (int t = 0; t < SPL; t++) {
-                ok[t] = c1m[t] == all1 && c2m[t] == all2;
-                any |= ok[t];
+            const bool ok = (uint32_t)lane < n && c1m == all1 && c2m == all2;
+            const unsigned bal = __ballot_sync(0xffffffffu, ok);
+            if (ok) sm.q[nq + __popc(bal & below)] = off;
+            nq += __popc(bal);
+            // the rest moves up (at most 63 entries)
+            const uint32_t rest = nhalf - n;
+            const uint64_t v0 = (uint32_t)lane < rest ? sm.half[n + lane] : 0;
+            const uint64_t v1 = (uint32_t)lane + 32 < rest ? sm.half[n + 32 + lane] : 0;
+            __syncwarp();
+            if ((uint32_t)lane < rest) sm.half[lane] = v0;
+            if ((uint32_t)lane + 32 < rest) sm.half[32 + lane] = v1;
+            nhalf = rest;
+            __syncwarp();
+            if (nq >= kSh1Drain) drain();
+        };
+        // the keys staged for seeds seed0 + at, + at + 1, ...; how many such seeds they are good for
+        auto stage = [&](uint64_t at) {
+            uint32_t room = kSeedSpan;
+            for (uint32_t k = lane; k < m; k += 32) {
+                const uint64_t z = sm.keys[k] + seed0 + at;
+                sm.staged[k] = seed_key(z);
+                room = min(room, seed_room(z));
             }
-            if (__any_sync(0xffffffffu, any)) {
+            room = __reduce_min_sync(0xffffffffu, room);
+            __syncwarp();
+            return room;
+        };
+        uint64_t base0 = 0;
+        uint32_t room = stage(0);
+        const uint32_t batch = m <= kSh1SmallLeaf ? 1 : 32;
+        // SPL seeds per lane (x, x + 32, ...): one shared-memory key read feeds SPL evaluations.
+        constexpr uint32_t kStep = 32 * SPL * (BLOCK ? kLeafWarps : 1);
+        for (uint64_t base = BLOCK ? 32 * SPL * warp : 0; base < cap && found == ~0ull; base += kStep) {
+            if (BLOCK && base > *(volatile unsigned long long *)&block_best) break;
+            uint32_t mask[SPL], low[SPL];
 #pragma unroll
-                for (int t = 0; t < SPL; t++) {  // seeds in order: all lanes' x + 32 t before x + 32 (t + 1)
-                    const unsigned bal = __ballot_sync(0xffffffffu, ok[t]);
-                    if (ok[t]) sm.q[nq + __popc(bal & below)] = base + 32 * t + lane;
-                    nq += __popc(bal);
-                }
+            for (int t = 0; t < SPL; t++) mask[t] = 0, low[t] = ~0u;
+            const bool plain = base - base0 + 32 * SPL > room;
+            if (!plain) {
+                sh1_half_masks<SPL>(sm.staged, m, h2, (uint32_t)(base - base0) + lane, mask, low);
+            } else {  // some key's low bits run over in this round
+                for (uint32_t k = 0; k < m; k++)
+#pragma unroll
+                    for (int t = 0; t < SPL; t++)
+                        mask[t] |= 1u << fastrange32((uint32_t)(remix(sm.keys[k] + seed0 + base + lane + 32 * t) >> 32), h2);
+                base0 = base + kStep;
                 __syncwarp();
-                if (nq >= kSh1Drain) drain();
+                room = stage(base0);
             }
+#pragma unroll
+            for (int t = 0; t < SPL; t++) {  // seeds in order: all lanes' x + 32 t before x + 32 (t + 1)
+                const bool ok = sh1_half_passes(mask[t], low[t], all2, h2);
+                const unsigned bal = __ballot_sync(0xffffffffu, ok);
+                if (ok) sm.half[nhalf + __popc(bal & below)] = base + 32 * t + lane;
+                nhalf += __popc(bal);
+            }
+            __syncwarp();
+            while (found == ~0ull && nhalf >= batch) cover(min(nhalf, 32u));
         }
-        if (found == ~0ull && nq) drain();  // the last survivors, at the trial limit
+        while (found == ~0ull && nhalf) cover(min(nhalf, 32u));  // what still waits (the trial limit, or BLOCK)
+        if (found == ~0ull && nq) drain();
+        if constexpr (BLOCK) {
+            if (lane == 0 && found != ~0ull) atomicMin(&block_best, (unsigned long long)found);
+            __syncthreads();
+            found = block_best;
+            if (warp) continue;  // one warp writes the leaf's products
+        }
         if (found == ~0ull || found >= cap) {
             if (lane == 0) atomicOr(err, kErrTrialLimit);
             continue;
@@ -374,16 +450,15 @@ int leaves_sh1_warps_per_block() { return kLeafWarps; }
 void launch_leaves_sh1_ctr(const Node *nodes, const uint32_t *ids, uint32_t count, const uint64_t *keys, uint64_t *codes,
                            uint64_t *rib_keys, uint8_t *rib_bits, uint64_t max_trials, uint32_t *err,
                            unsigned long long *work, unsigned int *ctr, int grid, cudaStream_t s, uint32_t rot_leaf,
-                           int spl) {
+                           int spl, bool block) {
     if (!count) return;
+    block = block && !rot_leaf;
     cudaMemsetAsync(ctr, 0, sizeof(unsigned int), s);
     const size_t dyn = rot_leaf ? (size_t)kLeafWarps * 64 * 32 * sizeof(uint16_t) : 0;  // 16 KB per block
-    if (spl == 1)
-        k_leaves_sh1<1><<<grid, kLeafWarps * 32, dyn, s>>>(nodes, ids, count, keys, codes, rib_keys, rib_bits, max_trials,
-                                                           err, work, ctr, rot_leaf);
-    else
-        k_leaves_sh1<2><<<grid, kLeafWarps * 32, dyn, s>>>(nodes, ids, count, keys, codes, rib_keys, rib_bits, max_trials,
-                                                           err, work, ctr, rot_leaf);
+    auto kernel = block ? (spl == 1 ? k_leaves_sh1<1, true> : k_leaves_sh1<2, true>)
+                        : (spl == 1 ? k_leaves_sh1<1, false> : k_leaves_sh1<2, false>);
+    kernel<<<grid, kLeafWarps * 32, dyn, s>>>(nodes, ids, count, keys, codes, rib_keys, rib_bits, max_trials, err, work, ctr,
+                                              rot_leaf);
 }
 
 } // namespace shg

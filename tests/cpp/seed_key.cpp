@@ -30,6 +30,22 @@ int main() {
         for (uint32_t t : ts)
             if (check<17>(k, z, t)) return 1;
     }
+    // the original leaves' first sieve (shg_sh1.cuh): a cell taken without remix's last xor-shift is the
+    // exact one, or the low word says that it may not be
+    for (uint32_t h2 = 1; h2 <= 30; h2++) {
+        for (uint64_t j = 0; j <= h2; j++)
+            for (int d = -70; d <= 70; d++) {
+                const uint32_t t = (uint32_t)((j << 32) / h2 + d);
+                const uint64_t p = (uint64_t)t * h2 + h2;
+                const uint32_t cell = fastrange32(t ^ (t >> 31), h2);
+                if ((uint32_t)p >= 2 * h2 && (uint32_t)(p >> 32) != cell) return printf("h2 %u t %u\n", h2, t), 1;
+            }
+    }
+    for (int i = 0; i < 200000; i++) {  // the high word of the second product
+        const uint64_t z = rng();
+        const uint32_t t = (uint32_t)(rng() % seed_room(z)), hi = seed_hi_product(seed_key(z), t);
+        if ((hi ^ (hi >> 31)) != (uint32_t)(remix(z + t) >> 32)) return printf("hi z %llx\n", (unsigned long long)z), 1;
+    }
     printf("ok\n");
     return 0;
 }
