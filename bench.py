@@ -46,7 +46,7 @@ LEAF, BUCKET, VARIANT = 64, 2000, 2
 SEED = 7
 METRIC = "build ns/key on 1 B200, batched vs per-leaf GPU vs CPU, bit-exact; p99 latency"
 CONFIG_NAME = "ShockHash2<64> b=2000, 10M uint64 keys (mt19937_64 seed 7) hashed to 128-bit"
-MODES = ["default (work queue for ShockHash2 with leaves of up to 64 keys, else levels)", "levels", "per_leaf",
+MODES = ["default (by size: levels or queue)", "levels", "per_leaf",
          "pipelined", "queue"]
 # DRAM bytes (read + write) per key of one launch, from one ncu capture of the 1M-key case
 # (profiles/k_tree_queue_sh2_l64.md, profiles/k_split_sh2_l64.md) scaled by keys: the work-queue
@@ -655,8 +655,7 @@ def main():
     barrier()
     r2.free()
 
-    # the level schedule's stages, measured apart for the per-kernel fractions when the default build
-    # runs both searches in the work-queue kernel
+    # the level schedule's stages, measured apart for the per-kernel fractions
     lv = None
     if VARIANT == 2 and LEAF <= 64 and args.mode in (0, 4):
         t_lv, st_lv, last_lv = timed_device_builds(eng, d_keys.data_ptr(), n, shg.MODE_LEVELS, flush, reps=2)
@@ -680,7 +679,7 @@ def main():
     achieved = last.work["split_evals"] / (split_ms * 1e-3)
     # denominator: each node kind's useful evaluations at that kind's measured loop peak
     peak_eff = shg.weighted_split_peak(split_kinds, peaks)
-    # the default ShockHash2 build (leaves <= 64) runs both searches in the one work-queue kernel,
+    # a work-queue build (ShockHash2, leaves <= 64) runs both searches in the one kernel,
     # whose time is the split stage's: its ceiling is the split ceiling plus the leaf ceiling
     # (the library reports the whole launch as the split stage and no separate leaf stage then)
     queue_used = VARIANT == 2 and LEAF <= 64 and args.mode in (0, 4) and leaf_ms < 0.05 * split_ms

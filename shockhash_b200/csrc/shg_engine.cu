@@ -128,7 +128,7 @@ struct shg_engine {
         DevBuf cnt, nodes, node_off, singles, single_off, skip_bits;
     };
     std::vector<Shapes *> shapes;
-    DevBuf plan_offs, ret_scratch, qdone, qorder;
+    DevBuf plan_offs, ret_scratch, qdone, qorder, split_best;
     cudaEvent_t ev[8] = {};
     cudaStream_t stream2 = nullptr;  // leaves of the pipelined mode
     static constexpr int kMaxChunks = 64;
@@ -166,6 +166,7 @@ struct shg_engine {
         ret_scratch.release();
         qdone.release();
         qorder.release();
+        split_best.release();
         for (Shapes *sh : shapes) {
             DevBuf *sb[] = {&sh->cnt, &sh->nodes, &sh->node_off, &sh->singles, &sh->single_off, &sh->skip_bits};
             for (DevBuf *b : sb) b->release();
@@ -513,10 +514,14 @@ shg_status build_batch(shg_engine *e, const shg_params *p, const uint64_t *d_fir
     // runs. The pinned block is then taken before the splits, with room for descriptor words
     // bounded by the fixed bits plus 8 unary bits per node; a longer stream (not seen in
     // practice) takes a new block after encoding.
-    // the work-queue schedule: bipartite leaves of up to 64 keys (other builds take the level schedule)
-    // (the default schedule for these builds: measured faster than the level schedule on B200)
-    const bool queue = (p->mode == SHG_MODE_QUEUE || p->mode == SHG_MODE_DEFAULT) && p->variant == SHG_SHOCKHASH2 &&
-                       p->leaf_size <= 64;
+    // The work-queue schedule: bipartite leaves of up to 64 keys (other builds take the level schedule). By
+    // default only in the middle of the range, where it hides the ends of the level launches without
+    // filling the chip many times: level / queue, 1,000 keys 0.55 / 1.39 ms, 300,000 keys 2.7 / 3.1, 1M
+    // keys 6.4 / 6.1, 10M keys 44.6 / 47.2, 20M keys 87.4 / 93.4. Its blocks hold the leaf search's shared
+    // memory and registers, 24 warps per SM, during the splits too, and the two codes share the
+    // instruction cache.
+    const bool queue = p->variant == SHG_SHOCKHASH2 && p->leaf_size <= 64 &&
+                       (p->mode == SHG_MODE_QUEUE || (p->mode == SHG_MODE_DEFAULT && n >= 600000 && n < 2500000));
     const Tuning tun = e->tuning_of(p->variant, p->leaf_size);
     // with per-bucket leaf groups, the queue kernel writes each bucket's retrieval keys and bits
     // straight into the pinned result block as the bucket's leaves finish
@@ -579,11 +584,25 @@ shg_status build_batch(shg_engine *e, const shg_params *p, const uint64_t *d_fir
         sh1_block = !is_rotation(p->variant) && (uint64_t)nleaves * 1024 <= (uint64_t)most * wpb * trials;
         leaf_grid = std::max(1, std::min<int>(most, (int)(sh1_block ? nleaves : (nleaves + wpb - 1) / wpb)));
     }
+    // Blocks per split node of a launch of `count` nodes (a node takes fewer if it expects few trials):
+    // enough for twelve grids of five blocks per SM. A launch of few nodes leaves SMs idle, and one of
+    // a few thousand still ends with its longest searches alone (trial counts are geometric). Split
+    // levels, one block per node / striped: 1,000 keys 0.61 / 0.10 ms, 30,000 keys 1.47 / 0.40, 300,000 keys
+    // 2.76 / 1.80, 1M keys 5.07 / 4.70; with four grids 1M takes 5.17, with 32 grids 3M 12.3 instead of 11.3.
+    auto stripes_of = [&](uint64_t count) -> uint32_t {
+        const uint64_t want = 12ull * 5 * e->sms;
+        return (uint32_t)std::min<uint64_t>(32, std::max<uint64_t>(1, want / std::max<uint64_t>(count, 1)));
+    };
+    if (!queue && leaf_off) {
+        CU(e->split_best.ensure(leaf_off * sizeof(SplitBest)));
+        CU(cudaMemsetAsync(e->split_best.p, 0, leaf_off * sizeof(SplitBest), s));
+    }
     auto split_range = [&](size_t lv, uint64_t a, uint64_t b, cudaStream_t st) {
         if (b <= a) return;
         launch_split_level(e->nodes.as<Node>(), d_ids + level_off[lv] + a, (uint32_t)(b - a), e->keys.as<uint64_t>(),
                            e->codes.as<uint64_t>(), p->max_trials, &misc->err, &misc->work[0], misc->split_kind,
-                           std::min<uint32_t>(maxsz, tab.level_max[lv]), tun.split, st);
+                           std::min<uint32_t>(maxsz, tab.level_max[lv]), tun.split, stripes_of(b - a),
+                           e->split_best.as<SplitBest>() + level_off[lv] + a, st);
         launches++;
     };
     auto leaf_range = [&](uint64_t a, uint64_t b, cudaStream_t st, int grid) {

@@ -168,11 +168,18 @@ struct Tuning {
 };
 bool split_tuning_valid(int spl, int threads, int round_div, int arith);
 constexpr int kTuningFlat = 4;  // tuning-table variant key of ShockHash2Flat<k> (leaf size = k)
+// What the blocks of a striped split search share about a node.
+struct SplitBest {
+    unsigned long long inv_best;  // ~ the smallest valid trial found so far (0: none)
+    unsigned int done, pad;       // blocks that are done searching
+};
 // work[0] += useful evaluations; kind_work[k] += the same per inner loop (k = compared thresholds
 // - 1, or 3 for the quarter split). max_m: no node of the launch has more keys.
+// stripes: blocks per node; with more than one, best holds a zeroed SplitBest per node of the launch.
 void launch_split_level(const Node *nodes, const uint32_t *ids, uint32_t count, uint64_t *keys,
                         uint64_t *codes, uint64_t max_trials, uint32_t *err, unsigned long long *work,
-                        unsigned long long *kind_work, uint32_t max_m, const SplitTuning &t, cudaStream_t s);
+                        unsigned long long *kind_work, uint32_t max_m, const SplitTuning &t, uint32_t stripes,
+                        SplitBest *best, cudaStream_t s);
 int leaves_sh1_warps_per_block();
 // Inner-loop peaks of the bipartite leaf search (kind 0 scan, 1 pair filter, 2 pseudoforest edges),
 // 256-thread blocks; operations per thread and iteration from sh2_op_peak_per_iter.

@@ -4,26 +4,30 @@
 
 namespace shg {
 
-template <int SPL, int THREADS, bool SIMD>
+template <int SPL, int THREADS, bool SIMD, bool STRIPED>
 __global__ void __launch_bounds__(THREADS) k_split(const Node *__restrict__ nodes, const uint32_t *__restrict__ ids,
                                                    uint64_t *__restrict__ keys, uint64_t *__restrict__ codes,
                                                    uint64_t max_trials, uint32_t *__restrict__ err,
                                                    unsigned long long *__restrict__ work,
-                                                   unsigned long long *__restrict__ kind_work, int round_div) {
+                                                   unsigned long long *__restrict__ kind_work, int round_div,
+                                                   uint32_t stripes, SplitBest *best) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
     SplitSmem<SPL, THREADS, SIMD> &sm = *reinterpret_cast<SplitSmem<SPL, THREADS, SIMD> *>(smem_raw);
-    const uint32_t id = ids[blockIdx.x];
-    split_node<SPL, THREADS, SIMD>(sm, nodes[id], id, keys, codes, max_trials, err, work, kind_work, round_div);
+    const uint32_t i = STRIPED ? blockIdx.x / stripes : blockIdx.x;
+    const uint32_t id = ids[i];
+    split_node<SPL, THREADS, SIMD, false, STRIPED>(sm, nodes[id], id, keys, codes, max_trials, err, work, kind_work, round_div,
+                                                   SplitStripe{blockIdx.x - i * stripes, stripes, best + i});
 }
 
 template <int SPL, int THREADS, bool SIMD>
 static void launch_split_t(const Node *nodes, const uint32_t *ids, uint32_t count, uint64_t *keys, uint64_t *codes,
                            uint64_t max_trials, uint32_t *err, unsigned long long *work, unsigned long long *kind_work,
-                           uint32_t max_m, int round_div, cudaStream_t s) {
+                           uint32_t max_m, int round_div, uint32_t stripes, SplitBest *best, cudaStream_t s) {
     const size_t smem = split_smem_bytes<SPL, THREADS, SIMD>(max_m);
-    cudaFuncSetAttribute(k_split<SPL, THREADS, SIMD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_split<SPL, THREADS, SIMD><<<count, THREADS, smem, s>>>(nodes, ids, keys, codes, max_trials, err, work, kind_work,
-                                                             round_div);
+    auto kernel = stripes > 1 ? k_split<SPL, THREADS, SIMD, true> : k_split<SPL, THREADS, SIMD, false>;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    kernel<<<count * stripes, THREADS, smem, s>>>(nodes, ids, keys, codes, max_trials, err, work, kind_work, round_div, stripes,
+                                                  best);
 }
 
 // Parameters a tuning table may set (the SIMDShockHash form is chosen by the engine, not the table).
@@ -34,21 +38,21 @@ bool split_tuning_valid(int spl, int threads, int round_div, int arith) {
 
 void launch_split_level(const Node *nodes, const uint32_t *ids, uint32_t count, uint64_t *keys, uint64_t *codes,
                         uint64_t max_trials, uint32_t *err, unsigned long long *work, unsigned long long *kind_work,
-                        uint32_t max_m, const SplitTuning &t, cudaStream_t s) {
+                        uint32_t max_m, const SplitTuning &t, uint32_t stripes, SplitBest *best, cudaStream_t s) {
     if (!count) return;
     const bool simd = t.arith == kSplitArithSimd;
 #define SHG_SPLIT_CASE(SPL, TH)                                                                                      \
     if (t.spl == SPL && t.threads == TH)                                                                            \
         return simd ? launch_split_t<SPL, TH, true>(nodes, ids, count, keys, codes, max_trials, err, work, kind_work, \
-                                                    max_m, t.round_div, s)                                          \
+                                                    max_m, t.round_div, stripes, best, s)                                          \
                     : launch_split_t<SPL, TH, false>(nodes, ids, count, keys, codes, max_trials, err, work, kind_work, \
-                                                     max_m, t.round_div, s);
+                                                     max_m, t.round_div, stripes, best, s);
     SHG_SPLIT_CASE(1, 128) SHG_SPLIT_CASE(1, 256) SHG_SPLIT_CASE(1, 512)
     SHG_SPLIT_CASE(2, 128) SHG_SPLIT_CASE(2, 256) SHG_SPLIT_CASE(2, 512)
     SHG_SPLIT_CASE(4, 128) SHG_SPLIT_CASE(4, 256) SHG_SPLIT_CASE(4, 512)
 #undef SHG_SPLIT_CASE
     launch_split_level(nodes, ids, count, keys, codes, max_trials, err, work, kind_work, max_m,
-                       SplitTuning{2, 256, t.round_div, t.arith}, s);  // other values: the default shape
+                       SplitTuning{2, 256, t.round_div, t.arith}, stripes, best, s);  // other values: the default shape
 }
 
 } // namespace shg

@@ -69,6 +69,8 @@ template <int SPL, int THREADS, bool SIMD> struct SplitSmem {
     uint32_t part_counts[kWarps][32 * SPL][3];
     uint64_t scan[kWarps];
     uint32_t best[2];   // smallest valid seed slot of a round, by the round's parity
+    uint32_t stop[2];   // striped search: no smaller seed can come from this block's next rounds
+    uint64_t found;     // striped search, in the node's last block: the smallest seed of all its blocks
     uint32_t room;      // smallest seed_room of the staged keys
     SplitKey<SIMD> keys[kMaxBucket];  // last: a launch takes memory for the keys of its largest node only
 };
@@ -199,13 +201,23 @@ template <class Smem> __device__ __forceinline__ void merge_room(Smem &sm, uint3
     if ((threadIdx.x & 31) == 0 && room < kSeedSpan) atomicMin(&sm.room, room);
 }
 
+// A node searched by several blocks (its stripes): block `index` of `count` takes every count-th round and
+// stops once its next round begins past the smallest valid seed that any of them has found. So every
+// smaller seed has been tried when the last of them is done, and that block (nobody waits for another)
+// partitions the node.
+struct SplitStripe {
+    uint32_t index, count;
+    SplitBest *node;  // zero before the launch
+};
+
 // Smallest valid trial index (seed - seed0), or ~0 when `cap` trials were exhausted. The keys are
 // staged for seeds seed0 + base0, base0 + 1, ... (base0: 0 on entry, moved on when a key's low bits run
-// over). NT = number of part thresholds compared (1..3); NT = 4 selects the quarter split.
-template <int NT, int SPL, int THREADS, bool SIMD>
+// over). NT = number of part thresholds compared (1..3); NT = 4 selects the quarter split. STRIPED: the
+// smallest among this block's rounds, or ~0 when another block's seed makes the search end.
+template <int NT, bool STRIPED, int SPL, int THREADS, bool SIMD>
 __device__ __forceinline__ uint64_t search_seeds(SplitSmem<SPL, THREADS, SIMD> &sm, uint32_t m, const uint32_t T0, const uint32_t T1,
                                  const uint32_t T2, const uint32_t N0, const uint32_t N1, const uint32_t N2, int G,
-                                 uint64_t cap, uint64_t &base0) {
+                                 uint64_t cap, uint64_t &base0, const SplitStripe &stripe) {
     constexpr int kWarps = THREADS / 32, kSeedsPerWarp = 32 * SPL;
     constexpr int NC = NT == 4 ? 1 : NT;  // counters per seed
     const uint32_t need[3] = {N0, N1, N2};
@@ -216,7 +228,8 @@ __device__ __forceinline__ uint64_t search_seeds(SplitSmem<SPL, THREADS, SIMD> &
     const uint32_t per_round = (uint32_t)(kSeedsPerWarp * G);
     const uint32_t slot0 = (uint32_t)group * kSeedsPerWarp + lane;  // seed slot s is slot0 + 32 s
     uint32_t room = sm.room, parity = 0;
-    for (uint64_t base = 0; base < cap; base += per_round) {
+    const uint64_t step = STRIPED ? (uint64_t)per_round * stripe.count : per_round;
+    for (uint64_t base = STRIPED ? (uint64_t)per_round * stripe.index : 0; base < cap; base += step) {
         uint32_t c[SPL][3] = {};
         const uint64_t at = base - base0;
         const bool plain = at + per_round > room;
@@ -249,23 +262,26 @@ __device__ __forceinline__ uint64_t search_seeds(SplitSmem<SPL, THREADS, SIMD> &
                 if (ok) atomicMin(&sm.best[parity], slot0 + 32u * s);
             }
         }
+        if (STRIPED && threadIdx.x == 0)
+            sm.stop[parity] = ~*(volatile unsigned long long *)&stripe.node->inv_best <= base + step;
         __syncthreads();
         const uint32_t b = sm.best[parity];
         if (b != 0xffffffffu) return base + b < cap ? base + b : ~0ull;  // at most `cap` seeds count
+        if (STRIPED && sm.stop[parity]) return ~0ull;
         parity ^= 1;  // a warp that is ahead writes the other word while this one is still read
         if (plain) {  // stage the keys again from the next round's first seed on
             if (threadIdx.x == 0) sm.room = kSeedSpan;
             __syncthreads();
             uint32_t mine = kSeedSpan;
             for (uint32_t i = threadIdx.x; i < m; i += THREADS) {
-                const uint64_t z = sm.keys[i].z() + at + per_round;
+                const uint64_t z = sm.keys[i].z() + at + step;
                 sm.keys[i] = SplitKey<SIMD>::make(z);
                 mine = min(mine, seed_room(z));
             }
             merge_room(sm, mine);
             __syncthreads();
             room = sm.room;
-            base0 = base + per_round;
+            base0 = base + step;
         }
     }
     return ~0ull;
@@ -277,12 +293,14 @@ __device__ __forceinline__ uint64_t search_seeds(SplitSmem<SPL, THREADS, SIMD> &
 // whose search reaches its trial cap sets kErrTrialLimit and leaves its keys as they were.
 // L2: load the node's keys past L1 (needed when another SM may have rewritten them since this SM
 // last read those lines, as in the work-queue kernel; the per-level launches start with clean L1s).
-template <int SPL, int THREADS, bool SIMD, bool L2 = false>
+// STRIPED: the calling block is one stripe of the node's search.
+template <int SPL, int THREADS, bool SIMD, bool L2 = false, bool STRIPED = false>
 __device__ __forceinline__ void split_node(SplitSmem<SPL, THREADS, SIMD> &sm, const Node nd, const uint32_t id,
                                            uint64_t *__restrict__ keys, uint64_t *__restrict__ codes,
                                            const uint64_t max_trials, uint32_t *__restrict__ err,
                                            unsigned long long *__restrict__ work,
-                                           unsigned long long *__restrict__ kind_work, const int round_div) {
+                                           unsigned long long *__restrict__ kind_work, const int round_div,
+                                           SplitStripe stripe = SplitStripe{0, 1, nullptr}) {
     constexpr int kWarps = THREADS / 32, kSeedsPerWarp = 32 * SPL;
     const uint32_t m = nd.m;
     const uint64_t seed0 = start_seed(nd.level);
@@ -321,8 +339,14 @@ __device__ __forceinline__ void split_node(SplitSmem<SPL, THREADS, SIMD> &sm, co
         sp *= sqrt((double)(m - (uint32_t)NT * nd.unit));
         p = sqrt((double)m) / (pow(2 * M_PI, NT / 2.0) * sp);
     }
-    // Warp groups: aim for a round of ~1/round_div of the expected trials.
-    const double expect = 1.0 / p;
+    // Warp groups: aim for a round (of all stripes together) of ~1/round_div of the expected trials. A stripe
+    // for which fewer than two rounds of the smallest size are expected takes no part.
+    double expect = 1.0 / p;
+    if constexpr (STRIPED) {
+        stripe.count = min(stripe.count, max(1u, (uint32_t)(expect / (2 * kSeedsPerWarp))));
+        if (stripe.index >= stripe.count) return;
+        expect /= stripe.count;
+    }
     int G = 1;
     while (G < kWarps && (double)(kSeedsPerWarp * G * 2) * (double)round_div <= expect) G <<= 1;
     __syncthreads();
@@ -338,10 +362,23 @@ __device__ __forceinline__ void split_node(SplitSmem<SPL, THREADS, SIMD> &sm, co
         need[0] = quarter_need(nd.unit);
     }
     switch (NT) {
-        case 1: trial = search_seeds<1, SPL, THREADS, SIMD>(sm, m, T[0], T[1], T[2], need[0], need[1], need[2], G, cap, base0); break;
-        case 2: trial = search_seeds<2, SPL, THREADS, SIMD>(sm, m, T[0], T[1], T[2], need[0], need[1], need[2], G, cap, base0); break;
-        case 3: trial = search_seeds<3, SPL, THREADS, SIMD>(sm, m, T[0], T[1], T[2], need[0], need[1], need[2], G, cap, base0); break;
-        default: trial = search_seeds<4, SPL, THREADS, SIMD>(sm, m, T[0], T[1], T[2], need[0], need[1], need[2], G, cap, base0); break;
+        case 1: trial = search_seeds<1, STRIPED>(sm, m, T[0], T[1], T[2], need[0], need[1], need[2], G, cap, base0, stripe); break;
+        case 2: trial = search_seeds<2, STRIPED>(sm, m, T[0], T[1], T[2], need[0], need[1], need[2], G, cap, base0, stripe); break;
+        case 3: trial = search_seeds<3, STRIPED>(sm, m, T[0], T[1], T[2], need[0], need[1], need[2], G, cap, base0, stripe); break;
+        default: trial = search_seeds<4, STRIPED>(sm, m, T[0], T[1], T[2], need[0], need[1], need[2], G, cap, base0, stripe); break;
+    }
+    if constexpr (STRIPED) {
+        if (threadIdx.x == 0) {
+            if (trial != ~0ull) atomicMax(&stripe.node->inv_best, ~trial);
+            __threadfence();  // the seed before the count of finished blocks
+            const bool last = atomicAdd(&stripe.node->done, 1u) == stripe.count - 1;
+            __threadfence();
+            sm.stop[0] = last;
+            if (last) sm.found = ~atomicMax(&stripe.node->inv_best, 0ull);
+        }
+        __syncthreads();
+        if (!sm.stop[0]) return;
+        trial = sm.found;
     }
     if (trial == ~0ull) {
         if (threadIdx.x == 0) atomicOr(err, kErrTrialLimit);
