@@ -75,19 +75,20 @@ __global__ void __launch_bounds__(kPeakThreads) k_int_peak_sh1(uint64_t iters, u
     sink[blockIdx.x * (uint64_t)blockDim.x + threadIdx.x] = hits;
 }
 
-// The arithmetic of the bipartite leaf search's raw-seed loop: remix, fastrange64 to the half
-// table (as the kernel computes it for a range below 2^32), one bit into a 64-bit mask; two seeds
-// per lane.
-__global__ void __launch_bounds__(kPeakThreads) k_int_peak_sh2(uint64_t iters, uint64_t half, unsigned long long *sink) {
-    const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    uint64_t k0 = shg::remix(tid * 0x9E3779B97F4A7C15ULL), k1 = shg::remix(k0);
-    const uint64_t x0 = 0x643e521ddbd2be98ULL + tid;
-    uint64_t a0 = 0, a1 = 0;
-    for (uint64_t i = 0; i < iters; i++) {
-        a0 |= 1ull << shg::fastrange64_32(shg::remix(k0 + x0 + i), (uint32_t)half);
-        a1 |= 1ull << shg::fastrange64_32(shg::remix(k1 + x0 + i), (uint32_t)half);
+// The bipartite leaf search's raw-seed hashing alone: 64 staged keys, two seeds per lane, the same arithmetic
+// as the original leaves' first sieve (high product word, range reduction, one bit into a 32-bit mask).
+__global__ void __launch_bounds__(kPeakThreads) k_int_peak_sh2(uint64_t iters, uint32_t half, unsigned long long *sink) {
+    __shared__ shg::SeedKey keys[64];
+    for (int i = threadIdx.x; i < 64; i += blockDim.x)
+        keys[i] = shg::seed_key(shg::remix(0x9E3779B97F4A7C15ULL * (i + 1) + blockIdx.x) & ~(uint64_t)(shg::kSeedSpan - 1));
+    __syncthreads();
+    uint32_t at = (threadIdx.x >> 5) * 64 + (threadIdx.x & 31), out = 0;
+    for (uint64_t done = 0; done < iters; done += 64, at = (at + 512) & (shg::kSeedSpan / 2 - 1)) {
+        uint32_t mask[2] = {0, 0}, low[2] = {~0u, ~0u};
+        shg::sh1_half_masks<2>(keys, 64, half, at, mask, low);
+        out ^= mask[0] ^ mask[1] ^ low[0] ^ low[1];
     }
-    sink[tid] = a0 ^ a1;
+    sink[blockIdx.x * (uint64_t)blockDim.x + threadIdx.x] = out;
 }
 
 } // namespace
@@ -208,7 +209,9 @@ int shg_int_peak_kind(int device, int kind, uint64_t iters, double *evals_per_s,
         per_iter = shg::sh2_op_peak_per_iter(6);
     } else if (kind == 1) {
         timed_iters = (iters + 39) / 40 * 40;  // whole rounds of the 40-key leaf
-    } else if (kind != 2) {
+    } else if (kind == 2) {
+        timed_iters = (iters + 63) / 64 * 64;  // whole rounds of the 64-key leaf
+    } else {
         timed_iters = (iters + kPeakKeys - 1) / kPeakKeys * kPeakKeys;  // whole rounds of the split loops' keys
     }
     *evals_per_s = per_iter * (double)timed_iters * blocks * kPeakThreads / (ms * 1e-3);

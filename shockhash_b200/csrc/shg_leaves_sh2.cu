@@ -77,17 +77,13 @@ template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile(
 
 template <int MAXM> struct alignas(16) Sh2Smem {  // 16-byte aligned per warp: the masks are read 16 bytes at a time
     using C = Sh2Cfg<MAXM>;
-    uint64_t keys[MAXM];  // finder order (QuadSplit: even keys in order, odd keys from the back)
-    uint64_t orig[MAXM];  // leaf order
+    SeedKey keys[MAXM];  // finder order (QuadSplit: even keys in order, odd keys from the back), staged for seed 0
     MaskPair<typename C::Mask> mask[C::SMS];
     uint32_t csa[C::CMS], csb[C::CMS];           // raw seeds (seedA, seedB) of each candidate
     uint64_t iso[C::CMS][C::ISO_WORDS];          // isolated-key masks
     uint8_t uf[MAXM * 32];                       // per-lane union-find parents / per-lane hash rows
     uint32_t surv[64];                           // survivor queue: j << 16 | i
     uint32_t nsurv;
-    uint8_t c1[MAXM], c2[MAXM];                  // retrieval cuckoo insertion
-    int16_t cell[MAXM];
-    uint8_t xr[MAXM];
     MaskRing<typename C::Mask, C::RING> ring;
 };
 
@@ -181,23 +177,71 @@ template <int MAXM> struct LaneUF2 {
     }
 };
 
-__device__ bool cuckoo_insert2(int16_t *cell, uint8_t *xr, int e, uint32_t c1, uint32_t c2, int limit) {
-    xr[e] = (uint8_t)(c1 ^ c2);
-    if (cell[c1] < 0) { cell[c1] = (int16_t)e; return true; }
-    if (cell[c2] < 0) { cell[c2] = (int16_t)e; return true; }
-    uint32_t cur = c1;
-    const uint32_t orig_cell = cur;
-    int entry = e;
-    for (int step = 0; step < limit; step++) {
-        const uint32_t alt = xr[entry] ^ cur;
-        const int displaced = cell[alt];
-        cell[alt] = (int16_t)entry;
-        entry = displaced;
-        if (entry < 0) return true;
-        cur = alt;
-        if (cur == orig_cell && entry == e) return false;
+// Leaves whose seed is found but whose retrieval bits are not written yet: lane i of the warp holds
+// entry i. The ordered insertion that gives the bits is one serial chain per leaf, so a warp saves up
+// kInsert leaves and walks their chains side by side, one per lane, in the idle union-find area.
+constexpr int kInsert = 8;
+struct PendingLeaves {
+    uint32_t start = 0, m = 0;
+    uint64_t answer = 0;
+    int n = 0;  // the same in every lane
+};
+
+// Retrieval bits of the pending leaves (constructRetrieval, ShockHash2-internal.h:548-572): ordered
+// cuckoo insertion of the leaf keys in leaf order; bit 1 when a key rests in its seed2 cell.
+template <int MAXM, bool L2>
+__device__ __noinline__ void sh2_insert(PendingLeaves &pend, const uint64_t *__restrict__ keys, uint8_t *__restrict__ rib_bits,
+                                        uint8_t *__restrict__ area, int lane, uint32_t quad_min, uint32_t *__restrict__ err) {
+    // [key or cell][slot], one byte each: both cells of every key, the key in every cell (0xFF: none)
+    uint8_t *const c1 = area, *const c2 = area + MAXM * kInsert, *const cell = area + 2 * MAXM * kInsert;
+    constexpr uint32_t kNone = 0xFF;
+    __syncwarp();
+    for (uint32_t i = lane; i < MAXM * kInsert / 4; i += 32) reinterpret_cast<uint32_t *>(cell)[i] = ~0u;
+    for (int i = 0; i < pend.n; i++) {
+        const uint32_t start = __shfl_sync(0xffffffffu, pend.start, i), m = __shfl_sync(0xffffffffu, pend.m, i);
+        const uint64_t answer = __shfl_sync(0xffffffffu, pend.answer, i);
+        uint64_t s1, s2;
+        unpair_triangular(answer, s1, s2);
+        for (uint32_t k = lane; k < m; k += 32) {
+            const uint64_t key = L2 ? __ldcg(&keys[start + k]) : keys[start + k];
+            c1[k * kInsert + i] = (uint8_t)(sh2_cand_hash(key, s1, m, m >= quad_min) + m / 2);
+            c2[k * kInsert + i] = (uint8_t)sh2_cand_hash(key, s2, m, m >= quad_min);
+        }
     }
-    return false;
+    __syncwarp();
+    if (lane < pend.n) {
+        const uint32_t m = pend.m, limit = 8 * m + 16;
+        bool ok = true;
+        for (uint32_t k = 0; k < m && ok; k++) {
+            const uint32_t a = c1[k * kInsert + lane], b = c2[k * kInsert + lane];
+            if (cell[a * kInsert + lane] == kNone) cell[a * kInsert + lane] = (uint8_t)k;
+            else if (cell[b * kInsert + lane] == kNone) cell[b * kInsert + lane] = (uint8_t)k;
+            else {
+                uint32_t cur = a, entry = k;
+                ok = false;
+                for (uint32_t step = 0; step < limit; step++) {
+                    const uint32_t alt = (uint32_t)(c1[entry * kInsert + lane] ^ c2[entry * kInsert + lane]) ^ cur;
+                    const uint32_t displaced = cell[alt * kInsert + lane];
+                    cell[alt * kInsert + lane] = (uint8_t)entry;
+                    entry = displaced;
+                    if (entry == kNone) {
+                        ok = true;
+                        break;
+                    }
+                    cur = alt;
+                    if (cur == a && entry == k) break;
+                }
+            }
+        }
+        if (!ok) atomicOr(err, kErrInternal);
+    }
+    __syncwarp();
+    for (int i = 0; i < pend.n; i++) {
+        const uint32_t start = __shfl_sync(0xffffffffu, pend.start, i), m = __shfl_sync(0xffffffffu, pend.m, i);
+        for (uint32_t k = lane; k < m; k += 32) rib_bits[start + k] = cell[c2[k * kInsert + i] * kInsert + i] == k ? 1 : 0;
+    }
+    pend.n = 0;
+    __syncwarp();
 }
 
 template <int MAXM> struct LeafCtx {
@@ -239,7 +283,7 @@ template <int MAXM> struct LeafCtx {
         }
         const uint64_t ja = csa(j), jb = csb(j), ia = csa(i), ib = csb(i);
         for (uint32_t k = 0; k < m; k++) {
-            const uint64_t key = sm.keys[k];
+            const uint64_t key = seed_key_z(sm.keys[k]);
             const bool inA = k < sizeA;
             const uint32_t u = half_hash(key, inA ? ja : jb, half) + off;
             const uint32_t v = half_hash(key, inA ? ia : ib, half);
@@ -293,13 +337,13 @@ struct LeafWork {
 // global scratch `g` and union-find `uf` are reused from leaf to leaf. Errors set bits of *err.
 // L2: read the leaf's keys past L1 (the work-queue kernel, where another SM's partition may have
 // rewritten them after this SM cached the lines).
-// SIDE_WORDS: hash whole 8-key words that lie on one side of the leaf without per-key selects
-// (measured faster inside the work-queue kernel, slower in the level schedule's leaf kernel).
-template <int MAXM, class Src, bool L2 = false, bool SIDE_WORDS = false>
+// The leaf's retrieval bits are left to sh2_insert: the caller runs it on what is still pending.
+template <int MAXM, class Src, bool L2 = false>
 __device__ __forceinline__ void sh2_leaf(const Src &src, uint32_t li, const uint64_t *__restrict__ keys,
                                          uint8_t *__restrict__ rib_bits, Sh2Smem<MAXM> &sm, Sh2Global<MAXM> &g,
                                          LaneUF2<MAXM> &uf, const int lane, const uint32_t smax, const uint32_t cmax,
-                                         const uint32_t quad_min, uint32_t *__restrict__ err, LeafWork &lw) {
+                                         const uint32_t quad_min, uint32_t *__restrict__ err, LeafWork &lw,
+                                         PendingLeaves &pend) {
     const unsigned below = (1u << lane) - 1;
     unsigned long long &w_evals = lw.evals, &w_pairs = lw.pairs, &w_filtered = lw.filtered, &w_edges = lw.edges,
                        &w_scan = lw.scan;
@@ -320,6 +364,7 @@ __device__ __forceinline__ void sh2_leaf(const Src &src, uint32_t li, const uint
     const uint32_t m = cx.m, half = cx.half;
 
     // keys in finder order (QuadSplitCandidateFinder ctor, ShockHash2-internal.h:397-407)
+    uint32_t room = kSeedSpan;  // raw seeds for which the staged keys are good
     {
         uint32_t evens = 0, odds = 0;
         for (uint32_t k0 = 0; k0 < m; k0 += 32) {
@@ -329,15 +374,18 @@ __device__ __forceinline__ void sh2_leaf(const Src &src, uint32_t li, const uint
             const unsigned be = __ballot_sync(0xffffffffu, k < m && even);
             const unsigned bo = __ballot_sync(0xffffffffu, k < m && !even);
             if (k < m) {
-                sm.orig[k] = key;
                 uint32_t pos = k;
                 if (cx.quad) pos = even ? evens + __popc(be & below) : m - 1 - (odds + __popc(bo & below));
-                sm.keys[pos] = key;
+                sm.keys[pos] = seed_key(key);
+                room = min(room, seed_room(key));
             }
             evens += __popc(be);
             odds += __popc(bo);
         }
         cx.sizeA = cx.quad ? evens : m;
+        // the last word's missing keys: any valid key, their cells are dropped
+        if (m + lane < ((m + 7) & ~7u)) sm.keys[m + lane] = seed_key(0);
+        room = __reduce_min_sync(0xffffffffu, room);
     }
     if (lane == 0) sm.nsurv = 0;
     __syncwarp();
@@ -394,33 +442,61 @@ __device__ __forceinline__ void sh2_leaf(const Src &src, uint32_t li, const uint
             Mask tA = 0, tB = 0;
             uint64_t *rrow = s < g.rawcap ? g.raw + s * (MAXM / 8) : nullptr;
             const uint32_t sizeA = cx.sizeA;
-            // eight independent hash chains per row word (keys 8w..8w+7; MAXM is a multiple of 8, so
-            // sm.keys[8w + 7] is in bounds, and the cells of keys past m are dropped)
-            for (uint32_t k0 = 0; k0 < m; k0 += 8) {
-                uint64_t word = 0;
-                if (SIDE_WORDS && k0 + 8 <= m && (k0 + 8 <= sizeA || k0 >= sizeA)) {
-                    // the whole word inside the leaf and on one side (the same in every lane)
-                    Mask w8 = 0;
+            // A cell is floor(remix * half / 2^64), and remix's high word is the product word t with its
+            // lowest bit perhaps flipped: so the cell is the high word of t * half + 2 * half unless that
+            // number's low word is below 3 * half (the flip moves it by half at most, remix's low word adds
+            // less than half). Then, about once in 20,000 rounds, the round is hashed in plain form.
+            uint32_t low = 0;
+            if (S + 32 <= room) {
+                low = ~0u;
+                const uint64_t range = half, bias = 2 * half;
+#pragma unroll 1
+                for (uint32_t k0 = 0; k0 < m; k0 += 8) {
+                    Mask bit[8];
+                    uint32_t w0 = 0, w1 = 0;
 #pragma unroll
                     for (uint32_t t = 0; t < 8; t++) {
-                        const uint32_t h = half_hash(sm.keys[k0 + t], s, half);
-                        w8 |= (Mask)1 << h;
-                        word |= (uint64_t)h << (8 * t);
+                        const uint64_t p = seed_hi_product(sm.keys[k0 + t], (uint32_t)s) * range + bias;
+                        const uint32_t h = (uint32_t)(p >> 32);
+                        low = min(low, (uint32_t)p);
+                        bit[t] = (Mask)1 << h;
+                        if (t < 4) w0 |= h << (8 * t);
+                        else w1 |= h << (8 * t - 32);
                     }
-                    if (k0 + 8 <= sizeA) tA |= w8;
-                    else tB |= w8;
-                } else {
+                    if (k0 + 8 <= m && (k0 + 8 <= sizeA || k0 >= sizeA)) {
+                        // the whole word inside the leaf and on one side (the same in every lane)
+                        const Mask w8 = bit[0] | bit[1] | bit[2] | bit[3] | bit[4] | bit[5] | bit[6] | bit[7];
+                        if (k0 >= sizeA) tB |= w8;
+                        else tA |= w8;
+                    } else {
 #pragma unroll
-                    for (uint32_t t = 0; t < 8; t++) {
-                        const uint32_t k = k0 + t;
-                        const uint32_t h = half_hash(sm.keys[k], s, half);
-                        const Mask bit = k < m ? (Mask)1 << h : (Mask)0;
-                        tA |= k < sizeA ? bit : (Mask)0;
-                        tB |= k < sizeA ? (Mask)0 : bit;
-                        word |= k < m ? (uint64_t)h << (8 * t) : 0ull;
+                        for (uint32_t t = 0; t < 8; t++) {
+                            if (k0 + t < sizeA) tA |= bit[t];
+                            else if (k0 + t < m) tB |= bit[t];
+                        }
+                        if (k0 + 8 > m) {
+                            const uint64_t keep = (1ull << (8 * (m - k0))) - 1;
+                            w0 &= (uint32_t)keep;
+                            w1 &= (uint32_t)(keep >> 32);
+                        }
                     }
+                    if (rrow) rrow[k0 >> 3] = (uint64_t)w1 << 32 | w0;
                 }
-                if (rrow) rrow[k0 >> 3] = word;
+            }
+            if (__any_sync(0xffffffffu, low < 3 * half)) {
+                tA = tB = 0;
+#pragma unroll 1
+                for (uint32_t k0 = 0; k0 < m; k0 += 8) {
+                    uint64_t word = 0;
+#pragma unroll 1
+                    for (uint32_t k = k0; k < min(m, k0 + 8); k++) {
+                        const uint32_t h = half_hash(seed_key_z(sm.keys[k]), s, half);
+                        if (k < sizeA) tA |= (Mask)1 << h;
+                        else tB |= (Mask)1 << h;
+                        word |= (uint64_t)h << (8 * (k - k0));
+                    }
+                    if (rrow) rrow[k0 >> 3] = word;
+                }
             }
             cx.mp(s) = MaskPair<typename LeafCtx<MAXM>::Mask>{tA, tB};
             w_evals += m;
@@ -434,6 +510,7 @@ __device__ __forceinline__ void sh2_leaf(const Src &src, uint32_t li, const uint
         // each lane's partners in scan order, in the union-find area (idle until this round's pair
         // tests; [entry][lane], one column per lane): A side in entries 0..kPartners-1, B side after
         constexpr uint32_t kPartners = MAXM / 4;
+        static_assert(3 * MAXM * kInsert <= sizeof(sm.uf), "pending insertions fit the union-find area");
         static_assert(2 * kPartners * 32 * sizeof(uint16_t) <= sizeof(sm.uf), "partner lists fit the union-find area");
         uint16_t *const plist = reinterpret_cast<uint16_t *>(sm.uf);
         if (live) w_scan += cx.quad ? s + 1 : 1;  // mask pairs this raw seed is tested against
@@ -751,7 +828,7 @@ __device__ __forceinline__ void sh2_leaf(const Src &src, uint32_t li, const uint
                 uint64_t seen1 = 0, seen2 = 0, word = 0;
                 uint64_t *row = c < g.rcap ? g.rows + (uint64_t)c * (MAXM / 8) : nullptr;
                 for (uint32_t k = 0; k < m; k++) {
-                    const uint32_t h = half_hash(sm.keys[k], k < cx.sizeA ? sa : sb, half);
+                    const uint32_t h = half_hash(seed_key_z(sm.keys[k]), k < cx.sizeA ? sa : sb, half);
                     sm.uf[k * 32 + lane] = (uint8_t)h;
                     word |= (uint64_t)h << (8 * (k & 7));
                     if ((k & 7) == 7 || k + 1 == m) {
@@ -828,25 +905,13 @@ __device__ __forceinline__ void sh2_leaf(const Src &src, uint32_t li, const uint
         return;
     }
 
-    // Retrieval bits (constructRetrieval, ShockHash2-internal.h:548-572): ordered cuckoo
-    // insertion of the leaf keys in leaf order; bit 1 when a key rests in its seed2 cell.
-    uint64_t s1, s2;
-    unpair_triangular(answer, s1, s2);
-    for (uint32_t k = lane; k < m; k += 32) {
-        sm.c1[k] = (uint8_t)(sh2_cand_hash(sm.orig[k], s1, m, cx.quad) + m / 2);
-        sm.c2[k] = (uint8_t)sh2_cand_hash(sm.orig[k], s2, m, cx.quad);
-        sm.cell[k] = -1;
-    }
-    __syncwarp();
-    if (lane == 0) {
-        bool okc = true;
-        for (uint32_t k = 0; k < m && okc; k++) okc = cuckoo_insert2(sm.cell, sm.xr, (int)k, sm.c1[k], sm.c2[k], 8 * (int)m + 16);
-        if (!okc) atomicOr(err, kErrInternal);
+    if (lane == pend.n) {
+        pend.start = start;
+        pend.m = m;
+        pend.answer = answer;
         *code_out = answer;
     }
-    __syncwarp();
-    for (uint32_t k = lane; k < m; k += 32) rib_bits[start + k] = sm.cell[sm.c2[k]] == (int16_t)k ? 1 : 0;
-    __syncwarp();
+    if (++pend.n == kInsert) sh2_insert<MAXM, L2>(pend, keys, rib_bits, sm.uf, lane, quad_min, err);
 }
 
 // MINB: blocks per SM the register allocation is bounded for (a tuning parameter; any value gives
@@ -869,13 +934,15 @@ __global__ void __launch_bounds__(128, MINB) k_leaves_sh2_v2(Src src, uint32_t c
     else g.carve(gbase, smax, cmax);
     LaneUF2<MAXM> uf{sm.uf, lane, 0, 0};
     LeafWork lw;
+    PendingLeaves pend;
     for (;;) {
         uint32_t li = 0;
         if (lane == 0) li = atomicAdd(next_leaf, 1u);
         li = __shfl_sync(0xffffffffu, li, 0);
         if (li >= count) break;
-        sh2_leaf<MAXM, Src>(src, li, keys, rib_bits, sm, g, uf, lane, smax, cmax, quad_min, err, lw);
+        sh2_leaf<MAXM, Src>(src, li, keys, rib_bits, sm, g, uf, lane, smax, cmax, quad_min, err, lw, pend);
     }
+    if (pend.n) sh2_insert<MAXM, false>(pend, keys, rib_bits, sm.uf, lane, quad_min, err);
     unsigned long long w_evals = lw.evals, w_pairs = lw.pairs, w_filtered = lw.filtered, w_edges = lw.edges,
                        w_scan = lw.scan;
     for (int o = 16; o; o >>= 1) {
@@ -1060,8 +1127,9 @@ __device__ void write_bucket_out(uint32_t b, const uint64_t *__restrict__ acc, c
 // register allocation apart from the leaf search's.
 __device__ __noinline__ void queue_leaf(const NodeLeaves &leaves, uint32_t li, const uint64_t *__restrict__ keys,
                                         uint8_t *__restrict__ rib_bits, Sh2Smem<64> &sm, Sh2Global<64> &g, LaneUF2<64> &uf,
-                                        int lane, uint32_t smax, uint32_t cmax, uint32_t *__restrict__ err, LeafWork &lw) {
-    sh2_leaf<64, NodeLeaves, true, true>(leaves, li, keys, rib_bits, sm, g, uf, lane, smax, cmax, kQuadMinRecSplit, err, lw);
+                                        int lane, uint32_t smax, uint32_t cmax, uint32_t *__restrict__ err, LeafWork &lw,
+                                        PendingLeaves &pend) {
+    sh2_leaf<64, NodeLeaves, true>(leaves, li, keys, rib_bits, sm, g, uf, lane, smax, cmax, kQuadMinRecSplit, err, lw, pend);
 }
 
 template <int SPL>
@@ -1084,6 +1152,7 @@ __global__ void __launch_bounds__(kQueueThreads, 3)
     g.carve(scratch + ((uint64_t)blockIdx.x * kQueueWarps + warp) * scratch_per_warp, smax, cmax);
     LaneUF2<64> uf{sm.uf, lane, 0, 0};
     LeafWork lw;
+    PendingLeaves pend;
     const NodeLeaves leaves{nodes, ids + nsplit, codes};
     const uint32_t *leaf_col = offs + (uint64_t)kColLeaves * stride;
     const uint32_t nitems = *nitems_p;
@@ -1128,8 +1197,9 @@ __global__ void __launch_bounds__(kQueueThreads, 3)
                     atomicOr(err, kErrInternal);
                 __syncwarp();
             }
-            queue_leaf(leaves, li, keys, rib_bits, sm, g, uf, lane, smax, cmax, err, lw);
+            queue_leaf(leaves, li, keys, rib_bits, sm, g, uf, lane, smax, cmax, err, lw, pend);
         }
+        if (pend.n) sh2_insert<64, true>(pend, keys, rib_bits, sm.uf, lane, kQuadMinRecSplit, err);
         if (!group) break;
         __syncthreads();  // every warp is done with its Sh2Smem before a split node reuses the memory
         if (out) write_bucket_out(b, acc, keys, rib_bits, singles, offs + (uint64_t)kColSingles * stride, out, nreq);
