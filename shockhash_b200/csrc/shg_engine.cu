@@ -33,8 +33,10 @@ void launch_leaves_sh1_ctr(const Node *nodes, const uint32_t *ids, uint32_t coun
 void launch_leaves_sh2_ctr(const Node *nodes, const uint32_t *ids, uint32_t count, const uint64_t *keys, uint64_t *codes,
                            uint8_t *rib_bits, uint8_t *scratch, uint64_t scratch_per_warp, uint32_t smax, uint32_t cmax,
                            uint32_t *err, unsigned long long *work, unsigned int *ctr, int grid, cudaStream_t s,
-                           int max_leaf, uint32_t quad_min = kQuadMinRecSplit, int minb = 6);
+                           int max_leaf, uint32_t quad_min = kQuadMinRecSplit, int minb = 6, bool block = false);
 int sh2_smem_per_warp(int max_leaf);
+bool sh2_block_leaves(int max_leaf, uint64_t nleaves, uint64_t nkeys, int sms);
+int sh2_block_grid(int max_leaf, uint64_t nleaves, int sms);
 int leaves_sh1_warps_per_block();
 } // namespace shg
 
@@ -561,7 +563,7 @@ shg_status build_batch(shg_engine *e, const shg_params *p, const uint64_t *d_fir
     const uint32_t smax = maxm > 64 ? 16384 : 4096, cmax = maxm > 64 ? 16384 : 2048;
     const uint64_t per_warp = (sh2_scratch_bytes(smax, cmax, maxm) + 255) & ~255ull;
     int leaf_grid;
-    bool sh1_block = false;
+    bool sh1_block = false, sh2_block = false;
     if (sh2) {
         const int per_block_smem = 4 * sh2_smem_per_warp(maxm);
         int blocks_per_sm = std::max(1, std::min(8, (228 * 1024) / (per_block_smem + 1024)));
@@ -570,6 +572,8 @@ shg_status build_batch(shg_engine *e, const shg_params *p, const uint64_t *d_fir
         // the leaves latency bound, so the two interleave)
         const int bps = pipelined ? std::max(1, blocks_per_sm / 2) : blocks_per_sm;
         leaf_grid = p->mode == SHG_MODE_PER_LEAF ? 1 : std::max(1, std::min<int>(e->sms * bps, (int)((nleaves + 3) / 4)));
+        sh2_block = p->mode != SHG_MODE_PER_LEAF && !pipelined && sh2_block_leaves(maxm, nleaves, n, e->sms);
+        if (sh2_block) leaf_grid = sh2_block_grid(maxm, nleaves, e->sms);
     } else {
         const int wpb = leaves_sh1_warps_per_block();
         const int bps = tun.leaf_bps > 0 ? tun.leaf_bps : 8;
@@ -611,7 +615,7 @@ shg_status build_batch(shg_engine *e, const shg_params *p, const uint64_t *d_fir
             launch_leaves_sh2_ctr(e->nodes.as<Node>(), d_ids + leaf_off + a, (uint32_t)(b - a), e->keys.as<uint64_t>(),
                                   e->codes.as<uint64_t>(), e->rib_bits.as<uint8_t>(), e->scratch.as<uint8_t>(), per_warp, smax,
                                   cmax, &misc->err, misc->work, &misc->leaf_ctr, grid, st, maxm, kQuadMinRecSplit,
-                                  tun.leaf_minb);
+                                  tun.leaf_minb, sh2_block);
         else
             launch_leaves_sh1_ctr(e->nodes.as<Node>(), d_ids + leaf_off + a, (uint32_t)(b - a), e->keys.as<uint64_t>(),
                                   e->codes.as<uint64_t>(), e->rib_keys.as<uint64_t>(), e->rib_bits.as<uint8_t>(), p->max_trials,
@@ -1086,12 +1090,14 @@ shg_status build_flat(shg_engine *e, uint64_t k, const char *bytes, const uint64
         const Tuning ftun = e->tuning_of(kTuningFlat, (int)k);
         int bps = std::max(1, std::min(8, (228 * 1024) / (4 * sh2_smem_per_warp((int)k) + 1024)));
         if (ftun.leaf_bps > 0) bps = std::min(bps, ftun.leaf_bps);
-        const int grid = std::max(1, std::min<int>(e->sms * bps, (int)((nbuckets + 3) / 4)));
+        const bool block = sh2_block_leaves((int)k, nbuckets, leaf_n, e->sms);
+        const int grid = block ? sh2_block_grid((int)k, nbuckets, e->sms)
+                               : std::max(1, std::min<int>(e->sms * bps, (int)((nbuckets + 3) / 4)));
         CU(e->scratch.ensure(per_warp * (uint64_t)grid * 4));
         CU(cudaMemsetAsync(&misc->work[1], 0, 5 * sizeof(unsigned long long), s));  // the fallback build's counts
         launch_leaves_sh2_ctr(e->f_nodes.as<Node>(), e->f_ids.as<uint32_t>(), (uint32_t)nbuckets, e->f_leaf_keys.as<uint64_t>(),
                               e->f_codes.as<uint64_t>(), e->f_bits.as<uint8_t>(), e->scratch.as<uint8_t>(), per_warp, smax, cmax,
-                              &misc->err, misc->work, &misc->leaf_ctr, grid, s, (int)k, kQuadMinFlat, ftun.leaf_minb);
+                              &misc->err, misc->work, &misc->leaf_ctr, grid, s, (int)k, kQuadMinFlat, ftun.leaf_minb, block);
         CU(cudaGetLastError());
         CU(cudaMemcpyAsync(e->flat_work, &misc->work[1], sizeof(e->flat_work), cudaMemcpyDeviceToHost, s));
     } else {
@@ -1770,11 +1776,13 @@ shg_status shg_sh2_construct_leaves(shg_engine *e, const uint64_t *keys, const u
     const uint64_t per_warp = (sh2_scratch_bytes(smax, cmax, (int)maxm) + 255) & ~255ull;
     const int per_block_smem = 4 * sh2_smem_per_warp((int)maxm);
     const int blocks_per_sm = std::max(1, std::min(8, (228 * 1024) / (per_block_smem + 1024)));
-    const int grid = std::max(1, std::min<int>(e->sms * blocks_per_sm, (int)((nleaves + 3) / 4)));
+    const bool block = sh2_block_leaves((int)maxm, nleaves, n, e->sms);
+    const int grid = block ? sh2_block_grid((int)maxm, nleaves, e->sms)
+                           : std::max(1, std::min<int>(e->sms * blocks_per_sm, (int)((nleaves + 3) / 4)));
     CU(e->scratch.ensure(per_warp * (uint64_t)grid * 4));
     launch_leaves_sh2_ctr(e->nodes.as<Node>(), e->ids.as<uint32_t>(), (uint32_t)nleaves, e->keys.as<uint64_t>(),
                           e->codes.as<uint64_t>(), e->rib_bits.as<uint8_t>(), e->scratch.as<uint8_t>(), per_warp, smax, cmax,
-                          &misc->err, misc->work, &misc->leaf_ctr, grid, s, (int)maxm);
+                          &misc->err, misc->work, &misc->leaf_ctr, grid, s, (int)maxm, kQuadMinRecSplit, 6, block);
     CU(cudaGetLastError());
     uint32_t err = 0;
     CU(cudaMemcpyAsync(seeds, e->codes.p, nleaves * 8, cudaMemcpyDeviceToHost, s));

@@ -77,6 +77,7 @@ template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile(
 
 template <int MAXM> struct alignas(16) Sh2Smem {  // 16-byte aligned per warp: the masks are read 16 bytes at a time
     using C = Sh2Cfg<MAXM>;
+    static constexpr uint32_t kMasks = C::SMS, kCands = C::CMS;
     SeedKey keys[MAXM];  // finder order (QuadSplit: even keys in order, odd keys from the back), staged for seed 0
     MaskPair<typename C::Mask> mask[C::SMS];
     uint32_t csa[C::CMS], csb[C::CMS];           // raw seeds (seedA, seedB) of each candidate
@@ -244,20 +245,30 @@ __device__ __noinline__ void sh2_insert(PendingLeaves &pend, const uint64_t *__r
     __syncwarp();
 }
 
-template <int MAXM> struct LeafCtx {
+// One leaf's search state; Smem is Sh2Smem (a warp's) or Sh2BlockSmem (a block's).
+template <int MAXM_, class Smem = Sh2Smem<MAXM_>> struct LeafCtx {
+    static constexpr int MAXM = MAXM_;
     using Mask = typename Sh2Cfg<MAXM>::Mask;
-    Sh2Smem<MAXM> &sm;
+    Smem &sm;
     Sh2Global<MAXM> g;
     uint32_t m, half, sizeA, smax, cmax;
     Mask full;
     bool quad;
-    __device__ __forceinline__ MaskPair<Mask> &mp(uint64_t s) { return s < Sh2Cfg<MAXM>::SMS ? sm.mask[s] : g.mask[s]; }
+    __device__ __forceinline__ void set_size(uint32_t m_, uint32_t quad_min, uint32_t smax_, uint32_t cmax_) {
+        m = m_;
+        half = (m + 1) / 2;
+        full = half >= 8 * sizeof(Mask) ? ~(Mask)0 : (((Mask)1 << half) - 1);
+        quad = m >= quad_min;
+        smax = smax_;
+        cmax = cmax_;
+    }
+    __device__ __forceinline__ MaskPair<Mask> &mp(uint64_t s) { return s < Smem::kMasks ? sm.mask[s] : g.mask[s]; }
     __device__ __forceinline__ Mask maskA(uint64_t s) { return mp(s).a; }
     __device__ __forceinline__ Mask maskB(uint64_t s) { return mp(s).b; }
-    __device__ __forceinline__ uint32_t &csa(uint32_t j) { return j < Sh2Cfg<MAXM>::CMS ? sm.csa[j] : g.csa[j]; }
-    __device__ __forceinline__ uint32_t &csb(uint32_t j) { return j < Sh2Cfg<MAXM>::CMS ? sm.csb[j] : g.csb[j]; }
+    __device__ __forceinline__ uint32_t &csa(uint32_t j) { return j < Smem::kCands ? sm.csa[j] : g.csa[j]; }
+    __device__ __forceinline__ uint32_t &csb(uint32_t j) { return j < Smem::kCands ? sm.csb[j] : g.csb[j]; }
     __device__ __forceinline__ uint64_t &iso(uint32_t j, int w) {
-        return j < Sh2Cfg<MAXM>::CMS ? sm.iso[j][w] : g.iso[2 * (uint64_t)j + w];
+        return j < Smem::kCands ? sm.iso[j][w] : g.iso[2 * (uint64_t)j + w];
     }
     __device__ __forceinline__ uint64_t cseed(uint32_t j) {
         const uint32_t a = csa(j), b = csb(j);
@@ -293,6 +304,168 @@ template <int MAXM> struct LeafCtx {
         return true;
     }
 };
+
+// Hashes the leaf's keys under raw seed s (one per lane of a full warp): its two coverage masks, and its cell
+// row to the cache. staged: the staged keys are good for every lane's seed.
+template <class Cx>
+__device__ __forceinline__ void hash_raw_seeds(Cx &cx, uint64_t s, bool staged, typename Cx::Mask &tA, typename Cx::Mask &tB) {
+    using Mask = typename Cx::Mask;
+    constexpr int MAXM = Cx::MAXM;
+    tA = tB = 0;
+    uint64_t *rrow = s < cx.g.rawcap ? cx.g.raw + s * (MAXM / 8) : nullptr;
+    const uint32_t m = cx.m, half = cx.half, sizeA = cx.sizeA;
+    // A cell is floor(remix * half / 2^64), and remix's high word is the product word t with its
+    // lowest bit perhaps flipped: so the cell is the high word of t * half + 2 * half unless that
+    // number's low word is below 3 * half (the flip moves it by half at most, remix's low word adds
+    // less than half). Then, about once in 20,000 rounds, the round is hashed in plain form.
+    uint32_t low = 0;
+    if (staged) {
+        low = ~0u;
+        const uint64_t range = half, bias = 2 * half;
+#pragma unroll 1
+        for (uint32_t k0 = 0; k0 < m; k0 += 8) {
+            Mask bit[8];
+            uint32_t w0 = 0, w1 = 0;
+#pragma unroll
+            for (uint32_t t = 0; t < 8; t++) {
+                const uint64_t p = seed_hi_product(cx.sm.keys[k0 + t], (uint32_t)s) * range + bias;
+                const uint32_t h = (uint32_t)(p >> 32);
+                low = min(low, (uint32_t)p);
+                bit[t] = (Mask)1 << h;
+                if (t < 4) w0 |= h << (8 * t);
+                else w1 |= h << (8 * t - 32);
+            }
+            if (k0 + 8 <= m && (k0 + 8 <= sizeA || k0 >= sizeA)) {
+                // the whole word inside the leaf and on one side (the same in every lane)
+                const Mask w8 = bit[0] | bit[1] | bit[2] | bit[3] | bit[4] | bit[5] | bit[6] | bit[7];
+                if (k0 >= sizeA) tB |= w8;
+                else tA |= w8;
+            } else {
+#pragma unroll
+                for (uint32_t t = 0; t < 8; t++) {
+                    if (k0 + t < sizeA) tA |= bit[t];
+                    else if (k0 + t < m) tB |= bit[t];
+                }
+                if (k0 + 8 > m) {
+                    const uint64_t keep = (1ull << (8 * (m - k0))) - 1;
+                    w0 &= (uint32_t)keep;
+                    w1 &= (uint32_t)(keep >> 32);
+                }
+            }
+            if (rrow) rrow[k0 >> 3] = (uint64_t)w1 << 32 | w0;
+        }
+    }
+    if (__any_sync(0xffffffffu, low < 3 * half)) {
+        tA = tB = 0;
+#pragma unroll 1
+        for (uint32_t k0 = 0; k0 < m; k0 += 8) {
+            uint64_t word = 0;
+#pragma unroll 1
+            for (uint32_t k = k0; k < min(m, k0 + 8); k++) {
+                const uint32_t h = half_hash(seed_key_z(cx.sm.keys[k]), s, half);
+                if (k < sizeA) tA |= (Mask)1 << h;
+                else tB |= (Mask)1 << h;
+                word |= (uint64_t)h << (8 * (k - k0));
+            }
+            if (rrow) rrow[k0 >> 3] = word;
+        }
+    }
+}
+
+// The isolated-key mask of candidate c (calculateIsolatedVertices) and its cell row to the cache; uf: the
+// calling warp's union-find area, idle meanwhile.
+template <class Cx>
+__device__ __forceinline__ void candidate_iso(Cx &cx, uint32_t c, uint8_t *uf, int lane, unsigned long long &w_evals) {
+    constexpr int MAXM = Cx::MAXM;
+    const Sh2Global<MAXM> &g = cx.g;
+    const uint32_t m = cx.m, half = cx.half;
+    if (cx.csa(c) < g.rawcap && cx.csb(c) < g.rawcap) {
+        // cells from the two raw seeds' rows: set-A keys under seedA, set-B keys under seedB
+        const uint64_t *ra = g.raw + (uint64_t)cx.csa(c) * (MAXM / 8);
+        const uint64_t *rb = g.raw + (uint64_t)cx.csb(c) * (MAXM / 8);
+        uint64_t *row = c < g.rcap ? g.rows + (uint64_t)c * (MAXM / 8) : nullptr;
+        const uint32_t sizeA = cx.sizeA;
+        auto word_of = [&](uint32_t w) {  // cells of keys 8w..8w+7, one byte each
+            const uint32_t k0 = 8 * w;
+            uint64_t v;
+            if (k0 + 8 <= sizeA) v = ra[w];
+            else if (k0 >= sizeA) v = rb[w];
+            else {
+                const uint64_t keep = (1ull << (8 * (sizeA - k0))) - 1;
+                v = (ra[w] & keep) | (rb[w] & ~keep);
+            }
+            if (k0 + 8 > m) v &= (1ull << (8 * (m - k0))) - 1;
+            return v;
+        };
+        // the candidate's cell words go to its own column of the union-find area (idle until
+        // the pair tests) for the second pass; the next word's loads are issued before this
+        // word's stores, which would otherwise hold them back
+        uint64_t *const uw = reinterpret_cast<uint64_t *>(uf);  // [word][lane]
+        static_assert(MAXM / 8 * 32 * sizeof(uint64_t) <= MAXM * 32, "cell words fit the union-find area");
+        // cells are below (m + 1) / 2: 32-bit masks for leaves of up to 64 keys
+        using CMask = std::conditional_t<(MAXM <= 64), uint32_t, uint64_t>;
+        CMask seen1 = 0, seen2 = 0;
+        uint64_t v_next = word_of(0);
+#pragma unroll 1
+        for (uint32_t w = 0; 8 * w < m; w++) {
+            const uint64_t v = v_next;
+            if (8 * (w + 1) < m) v_next = word_of(w + 1);
+            uw[w * 32 + lane] = v;
+            if (row) row[w] = v;
+            const uint32_t kn = min(8u, m - 8 * w);
+#pragma unroll
+            for (uint32_t t = 0; t < 8; t++) {
+                if (t < kn) {
+                    const CMask bit = (CMask)1 << ((v >> (8 * t)) & 0xFF);
+                    seen2 |= seen1 & bit;
+                    seen1 |= bit;
+                }
+            }
+        }
+        const CMask single = seen1 & ~seen2;
+        uint64_t iso0 = 0, iso1 = 0;
+#pragma unroll 1
+        for (uint32_t w = 0; 8 * w < m; w++) {
+            const uint64_t v = uw[w * 32 + lane];
+            const uint32_t kn = min(8u, m - 8 * w);
+            uint64_t b8 = 0;
+#pragma unroll
+            for (uint32_t t = 0; t < 8; t++)
+                if (t < kn) b8 |= ((single >> ((v >> (8 * t)) & 0xFF)) & 1) << t;
+            const uint32_t k0 = 8 * w;
+            if (k0 < 64) iso0 |= b8 << k0; else iso1 |= b8 << (k0 - 64);
+        }
+        cx.iso(c, 0) = iso0;
+        if (Sh2Cfg<MAXM>::ISO_WORDS > 1) cx.iso(c, 1) = iso1;
+        w_evals += m;  // the reference hashes the candidate's keys here (makeCache)
+    } else {
+        const uint64_t sa = cx.csa(c), sb = cx.csb(c);
+        uint64_t seen1 = 0, seen2 = 0, word = 0;
+        uint64_t *row = c < g.rcap ? g.rows + (uint64_t)c * (MAXM / 8) : nullptr;
+        for (uint32_t k = 0; k < m; k++) {
+            const uint32_t h = half_hash(seed_key_z(cx.sm.keys[k]), k < cx.sizeA ? sa : sb, half);
+            uf[k * 32 + lane] = (uint8_t)h;
+            word |= (uint64_t)h << (8 * (k & 7));
+            if ((k & 7) == 7 || k + 1 == m) {
+                if (row) row[k >> 3] = word;
+                word = 0;
+            }
+            const uint64_t bit = 1ull << h;
+            seen2 |= seen1 & bit;
+            seen1 |= bit;
+        }
+        const uint64_t single = seen1 & ~seen2;
+        uint64_t iso0 = 0, iso1 = 0;
+        for (uint32_t k = 0; k < m; k++) {
+            const uint32_t h = uf[k * 32 + lane];
+            const uint64_t b = (single >> h) & 1;
+            if (k < 64) iso0 |= b << k; else iso1 |= b << (k - 64);
+        }
+        cx.iso(c, 0) = iso0;
+        if (Sh2Cfg<MAXM>::ISO_WORDS > 1) cx.iso(c, 1) = iso1;
+        w_evals += m;
+    }
+}
 
 // Where a leaf's keys and its output seed are: the engine's planned tree nodes...
 struct NodeLeaves {
@@ -354,14 +527,8 @@ __device__ __forceinline__ void sh2_leaf(const Src &src, uint32_t li, const uint
         return;
     }
     LeafCtx<MAXM> cx{sm, g};
-    cx.m = m_leaf;
-    cx.half = (cx.m + 1) / 2;
-    cx.full = cx.half >= 8 * sizeof(typename LeafCtx<MAXM>::Mask) ? ~(typename LeafCtx<MAXM>::Mask)0
-                                                                 : (((typename LeafCtx<MAXM>::Mask)1 << cx.half) - 1);
-    cx.quad = cx.m >= quad_min;
-    cx.smax = smax;
-    cx.cmax = cmax;
-    const uint32_t m = cx.m, half = cx.half;
+    cx.set_size(m_leaf, quad_min, smax, cmax);
+    const uint32_t m = cx.m;
 
     // keys in finder order (QuadSplitCandidateFinder ctor, ShockHash2-internal.h:397-407)
     uint32_t room = kSeedSpan;  // raw seeds for which the staged keys are good
@@ -438,66 +605,8 @@ __device__ __forceinline__ void sh2_leaf(const Src &src, uint32_t li, const uint
                 break;
             }
             const uint64_t s = S + lane;
-            using Mask = typename LeafCtx<MAXM>::Mask;
-            Mask tA = 0, tB = 0;
-            uint64_t *rrow = s < g.rawcap ? g.raw + s * (MAXM / 8) : nullptr;
-            const uint32_t sizeA = cx.sizeA;
-            // A cell is floor(remix * half / 2^64), and remix's high word is the product word t with its
-            // lowest bit perhaps flipped: so the cell is the high word of t * half + 2 * half unless that
-            // number's low word is below 3 * half (the flip moves it by half at most, remix's low word adds
-            // less than half). Then, about once in 20,000 rounds, the round is hashed in plain form.
-            uint32_t low = 0;
-            if (S + 32 <= room) {
-                low = ~0u;
-                const uint64_t range = half, bias = 2 * half;
-#pragma unroll 1
-                for (uint32_t k0 = 0; k0 < m; k0 += 8) {
-                    Mask bit[8];
-                    uint32_t w0 = 0, w1 = 0;
-#pragma unroll
-                    for (uint32_t t = 0; t < 8; t++) {
-                        const uint64_t p = seed_hi_product(sm.keys[k0 + t], (uint32_t)s) * range + bias;
-                        const uint32_t h = (uint32_t)(p >> 32);
-                        low = min(low, (uint32_t)p);
-                        bit[t] = (Mask)1 << h;
-                        if (t < 4) w0 |= h << (8 * t);
-                        else w1 |= h << (8 * t - 32);
-                    }
-                    if (k0 + 8 <= m && (k0 + 8 <= sizeA || k0 >= sizeA)) {
-                        // the whole word inside the leaf and on one side (the same in every lane)
-                        const Mask w8 = bit[0] | bit[1] | bit[2] | bit[3] | bit[4] | bit[5] | bit[6] | bit[7];
-                        if (k0 >= sizeA) tB |= w8;
-                        else tA |= w8;
-                    } else {
-#pragma unroll
-                        for (uint32_t t = 0; t < 8; t++) {
-                            if (k0 + t < sizeA) tA |= bit[t];
-                            else if (k0 + t < m) tB |= bit[t];
-                        }
-                        if (k0 + 8 > m) {
-                            const uint64_t keep = (1ull << (8 * (m - k0))) - 1;
-                            w0 &= (uint32_t)keep;
-                            w1 &= (uint32_t)(keep >> 32);
-                        }
-                    }
-                    if (rrow) rrow[k0 >> 3] = (uint64_t)w1 << 32 | w0;
-                }
-            }
-            if (__any_sync(0xffffffffu, low < 3 * half)) {
-                tA = tB = 0;
-#pragma unroll 1
-                for (uint32_t k0 = 0; k0 < m; k0 += 8) {
-                    uint64_t word = 0;
-#pragma unroll 1
-                    for (uint32_t k = k0; k < min(m, k0 + 8); k++) {
-                        const uint32_t h = half_hash(seed_key_z(sm.keys[k]), s, half);
-                        if (k < sizeA) tA |= (Mask)1 << h;
-                        else tB |= (Mask)1 << h;
-                        word |= (uint64_t)h << (8 * (k - k0));
-                    }
-                    if (rrow) rrow[k0 >> 3] = word;
-                }
-            }
+            typename LeafCtx<MAXM>::Mask tA, tB;
+            hash_raw_seeds(cx, s, S + 32 <= room, tA, tB);
             cx.mp(s) = MaskPair<typename LeafCtx<MAXM>::Mask>{tA, tB};
             w_evals += m;
             S += 32;
@@ -764,92 +873,7 @@ __device__ __forceinline__ void sh2_leaf(const Src &src, uint32_t li, const uint
         // 3. isolated-key masks of the new candidates (calculateIsolatedVertices), one per lane
         for (uint32_t c0 = J; c0 < J + T; c0 += 32) {
             const uint32_t c = c0 + lane;
-            if (c < J + T && cx.csa(c) < g.rawcap && cx.csb(c) < g.rawcap) {
-                // cells from the two raw seeds' rows: set-A keys under seedA, set-B keys under seedB
-                const uint64_t *ra = g.raw + (uint64_t)cx.csa(c) * (MAXM / 8);
-                const uint64_t *rb = g.raw + (uint64_t)cx.csb(c) * (MAXM / 8);
-                uint64_t *row = c < g.rcap ? g.rows + (uint64_t)c * (MAXM / 8) : nullptr;
-                const uint32_t sizeA = cx.sizeA;
-                auto word_of = [&](uint32_t w) {  // cells of keys 8w..8w+7, one byte each
-                    const uint32_t k0 = 8 * w;
-                    uint64_t v;
-                    if (k0 + 8 <= sizeA) v = ra[w];
-                    else if (k0 >= sizeA) v = rb[w];
-                    else {
-                        const uint64_t keep = (1ull << (8 * (sizeA - k0))) - 1;
-                        v = (ra[w] & keep) | (rb[w] & ~keep);
-                    }
-                    if (k0 + 8 > m) v &= (1ull << (8 * (m - k0))) - 1;
-                    return v;
-                };
-                // the candidate's cell words go to its own column of the union-find area (idle until
-                // the pair tests) for the second pass; the next word's loads are issued before this
-                // word's stores, which would otherwise hold them back
-                uint64_t *const uw = reinterpret_cast<uint64_t *>(sm.uf);  // [word][lane]
-                static_assert(MAXM / 8 * 32 * sizeof(uint64_t) <= sizeof(sm.uf), "cell words fit the union-find area");
-                // cells are below (m + 1) / 2: 32-bit masks for leaves of up to 64 keys
-                using CMask = std::conditional_t<(MAXM <= 64), uint32_t, uint64_t>;
-                CMask seen1 = 0, seen2 = 0;
-                uint64_t v_next = word_of(0);
-#pragma unroll 1
-                for (uint32_t w = 0; 8 * w < m; w++) {
-                    const uint64_t v = v_next;
-                    if (8 * (w + 1) < m) v_next = word_of(w + 1);
-                    uw[w * 32 + lane] = v;
-                    if (row) row[w] = v;
-                    const uint32_t kn = min(8u, m - 8 * w);
-#pragma unroll
-                    for (uint32_t t = 0; t < 8; t++) {
-                        if (t < kn) {
-                            const CMask bit = (CMask)1 << ((v >> (8 * t)) & 0xFF);
-                            seen2 |= seen1 & bit;
-                            seen1 |= bit;
-                        }
-                    }
-                }
-                const CMask single = seen1 & ~seen2;
-                uint64_t iso0 = 0, iso1 = 0;
-#pragma unroll 1
-                for (uint32_t w = 0; 8 * w < m; w++) {
-                    const uint64_t v = uw[w * 32 + lane];
-                    const uint32_t kn = min(8u, m - 8 * w);
-                    uint64_t b8 = 0;
-#pragma unroll
-                    for (uint32_t t = 0; t < 8; t++)
-                        if (t < kn) b8 |= ((single >> ((v >> (8 * t)) & 0xFF)) & 1) << t;
-                    const uint32_t k0 = 8 * w;
-                    if (k0 < 64) iso0 |= b8 << k0; else iso1 |= b8 << (k0 - 64);
-                }
-                cx.iso(c, 0) = iso0;
-                if (Sh2Cfg<MAXM>::ISO_WORDS > 1) cx.iso(c, 1) = iso1;
-                w_evals += m;  // the reference hashes the candidate's keys here (makeCache)
-            } else if (c < J + T) {
-                const uint64_t sa = cx.csa(c), sb = cx.csb(c);
-                uint64_t seen1 = 0, seen2 = 0, word = 0;
-                uint64_t *row = c < g.rcap ? g.rows + (uint64_t)c * (MAXM / 8) : nullptr;
-                for (uint32_t k = 0; k < m; k++) {
-                    const uint32_t h = half_hash(seed_key_z(sm.keys[k]), k < cx.sizeA ? sa : sb, half);
-                    sm.uf[k * 32 + lane] = (uint8_t)h;
-                    word |= (uint64_t)h << (8 * (k & 7));
-                    if ((k & 7) == 7 || k + 1 == m) {
-                        if (row) row[k >> 3] = word;
-                        word = 0;
-                    }
-                    const uint64_t bit = 1ull << h;
-                    seen2 |= seen1 & bit;
-                    seen1 |= bit;
-                }
-                const uint64_t single = seen1 & ~seen2;
-                uint64_t iso0 = 0, iso1 = 0;
-                for (uint32_t k = 0; k < m; k++) {
-                    const uint32_t h = sm.uf[k * 32 + lane];
-                    const uint64_t b = (single >> h) & 1;
-                    if (k < 64) iso0 |= b << k; else iso1 |= b << (k - 64);
-                }
-                cx.iso(c, 0) = iso0;
-                if (Sh2Cfg<MAXM>::ISO_WORDS > 1) cx.iso(c, 1) = iso1;
-                w_evals += m;
-            }
+            if (c < J + T) candidate_iso(cx, c, sm.uf, lane, w_evals);
         }
         __syncwarp();
         // 4. all pairs (j, i), J <= j < J+T, i < j, in lexicographic order
@@ -972,6 +996,321 @@ void launch_v2(const Node *nodes, const uint32_t *ids, uint32_t count, const uin
     k_leaves_sh2_v2<MAXM, NodeLeaves, MINB><<<grid, 128, smem, s>>>(NodeLeaves{nodes, ids, codes}, count, keys, rib_bits,
                                                                     scratch, scratch_per_warp, smax, cmax, err, work, ctr,
                                                                     quad_min);
+}
+
+// ------------------------------------------------------------------ a block per leaf
+// The same search with a block's W warps on one leaf: while a launch has few leaves for its warps, the
+// longest leaf sets its time (a 100-key leaf takes milliseconds on one warp). A round is 32 * W raw seeds,
+// one per thread; thread t lists the candidates of raw seed S + t, and warp w tests the w-th part of the
+// round's pairs, in order. The first passing pair of all parts is the answer, so the order in which
+// candidates and pairs count is the one of sh2_leaf.
+//
+// Eight warps for leaves of more than 64 keys, which take thousands of raw seeds: leaf stage of
+// ShockHash2Flat<100>, warp / block: 50 leaves 8.0 / 1.7 ms, 500 leaves 15.2 / 3.4, 5,000 leaves 22.9 / 14.1, 20,000
+// leaves 54.5 / 48.3. Four for smaller ones: 64-key leaves take about 150 raw seeds, so the rounds of a block
+// overshoot, and only launches of about one leaf per block gain (16 leaves 0.27 / 0.22 ms, 480 leaves 0.50 / 0.40,
+// 1,600 leaves 0.42 / 0.52).
+template <int MAXM> constexpr int kBlockLeafWarps = MAXM <= 64 ? 4 : 8;
+template <int MAXM> struct alignas(16) Sh2BlockSmem {
+    using C = Sh2Cfg<MAXM>;
+    static constexpr int W = kBlockLeafWarps<MAXM>;
+    static constexpr uint32_t kMasks = MAXM <= 64 ? 512 : 1536, kCands = 256;
+    SeedKey keys[MAXM];
+    MaskPair<typename C::Mask> mask[kMasks];
+    uint32_t csa[kCands], csb[kCands];
+    uint64_t iso[kCands][C::ISO_WORDS];
+    uint8_t uf[W][MAXM * 32];
+    uint32_t surv[W][64];
+    unsigned long long best;  // first passing pair of the round, j << 32 | i
+    uint32_t count[W], fits[W];  // candidates listed and raw seeds taken, per warp
+    uint32_t leaf, size_a, room, total;
+};
+
+template <int MAXM, class Src>
+__global__ void __launch_bounds__(kBlockLeafWarps<MAXM> * 32, 24 / kBlockLeafWarps<MAXM>) k_leaves_sh2_block(
+    Src src, uint32_t count, const uint64_t *__restrict__ keys, uint8_t *__restrict__ rib_bits, uint8_t *__restrict__ scratch,
+    uint64_t scratch_per_block, uint32_t smax, uint32_t cmax, uint32_t *__restrict__ err,
+    unsigned long long *__restrict__ work, unsigned int *__restrict__ next_leaf, uint32_t quad_min) {
+    using Smem = Sh2BlockSmem<MAXM>;
+    using Mask = typename Sh2Cfg<MAXM>::Mask;
+    constexpr int W = kBlockLeafWarps<MAXM>;
+    constexpr uint32_t NT = 32 * W;
+    extern __shared__ __align__(16) uint8_t smem_raw[];
+    Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t tid = threadIdx.x;
+    const unsigned below = (1u << lane) - 1;
+    LeafCtx<MAXM, Smem> cx{sm};
+    cx.g.carve(scratch + blockIdx.x * scratch_per_block, smax, cmax);
+    LaneUF2<MAXM> uf{sm.uf[warp], lane, 0, 0};
+    uint32_t *const surv = sm.surv[warp];
+    LeafWork lw;
+    PendingLeaves pend;  // warp 0's
+    for (;;) {
+        __syncthreads();  // the leaf before is done with the shared memory
+        if (tid == 0) sm.leaf = atomicAdd(next_leaf, 1u);
+        __syncthreads();
+        const uint32_t li = sm.leaf;
+        if (li >= count) break;
+        uint32_t start = 0, m = 0;
+        uint64_t *code_out = nullptr;
+        if (!src.get(li, start, m, code_out)) {
+            if (tid == 0) atomicOr(err, kErrArg);
+            continue;
+        }
+        cx.set_size(m, quad_min, smax, cmax);
+        if (warp == 0) {  // keys in finder order, as in sh2_leaf
+            uint32_t evens = 0, odds = 0, room = kSeedSpan;
+            for (uint32_t k0 = 0; k0 < m; k0 += 32) {
+                const uint32_t k = k0 + lane;
+                const uint64_t key = k < m ? keys[start + k] : 0;
+                const bool even = (key & 1) == 0;
+                const unsigned be = __ballot_sync(0xffffffffu, k < m && even);
+                const unsigned bo = __ballot_sync(0xffffffffu, k < m && !even);
+                if (k < m) {
+                    uint32_t pos = k;
+                    if (cx.quad) pos = even ? evens + __popc(be & below) : m - 1 - (odds + __popc(bo & below));
+                    sm.keys[pos] = seed_key(key);
+                    room = min(room, seed_room(key));
+                }
+                evens += __popc(be);
+                odds += __popc(bo);
+            }
+            if (m + lane < ((m + 7) & ~7u)) sm.keys[m + lane] = seed_key(0);
+            room = __reduce_min_sync(0xffffffffu, room);
+            if (lane == 0) {
+                sm.size_a = cx.quad ? evens : m;
+                sm.room = room;
+                sm.best = ~0ull;
+            }
+        }
+        __syncthreads();
+        cx.sizeA = sm.size_a;
+        const uint32_t room = sm.room;
+        const Mask full = cx.full;
+
+        uint32_t J = 0;               // candidates stored so far
+        uint64_t S = 0, S_proc = 0;   // raw seeds hashed, raw seeds listed
+        unsigned long long best = ~0ull;
+        bool overflow = false;
+        while (best == ~0ull) {
+            if (S_proc == S) {
+                if (S + NT > smax) {
+                    overflow = true;
+                    break;
+                }
+                const uint64_t s = S + tid;
+                Mask tA, tB;
+                hash_raw_seeds(cx, s, S + NT <= room, tA, tB);
+                cx.mp(s) = MaskPair<Mask>{tA, tB};
+                lw.evals += m;
+                S += NT;
+                __syncthreads();
+            }
+            // candidates whose larger raw seed is this thread's s
+            const uint64_t s = S_proc + tid;
+            const bool live = s < S;
+            uint32_t mineA = 0, mineB = 0, mine = 0;
+            constexpr uint32_t kPartners = MAXM / 4;  // per side, in the warp's union-find area: [entry][lane]
+            uint16_t *const plist = reinterpret_cast<uint16_t *>(sm.uf[warp]);
+            if (live) lw.scan += cx.quad ? s + 1 : 1;
+            if (cx.quad) {
+                const MaskPair<Mask> ts = live ? cx.mp(s) : MaskPair<Mask>{0, 0};
+                // no partner for a thread without a raw seed: nothing covers an empty half table
+                const Mask nA = live ? ~ts.a & full : ~(Mask)0, nB = live ? ~ts.b & full : ~(Mask)0;
+                auto visit = [&](uint64_t p, const MaskPair<Mask> &w) {
+                    if ((nB & ~w.a) == 0 && p < s && float_accurate_elegant_seeds(p, s)) {
+                        if (mineA < kPartners) plist[mineA * 32 + lane] = (uint16_t)p;
+                        mineA++;
+                    }
+                    if ((nA & ~w.b) == 0 && p <= s && float_accurate_elegant_seeds(s, p)) {
+                        if (mineB < kPartners) plist[(kPartners + mineB) * 32 + lane] = (uint16_t)p;
+                        mineB++;
+                    }
+                };
+                // every lane of a warp walks the same p, up to the warp's largest raw seed, eight at a time
+                auto walk = [&](const MaskPair<Mask> *masks, uint64_t p, uint64_t end) {
+                    for (; p + 8 <= end; p += 8) {
+                        MaskPair<Mask> w[8];
+#pragma unroll
+                        for (int u = 0; u < 8; u++) w[u] = masks[p + u];
+                        bool any = false;
+#pragma unroll
+                        for (int u = 0; u < 8; u++) any |= ((nB & ~w[u].a) == 0) | ((nA & ~w[u].b) == 0);
+                        if (any) {
+#pragma unroll 1
+                            for (int u = 0; u < 8; u++) visit(p + u, masks[p + u]);
+                        }
+                    }
+                    for (; p < end; p++) visit(p, masks[p]);
+                };
+                const uint64_t warp_end = min(S, S_proc + 32 * (warp + 1));
+                walk(sm.mask, 0, min(warp_end, (uint64_t)Smem::kMasks));
+                if (warp_end > Smem::kMasks) walk(cx.g.mask, Smem::kMasks, warp_end);
+                mine = mineA + mineB;
+            } else if (live) {
+                mine = cx.maskA(s) == full;
+            }
+            uint32_t incl = mine;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += y;
+            }
+            if (lane == 31) sm.count[warp] = incl;
+            __syncthreads();
+            for (int w = 0; w < warp; w++) incl += sm.count[w];
+            // the longest prefix of raw seeds whose candidates fit the candidate capacity
+            const uint32_t cap = min(cmax, 0xFFFFu);
+            const bool fit = live && J + incl <= cap;
+            const unsigned fits = __ballot_sync(0xffffffffu, fit);
+            if (lane == 0) sm.fits[warp] = __popc(fits);
+            if (tid == 0) sm.total = 0;
+            __syncthreads();
+            uint32_t take = 0;
+            for (int w = 0; w < W; w++) take += sm.fits[w];
+            if (tid + 1 == take) sm.total = incl;
+            if (fit) {
+                uint32_t pos = J + incl - mine;
+                if (cx.quad && mineA <= kPartners && mineB <= kPartners) {
+                    for (uint32_t t = 0; t < mineA; t++, pos++) {  // A side first: (a, s), a ascending
+                        cx.csa(pos) = plist[t * 32 + lane];
+                        cx.csb(pos) = (uint32_t)s;
+                    }
+                    for (uint32_t t = 0; t < mineB; t++, pos++) {  // then B side: (s, b), b ascending
+                        cx.csa(pos) = (uint32_t)s;
+                        cx.csb(pos) = plist[(kPartners + t) * 32 + lane];
+                    }
+                } else if (cx.quad) {  // more partners on a side than the lists hold: scan again
+                    const Mask tA = cx.maskA(s), tB = cx.maskB(s);
+                    for (uint64_t a = 0; a < s && mine; a++)
+                        if ((cx.maskA(a) | tB) == full && float_accurate_elegant_seeds(a, s)) {
+                            cx.csa(pos) = (uint32_t)a;
+                            cx.csb(pos) = (uint32_t)s;
+                            pos++;
+                        }
+                    for (uint64_t b = 0; b <= s && mine; b++)
+                        if ((cx.maskB(b) | tA) == full && float_accurate_elegant_seeds(s, b)) {
+                            cx.csa(pos) = (uint32_t)s;
+                            cx.csb(pos) = (uint32_t)b;
+                            pos++;
+                        }
+                } else if (mine) {
+                    cx.csa(pos) = (uint32_t)s;
+                    cx.csb(pos) = (uint32_t)s;
+                }
+            }
+            __syncthreads();
+            if (take == 0) {
+                overflow = true;
+                break;
+            }
+            const uint32_t T = sm.total;
+            S_proc += take;
+            if (T == 0) {
+                __syncthreads();  // sm.total is read before the next round clears it
+                continue;
+            }
+            for (uint32_t c = J + tid; c < J + T; c += NT) candidate_iso(cx, c, sm.uf[warp], lane, lw.evals);
+            __syncthreads();
+            // all pairs (j, i), J <= j < J + T, i < j, in lexicographic order: pair q = j (j - 1) / 2 + i. Warp w
+            // takes the w-th part of them, 32 at a time, survivors tested for the pseudoforest property as
+            // they fill a warp and at the part's end.
+            const uint64_t q0 = (uint64_t)J * (J - (J > 0)) / 2, q1 = (uint64_t)(J + T) * (J + T - 1) / 2, len = q1 - q0;
+            const uint64_t qa = q0 + len * warp / W, qz = q0 + len * (warp + 1) / W;
+            uint32_t jb = (uint32_t)((1.0 + sqrt(1.0 + 8.0 * (double)qa)) * 0.5);
+            while ((uint64_t)jb * (jb - 1) / 2 > qa) jb--;
+            while ((uint64_t)(jb + 1) * jb / 2 <= qa) jb++;
+            uint32_t ib = (uint32_t)(qa - (uint64_t)jb * (jb - 1) / 2), nsurv = 0;
+            bool done = false;
+            auto drain = [&](uint32_t cnt) {  // the first cnt <= 32 survivors; done when one passes
+                bool ok = false;
+                uint32_t e = 0;
+                if ((uint32_t)lane < cnt) {
+                    e = surv[lane];
+                    ok = cx.pair_ok(uf, e >> 16, e & 0xFFFF, lw.edges);
+                }
+                for (unsigned pass = __ballot_sync(0xffffffffu, ok); pass && !done; pass &= pass - 1) {
+                    const uint32_t f = __shfl_sync(0xffffffffu, e, __ffs(pass) - 1);
+                    if (float_accurate_triangular(cx.cseed(f >> 16), cx.cseed(f & 0xFFFF))) {
+                        if (lane == 0) atomicMin(&sm.best, (unsigned long long)(f >> 16) << 32 | (f & 0xFFFF));
+                        done = true;
+                    }
+                }
+                const uint32_t rest = nsurv - cnt;  // at most 31
+                const uint32_t v = (uint32_t)lane < rest ? surv[cnt + lane] : 0;
+                __syncwarp();
+                if ((uint32_t)lane < rest) surv[lane] = v;
+                nsurv = rest;
+                __syncwarp();
+            };
+            for (uint64_t qb = qa; qb < qz && !done; qb += 32) {
+                // a pair that comes before this warp's next one has passed already
+                if (*(volatile unsigned long long *)&sm.best < ((unsigned long long)jb << 32 | ib)) break;
+                uint32_t j = jb, i = ib + lane;
+                while (i >= j) {
+                    i -= j;
+                    j++;
+                }
+                bool filt = false;
+                if (qb + lane < qz) {
+                    uint64_t x = cx.iso(j, 0) & cx.iso(i, 0);
+                    if (Sh2Cfg<MAXM>::ISO_WORDS > 1) x |= cx.iso(j, 1) & cx.iso(i, 1);
+                    filt = x == 0;
+                    lw.pairs++;
+                    lw.filtered += filt;
+                }
+                for (uint32_t adv = ib + 32;;) {  // the next 32 pairs' first one
+                    if (adv < jb) {
+                        ib = adv;
+                        break;
+                    }
+                    adv -= jb;
+                    jb++;
+                }
+                const unsigned bal = __ballot_sync(0xffffffffu, filt);
+                if (filt) surv[nsurv + __popc(bal & below)] = j << 16 | i;
+                nsurv += __popc(bal);
+                __syncwarp();
+                if (nsurv >= 32) drain(32);
+            }
+            if (!done && nsurv) drain(nsurv);
+            __syncthreads();
+            best = sm.best;
+            J += T;
+        }
+        if (best == ~0ull) {
+            if (overflow && tid == 0) atomicOr(err, kErrScratch);
+            continue;
+        }
+        if (warp == 0) {
+            const uint64_t answer = pair_triangular(cx.cseed((uint32_t)(best >> 32)), cx.cseed((uint32_t)best));
+            if (lane == pend.n) {
+                pend.start = start;
+                pend.m = m;
+                pend.answer = answer;
+                *code_out = answer;
+            }
+            if (++pend.n == kInsert) sh2_insert<MAXM, false>(pend, keys, rib_bits, sm.uf[0], lane, quad_min, err);
+        }
+    }
+    if (pend.n) sh2_insert<MAXM, false>(pend, keys, rib_bits, sm.uf[0], lane, quad_min, err);
+    unsigned long long w[5] = {lw.evals, lw.pairs, lw.filtered, lw.edges, lw.scan};
+#pragma unroll
+    for (int k = 0; k < 5; k++)
+        for (int o = 16; o; o >>= 1) w[k] += __shfl_xor_sync(0xffffffffu, w[k], o);
+    if (lane == 0)
+        for (int k = 0; k < 5; k++) atomicAdd(&work[1 + k], w[k]);
+}
+
+template <int MAXM>
+void launch_block(const Node *nodes, const uint32_t *ids, uint32_t count, const uint64_t *keys, uint64_t *codes,
+                  uint8_t *rib_bits, uint8_t *scratch, uint64_t scratch_per_block, uint32_t smax, uint32_t cmax, uint32_t *err,
+                  unsigned long long *work, unsigned int *ctr, int grid, cudaStream_t s, uint32_t quad_min) {
+    const size_t smem = sizeof(Sh2BlockSmem<MAXM>);
+    cudaFuncSetAttribute(k_leaves_sh2_block<MAXM, NodeLeaves>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    k_leaves_sh2_block<MAXM, NodeLeaves><<<grid, kBlockLeafWarps<MAXM> * 32, smem, s>>>(
+        NodeLeaves{nodes, ids, codes}, count, keys, rib_bits, scratch, scratch_per_block, smax, cmax, err, work, ctr, quad_min);
 }
 
 // ------------------------------------------------------------------ work-queue schedule
@@ -1241,9 +1580,14 @@ uint64_t sh2_scratch_bytes(uint32_t smax, uint32_t cmax, int max_leaf) { return 
 void launch_leaves_sh2_ctr(const Node *nodes, const uint32_t *ids, uint32_t count, const uint64_t *keys, uint64_t *codes,
                            uint8_t *rib_bits, uint8_t *scratch, uint64_t scratch_per_warp, uint32_t smax, uint32_t cmax,
                            uint32_t *err, unsigned long long *work, unsigned int *ctr, int grid, cudaStream_t s,
-                           int max_leaf, uint32_t quad_min, int minb) {
+                           int max_leaf, uint32_t quad_min, int minb, bool block) {
     if (!count) return;
     cudaMemsetAsync(ctr, 0, sizeof(unsigned int), s);
+    if (block)
+        return max_leaf > 64 ? launch_block<128>(nodes, ids, count, keys, codes, rib_bits, scratch, scratch_per_warp, smax, cmax,
+                                                 err, work, ctr, grid, s, quad_min)
+                             : launch_block<64>(nodes, ids, count, keys, codes, rib_bits, scratch, scratch_per_warp, smax, cmax,
+                                                err, work, ctr, grid, s, quad_min);
     if (max_leaf > 64)
         launch_v2<128, 4>(nodes, ids, count, keys, codes, rib_bits, scratch, scratch_per_warp, smax, cmax, err, work, ctr, grid,
                           s, quad_min);
@@ -1256,6 +1600,16 @@ void launch_leaves_sh2_ctr(const Node *nodes, const uint32_t *ids, uint32_t coun
     else
         launch_v2<64, 6>(nodes, ids, count, keys, codes, rib_bits, scratch, scratch_per_warp, smax, cmax, err, work, ctr, grid,
                          s, quad_min);
+}
+
+// Whether a launch of nleaves leaves with nkeys keys in all is better searched by a block per leaf (the
+// figures are at kBlockLeafWarps; leaves of up to 56 keys lose at any count, so most leaves have to be
+// larger), and the blocks of such a launch.
+bool sh2_block_leaves(int max_leaf, uint64_t nleaves, uint64_t nkeys, int sms) {
+    return max_leaf > 64 ? nleaves <= 192ull * sms : max_leaf > 56 && nleaves <= 4ull * sms && nkeys >= 48 * nleaves;
+}
+int sh2_block_grid(int max_leaf, uint64_t nleaves, int sms) {
+    return (int)std::max<uint64_t>(1, std::min<uint64_t>(nleaves, (uint64_t)sms * (max_leaf > 64 ? 3 : 6)));
 }
 
 int sh2_smem_per_warp(int max_leaf) { return max_leaf <= 64 ? (int)sizeof(Sh2Smem<64>) : (int)sizeof(Sh2Smem<128>); }
