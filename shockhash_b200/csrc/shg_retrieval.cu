@@ -46,61 +46,167 @@ __global__ void k_ret_scatter(const uint64_t *__restrict__ keys, const uint8_t *
     }
 }
 
-struct RetWarpSmem {
-    uint64_t rows[kRetWords][kRetRows];  // word-major: lane r reads rows[w][r], consecutive addresses
+// A bucket's system as 32-bit words, word-major: lane l owns the rows l + 32 k.
+constexpr int kRetWords32 = 2 * kRetWords, kRetOwn = kRetRows / 32;
+struct alignas(16) RetWarpSmem {
+    union {
+        struct {
+            uint32_t table[32][kRetWords32];  // sums of the block's pivots 0..3 (entries 0..15) and 4..7 (16..31)
+            uint32_t pivots[8][kRetWords32];  // the block's pivot rows, one per column of the block
+        };
+        uint32_t hist[kRetPrio];  // only before the elimination
+    };
+    uint32_t rows[kRetWords32][kRetRows];
     uint8_t rhs[kRetRows];
-    uint16_t pivot_row[kRetRows];        // per column, or 0xFFFF for a free column
-    uint32_t hist[kRetPrio];
+    uint16_t pivot_row[kRetRows];     // per column, or 0xFFFF for a free column
 };
 
-// Forward elimination over rows [0, n) of the warp's system; returns true when it is consistent.
-__device__ bool ret_eliminate(RetWarpSmem &sm, uint32_t n, int lane) {
+// Forward elimination over rows [0, n) of the warp's system; returns true when it is consistent. rhs: bit k
+// the right-hand side of the lane's row l + 32 k.
+//
+// Eight columns at a time (the method of the four Russians): a row's byte in those columns, its
+// right-hand side and the set of the block's pivots added to it so far sit in one register, so the pivot
+// search and the eight eliminations touch no memory; then the rows' remaining words take the sum of their
+// pivots in one pass, from two tables of 16 sums. The plain form rewrote the rows once per column, bound by
+// those shared-memory updates. Which rows become pivots does not change the solution: the columns that have
+// one are the same in any order of rows, and free columns are set to zero. 8,334 buckets: 1.20 -> 0.64 ms, a single bucket 0.18 -> 0.07 ms.
+__device__ bool ret_eliminate(RetWarpSmem &sm, uint32_t n, int lane, uint32_t &rhs) {
     uint32_t done = 0;  // per lane: its rows lane + 32k that are pivots (or beyond n)
+    rhs = 0;
 #pragma unroll
-    for (int k = 0; k < kRetRows / 32; k++)
-        if ((uint32_t)(lane + 32 * k) >= n) done |= 1u << k;
+    for (int k = 0; k < kRetOwn; k++) {
+        const uint32_t r = lane + 32 * k;
+        if (r >= n) done |= 1u << k;
+        else rhs |= (uint32_t)sm.rhs[r] << k;
+    }
+#pragma unroll 1
+    for (int w = 0; w < kRetWords32; w++) {
+        if (__all_sync(0xffffffffu, done == (1u << kRetOwn) - 1)) {  // no row left: free columns from here on
+            for (int c = w * 32 + lane; c < 32 * kRetWords32; c += 32) sm.pivot_row[c] = 0xFFFF;
+            __syncwarp();
+            break;
+        }
+#pragma unroll 1
+        for (int shift = 0; shift < 32; shift += 8) {
+            // bits 0..7 the row's columns, bit 8 its right-hand side, bits 16..23 the pivots added to it, bits
+            // 24..26 k (a row that is a pivot already has no columns left here, and is not rewritten below)
+            uint32_t val[kRetOwn];
 #pragma unroll
-    for (int w = 0; w < kRetWords; w++) {
-        for (int bit = 0; bit < 64; bit++) {
-            const int c = w * 64 + bit;
-            uint32_t has = 0;
+            for (int k = 0; k < kRetOwn; k++)
+                val[k] = (uint32_t)k << 24 |
+                         ((done >> k) & 1 ? 0u : ((sm.rows[w][lane + 32 * k] >> shift) & 0xFF) | ((rhs >> k) & 1) << 8);
+            int prow[8];
+            uint32_t padd[8];
 #pragma unroll
-            for (int k = 0; k < kRetRows / 32; k++)
-                if (!((done >> k) & 1) && ((sm.rows[w][lane + 32 * k] >> bit) & 1)) has |= 1u << k;
-            int p = -1;
+            for (int b = 0; b < 8; b++) {
+                int p = -1;
+                uint32_t pv = 0;
+                const uint32_t any = val[0] | val[1] | val[2] | val[3] | val[4] | val[5] | val[6] | val[7];
+                const uint32_t has = __ballot_sync(0xffffffffu, (any >> b) & 1);
+                if (has) {  // warp-uniform
+                    const int src = __ffs(has) - 1;
 #pragma unroll
-            for (int k = 0; k < kRetRows / 32; k++) {
-                const uint32_t m = __ballot_sync(0xffffffffu, (has >> k) & 1);
-                if (p < 0 && m) p = 32 * k + __ffs(m) - 1;
+                    for (int k = kRetOwn - 1; k >= 0; k--)
+                        if ((val[k] >> b) & 1) pv = val[k];
+                    pv = __shfl_sync(0xffffffffu, pv, src);
+                    const int k0 = pv >> 24;
+                    p = 32 * k0 + src;
+                    if (lane == src) {  // final from here on
+                        done |= 1u << k0;
+                        rhs = (rhs & ~(1u << k0)) | ((pv >> 8) & 1) << k0;
+                    }
+                    const uint32_t add = (pv & 0x1FF) | 1u << (16 + b);
+#pragma unroll
+                    for (int k = 0; k < kRetOwn; k++)
+                        if ((val[k] >> b) & 1) val[k] ^= add;  // the pivot itself has no columns left then
+                }
+                prow[b] = p;
+                padd[b] = (pv >> 16) & 0xFF;
+                if (lane == 0) sm.pivot_row[w * 32 + shift + b] = p < 0 ? 0xFFFF : (uint16_t)p;
             }
-            if (lane == 0) sm.pivot_row[c] = p < 0 ? 0xFFFF : (uint16_t)p;
-            if (p < 0) continue;  // warp-uniform
-            if ((p & 31) == lane) {
-                done |= 1u << (p >> 5);
-                has &= ~(1u << (p >> 5));
-            }
-            uint64_t piv[kRetWords];
+            // the pivot rows (lane v: word v), each with the block's earlier pivots added to it
+            if (lane < kRetWords32 && lane >= w) {
+                uint32_t piv[8];
 #pragma unroll
-            for (int v = w; v < kRetWords; v++) piv[v] = sm.rows[v][p];
-            const uint8_t prhs = sm.rhs[p];
+                for (int b = 0; b < 8; b++) {
+                    uint32_t x = 0;
+                    if (prow[b] >= 0) {
+                        x = sm.rows[lane][prow[b]];
+#pragma unroll
+                        for (int j = 0; j < b; j++)
+                            if ((padd[b] >> j) & 1) x ^= piv[j];
+                        sm.rows[lane][prow[b]] = x;
+                    }
+                    piv[b] = x;
+                    sm.pivots[b][lane] = x;
+                }
+            }
+            __syncwarp();
+            {  // lane e: table entry e
+                const int half = (lane >> 4) * 4;
+                uint4 lo = make_uint4(0, 0, 0, 0), hi = lo;
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+                    if ((lane >> q) & 1) {
+                        const uint4 *pr = reinterpret_cast<const uint4 *>(sm.pivots[half + q]);
+                        const uint4 a = pr[0], c = pr[1];
+                        lo.x ^= a.x, lo.y ^= a.y, lo.z ^= a.z, lo.w ^= a.w;
+                        hi.x ^= c.x, hi.y ^= c.y, hi.z ^= c.z, hi.w ^= c.w;
+                    }
+                uint4 *t = reinterpret_cast<uint4 *>(sm.table[lane]);
+                t[0] = lo;
+                t[1] = hi;
+            }
             __syncwarp();
 #pragma unroll
-            for (int k = 0; k < kRetRows / 32; k++) {
-                if ((has >> k) & 1) {
+            for (int k = 0; k < kRetOwn; k++) {
+                const bool open = !((done >> k) & 1);
+                if (open) rhs = (rhs & ~(1u << k)) | ((val[k] >> 8) & 1) << k;
+                const uint32_t add = (val[k] >> 16) & 0xFF;
+                if (open && add) {
+                    const uint4 *t0 = reinterpret_cast<const uint4 *>(sm.table[add & 15]);
+                    const uint4 *t1 = reinterpret_cast<const uint4 *>(sm.table[16 + (add >> 4)]);
                     const int r = lane + 32 * k;
-#pragma unroll
-                    for (int v = w; v < kRetWords; v++) sm.rows[v][r] ^= piv[v];
-                    sm.rhs[r] ^= prhs;
+                    if (w < 4) {
+                        const uint4 a = t0[0], c = t1[0];
+                        sm.rows[0][r] ^= a.x ^ c.x;
+                        sm.rows[1][r] ^= a.y ^ c.y;
+                        sm.rows[2][r] ^= a.z ^ c.z;
+                        sm.rows[3][r] ^= a.w ^ c.w;
+                    }
+                    const uint4 a = t0[1], c = t1[1];
+                    sm.rows[4][r] ^= a.x ^ c.x;
+                    sm.rows[5][r] ^= a.y ^ c.y;
+                    sm.rows[6][r] ^= a.z ^ c.z;
+                    sm.rows[7][r] ^= a.w ^ c.w;
                 }
             }
             __syncwarp();
         }
     }
-    bool bad = false;
+    static_assert(kRetWords32 == 8 && kRetOwn == 8, "two 16-byte loads per table entry, eight rows per lane");
+    return !__any_sync(0xffffffffu, (rhs & ~done) != 0);
+}
+
+// Back substitution, free columns at zero: columns from the last down, x_c = the right-hand side of column
+// c's pivot row; a one is added to the right-hand sides of all rows that have column c.
+__device__ __forceinline__ void ret_substitute(const RetWarpSmem &sm, int lane, uint32_t rhs, uint32_t (&x)[kRetWords32]) {
 #pragma unroll
-    for (int k = 0; k < kRetRows / 32; k++)
-        if (!((done >> k) & 1) && sm.rhs[lane + 32 * k]) bad = true;
-    return !__any_sync(0xffffffffu, bad);
+    for (int w = kRetWords32 - 1; w >= 0; w--) {
+        uint32_t word[kRetOwn], xw = 0;
+#pragma unroll
+        for (int k = 0; k < kRetOwn; k++) word[k] = sm.rows[w][lane + 32 * k];
+#pragma unroll 1
+        for (int bit = 31; bit >= 0; bit--) {
+            const uint32_t p = sm.pivot_row[w * 32 + bit];
+            if (p == 0xFFFF) continue;
+            if (!((__shfl_sync(0xffffffffu, rhs, p & 31) >> (p >> 5)) & 1)) continue;
+            xw |= 1u << bit;
+#pragma unroll
+            for (int k = 0; k < kRetOwn; k++) rhs ^= ((word[k] >> bit) & 1) << k;
+        }
+        x[w] = xw;
+    }
 }
 
 // One warp per bucket: pick the threshold, solve, store the solution, pass the rest on.
@@ -144,6 +250,7 @@ __global__ void __launch_bounds__(kRetWarps * 32) k_ret_solve(const uint64_t *__
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) t = max(t, __shfl_xor_sync(0xffffffffu, t, o));
         // solve; an inconsistent kept set drops its highest priority value and is solved again
+        uint32_t rhs = 0;
         for (;;) {
             uint32_t n = 0, pmax = 0;
             for (uint32_t base = 0; base < m; base += 32) {
@@ -159,7 +266,11 @@ __global__ void __launch_bounds__(kRetWarps * 32) k_ret_solve(const uint64_t *__
                 if (keep) {
                     const uint32_t r = n + __popc(bal & ((1u << lane) - 1));
 #pragma unroll
-                    for (int v = 0; v < kRetWords; v++) sm.rows[v][r] = ret_row_word(h, v);
+                    for (int v = 0; v < kRetWords; v++) {
+                        const uint64_t word = ret_row_word(h, v);
+                        sm.rows[2 * v][r] = (uint32_t)word;
+                        sm.rows[2 * v + 1][r] = (uint32_t)(word >> 32);
+                    }
                     sm.rhs[r] = bbits[a0 + i];
                     pmax = max(pmax, p);
                 }
@@ -168,23 +279,15 @@ __global__ void __launch_bounds__(kRetWarps * 32) k_ret_solve(const uint64_t *__
             __syncwarp();
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) pmax = max(pmax, __shfl_xor_sync(0xffffffffu, pmax, o));
-            if (ret_eliminate(sm, n, lane) || n == 0) break;
+            if (ret_eliminate(sm, n, lane, rhs) || n == 0) break;
             t = pmax;  // keep p < pmax: at least one key fewer
             __syncwarp();
         }
-        // back substitution, free columns at zero: x_c = rhs(P_c) ^ parity(P_c & x) over columns > c
-        uint64_t x[kRetWords] = {0, 0, 0, 0};
+        uint32_t x32[kRetWords32];
+        ret_substitute(sm, lane, rhs, x32);
+        uint64_t x[kRetWords];
 #pragma unroll
-        for (int w = kRetWords - 1; w >= 0; w--) {
-            for (int bit = 63; bit >= 0; bit--) {
-                const uint32_t pr = sm.pivot_row[w * 64 + bit];
-                if (pr == 0xFFFF) continue;
-                uint32_t par = sm.rhs[pr];
-#pragma unroll
-                for (int v = w; v < kRetWords; v++) par += (uint32_t)__popcll(sm.rows[v][pr] & x[v]);
-                if (par & 1) x[w] |= 1ull << bit;
-            }
-        }
+        for (int v = 0; v < kRetWords; v++) x[v] = (uint64_t)x32[2 * v + 1] << 32 | x32[2 * v];
         if (lane == 0) {
 #pragma unroll
             for (int v = 0; v < kRetWords; v++) sol[b * kRetWords + v] = x[v];
