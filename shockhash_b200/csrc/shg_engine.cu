@@ -82,6 +82,32 @@ struct DevBuf {
     }
 };
 
+// Host buffer for a build's small transfers: pinned, so that they run without staging copies, or plain
+// memory when no pinned memory can be had.
+struct HostBuf {
+    void *p = nullptr;
+    size_t cap = 0;
+    bool pinned = false;
+    bool ensure(size_t bytes) {
+        if (bytes <= cap) return true;
+        release();
+        const size_t want = bytes + bytes / 4 + 4096;
+        pinned = cudaHostAlloc(&p, want, cudaHostAllocDefault) == cudaSuccess;
+        if (!pinned) {
+            cudaGetLastError();
+            p = malloc(want);
+        }
+        if (p) cap = want;
+        return p != nullptr;
+    }
+    void release() {
+        if (p && pinned) cudaFreeHost(p);
+        else free(p);
+        p = nullptr;
+        cap = 0;
+    }
+};
+
 } // namespace
 
 // Pinned host block that a result's arrays live in; reused across builds once released. One
@@ -130,7 +156,8 @@ struct shg_engine {
         DevBuf cnt, nodes, node_off, singles, single_off, skip_bits;
     };
     std::vector<Shapes *> shapes;
-    DevBuf plan_offs, ret_scratch, qdone, qorder, split_best;
+    DevBuf plan_offs, ret_scratch, qdone, qorder, split_best, breq;
+    HostBuf small;
     cudaEvent_t ev[8] = {};
     cudaStream_t stream2 = nullptr;  // leaves of the pipelined mode
     static constexpr int kMaxChunks = 64;
@@ -169,6 +196,8 @@ struct shg_engine {
         qdone.release();
         qorder.release();
         split_best.release();
+        breq.release();
+        small.release();
         for (Shapes *sh : shapes) {
             DevBuf *sb[] = {&sh->cnt, &sh->nodes, &sh->node_off, &sh->singles, &sh->single_off, &sh->skip_bits};
             for (DevBuf *b : sb) b->release();
@@ -399,6 +428,24 @@ shg_status build_batch(shg_engine *e, const shg_params *p, const uint64_t *d_fir
     CU(cudaMemsetAsync(misc, 0, sizeof(Misc), s));
     CU(e->counts.ensure(nb * 4));
     CU(e->cursor.ensure(nb * 4));
+    // the host side of the build's small transfers
+    if (!e->small.ensure((2 * nb + 1 + R) * 8 + sizeof(Misc) + kMaxPlanCols * 4 + R * (sizeof(BatchReq) + sizeof(QueueOut) + 8) + 64))
+        return fail(SHG_ERR_OOM, "host allocation failed");
+    uint64_t *const acc = (uint64_t *)e->small.p, *const pos = acc + nb + 1;
+    Misc *const hmisc = (Misc *)(pos + nb + R);
+    BatchReq *const hreq = (BatchReq *)(hmisc + 1);
+    QueueOut *const hqout = (QueueOut *)(hreq + R);
+    uint64_t *const hwoff = (uint64_t *)(hqout + R);
+    uint32_t *const totals = (uint32_t *)(hwoff + R);
+    // a batch's requests go through the partition and the encoding together, from this table
+    const bool batch = R > 1;
+    const BatchReq *d_req = nullptr;
+    if (batch) {
+        for (size_t r = 0; r < R; r++) hreq[r] = BatchReq{off[r], nr[r], boff[r], nbr[r], nb_map[r], b0[r]};
+        CU(e->breq.ensure(R * (sizeof(BatchReq) + 8)));
+        CU(cudaMemcpyAsync(e->breq.p, hreq, R * sizeof(BatchReq), cudaMemcpyHostToDevice, s));
+        d_req = e->breq.as<BatchReq>();
+    }
     CU(e->acc.ensure((nb + 1) * 8));
     CU(e->sfirst.ensure(std::max<uint64_t>(n, 1) * 8));
     CU(e->sidx.ensure(std::max<uint64_t>(n, 1) * 4));
@@ -422,22 +469,21 @@ shg_status build_batch(shg_engine *e, const shg_params *p, const uint64_t *d_fir
         return err;
     };
     CU(cudaEventRecord(e->ev[0], s));
-    for (size_t r = 0; r < R; r++)
-        launch_bucket_count(d_first + off[r], nr[r], nbr[r], nb_map[r], b0[r], e->counts.as<uint32_t>() + boff[r], &misc->err,
-                            s);
+    if (batch) {
+        CU(cudaMemsetAsync(e->counts.p, 0, nb * 4, s));
+        launch_batch_count(d_first, d_req, (uint32_t)R, e->counts.as<uint32_t>(), &misc->err, s);
+    } else {
+        launch_bucket_count(d_first, n, nb, nb_map[0], b0[0], e->counts.as<uint32_t>(), &misc->err, s);
+    }
     launch_scan_counts(e->counts.as<uint32_t>(), nb, e->acc.as<uint64_t>(), e->cursor.as<uint32_t>(), &misc->maxsz, s);
     CU(plan_scan());
-    std::vector<uint64_t> acc(nb + 1);
-    uint32_t totals[kMaxPlanCols] = {};
-    uint32_t maxsz = 0;
-    CU(cudaMemcpyAsync(acc.data(), e->acc.p, (nb + 1) * 8, cudaMemcpyDeviceToHost, s));
-    CU(cudaMemcpyAsync(&maxsz, &misc->maxsz, 4, cudaMemcpyDeviceToHost, s));
+    CU(cudaMemcpyAsync(acc, e->acc.p, (nb + 1) * 8, cudaMemcpyDeviceToHost, s));
+    CU(cudaMemcpyAsync(hmisc, misc, sizeof(Misc), cudaMemcpyDeviceToHost, s));
     CU(cudaMemcpyAsync(totals, e->plan_offs.as<uint32_t>() + shp->host.ncol * offs_stride, shp->host.ncol * 4,
                        cudaMemcpyDeviceToHost, s));
-    uint32_t perr = 0;
-    CU(cudaMemcpyAsync(&perr, &misc->err, 4, cudaMemcpyDeviceToHost, s));
     CU(cudaStreamSynchronize(s));
-    if (perr & kErrArg) return fail(SHG_ERR_ARG, "a key lies outside the shard's bucket range");
+    const uint32_t maxsz = hmisc->maxsz;
+    if (hmisc->err & kErrArg) return fail(SHG_ERR_ARG, "a key lies outside the shard's bucket range");
     if (maxsz >= (uint32_t)kMaxBucket)
         return fail(SHG_ERR_BUCKET, "a bucket holds " + std::to_string(maxsz) + " keys (MAX_BUCKET_SIZE is 3000)");
     if (maxsz >= shp->host.rows) {  // a bucket larger than the shape tables cover: grow them, scan again
@@ -449,10 +495,12 @@ shg_status build_batch(shg_engine *e, const shg_params *p, const uint64_t *d_fir
         CU(cudaStreamSynchronize(s));
     }
     const ShapeTables &tab = shp->host;
-    for (size_t r = 0; r < R; r++)
-        launch_bucket_scatter(d_first + off[r], nr[r], nbr[r], nb_map[r], b0[r], e->cursor.as<uint32_t>() + boff[r],
-                              e->sfirst.as<uint64_t>(),
-                              e->sidx.as<uint32_t>(), off[r], s);
+    if (batch)
+        launch_batch_scatter(d_first, d_req, (uint32_t)R, e->cursor.as<uint32_t>(), e->sfirst.as<uint64_t>(),
+                             e->sidx.as<uint32_t>(), s);
+    else
+        launch_bucket_scatter(d_first, n, nb, nb_map[0], b0[0], e->cursor.as<uint32_t>(), e->sfirst.as<uint64_t>(),
+                              e->sidx.as<uint32_t>(), 0, s);
     launch_bucket_sort(e->acc.as<uint64_t>(), nb, e->sfirst.as<uint64_t>(), e->sidx.as<uint32_t>(), d_second,
                        e->keys.as<uint64_t>(), s);
     CU(cudaEventRecord(e->ev[1], s));
@@ -529,25 +577,21 @@ shg_status build_batch(shg_engine *e, const shg_params *p, const uint64_t *d_fir
     // straight into the pinned result block as the bucket's leaves finish
     const bool stream_out = queue && tun.queue_lag > 0;
     const bool early_keys = p->variant == SHG_SHOCKHASH2 && p->mode != SHG_MODE_PIPELINED && !queue;
-    std::vector<uint64_t> wcap(R, 0);
-    std::vector<size_t> roff(R + 1, 0);
-    auto layout = [&]() {
-        for (size_t r = 0; r < R; r++) {
-            const size_t acc_bytes = (nbr[r] + 1) * 8;
-            roff[r + 1] = roff[r] + ((2 * acc_bytes + rnv[r] * 9 + wcap[r] * 8 + 64 + 63) & ~(size_t)63);
-        }
-    };
+    // The block's arrays lie one kind after another, each with the requests' parts back to back as on the
+    // device, so that a kind is one copy however many requests there are.
+    const uint64_t rn_all = n - soff[R];
+    const size_t acc_bytes = (nb + R) * 8, o_keys = 2 * acc_bytes, o_bits = o_keys + rn_all * 8,
+                 o_desc = (o_bits + rn_all + 7) & ~(size_t)7;
+    uint64_t wcap = 0;  // descriptor words there is room for
     PinnedBlock *blk = nullptr;
     if (early_keys || stream_out) {
         for (size_t r = 0; r < R; r++) {
             const uint64_t bits = rfixed[r] + 8 * rnodes[r] + 1;
-            wcap[r] = ((bits + 7) / 8 + 14) / 8;
+            wcap += ((bits + 7) / 8 + 14) / 8;
         }
-        layout();
-        blk = acquire_pinned(e, roff[R], (int)R);
+        blk = acquire_pinned(e, o_desc + wcap * 8, (int)R);
         if (!blk) return fail(SHG_ERR_OOM, "pinned host allocation failed");
     }
-    auto keys_host = [&](PinnedBlock *b, size_t r) { return (uint64_t *)((uint8_t *)b->p + roff[r] + 2 * (nbr[r] + 1) * 8); };
     auto release_all = [&](PinnedBlock *b) {  // drop every reference a failed build still holds
         for (size_t r = 0; r < R; r++) release_pinned(b);
     };
@@ -643,12 +687,11 @@ shg_status build_batch(shg_engine *e, const shg_params *p, const uint64_t *d_fir
         QueueOut *q_out = nullptr;
         if (stream_out) {
             // where each request's compacted retrieval keys and bits go in the pinned block
-            std::vector<QueueOut> qo(R);
             for (size_t r = 0; r < R; r++)
-                qo[r] = QueueOut{boff[r], off[r], soff[r], keys_host(blk, r), (uint8_t *)keys_host(blk, r) + rnv[r] * 8};
+                hqout[r] = QueueOut{boff[r], off[r], soff[r], (uint64_t *)((uint8_t *)blk->p + o_keys) + (off[r] - soff[r]),
+                                    (uint8_t *)blk->p + o_bits + (off[r] - soff[r])};
             q_out = (QueueOut *)(e->qorder.as<uint32_t>() + order_words);
-            CU(cudaMemcpyAsync(q_out, qo.data(), R * sizeof(QueueOut), cudaMemcpyHostToDevice, s));
-            CU(cudaStreamSynchronize(s));  // qo is pageable and leaves scope
+            CU(cudaMemcpyAsync(q_out, hqout, R * sizeof(QueueOut), cudaMemcpyHostToDevice, s));
         }
         CU(e->scratch.ensure(per_warp * (uint64_t)qgrid * tree_queue_warps_per_block()));
         CU(e->qdone.ensure(std::max<uint64_t>(nb, 1) * 4));
@@ -699,16 +742,13 @@ shg_status build_batch(shg_engine *e, const shg_params *p, const uint64_t *d_fir
         if (early_keys) {
             // compaction on the engine stream before the leaf kernel takes every SM; only the
             // copies run on the second stream, next to the leaves
-            for (size_t r = 0; r < R; r++)
-                if (rnv[r])
-                    launch_compact_ribbon(e->keys.as<uint64_t>() + off[r], nullptr, nr[r], e->singles.as<uint64_t>() + soff[r],
-                                          soff[r + 1] - soff[r], off[r], e->ckeys.as<uint64_t>() + off[r], nullptr, s);
+            if (rn_all)
+                launch_compact_ribbon(e->keys.as<uint64_t>(), nullptr, n, e->singles.as<uint64_t>(), nsingles, 0,
+                                      e->ckeys.as<uint64_t>(), nullptr, s);
             CU(cudaEventRecord(e->chunk_ev[0], s));
             CU(cudaStreamWaitEvent(e->stream2, e->chunk_ev[0], 0));
-            for (size_t r = 0; r < R; r++)
-                if (rnv[r])
-                    CU(cudaMemcpyAsync(keys_host(blk, r), e->ckeys.as<uint64_t>() + off[r], rnv[r] * 8, cudaMemcpyDeviceToHost,
-                                       e->stream2));
+            if (rn_all)
+                CU(cudaMemcpyAsync((uint8_t *)blk->p + o_keys, e->ckeys.p, rn_all * 8, cudaMemcpyDeviceToHost, e->stream2));
             CU(cudaEventRecord(e->join_ev, e->stream2));
         }
         if (p->mode == SHG_MODE_PER_LEAF)
@@ -721,16 +761,14 @@ shg_status build_batch(shg_engine *e, const shg_params *p, const uint64_t *d_fir
 
     // ---- Golomb-Rice encode, one stream per request
     CU(e->pos_acc.ensure((nb + R) * 8));
-    for (size_t r = 0; r < R; r++) {
-        launch_gr_bucket_bits(e->nodes.as<Node>(), d_bnb + boff[r], nbr[r], e->acc.as<uint64_t>() + boff[r],
-                              e->codes.as<uint64_t>(), d_skip, e->bucket_bits.as<uint64_t>() + boff[r], s);
-        launch_scan_u64(e->bucket_bits.as<uint64_t>() + boff[r], nbr[r], e->pos_acc.as<uint64_t>() + boff[r] + r, s);
-    }
-    std::vector<uint64_t> pos(nb + R);
-    CU(cudaMemcpyAsync(pos.data(), e->pos_acc.p, (nb + R) * 8, cudaMemcpyDeviceToHost, s));
-    uint32_t err = 0;
-    CU(cudaMemcpyAsync(&err, &misc->err, 4, cudaMemcpyDeviceToHost, s));
+    launch_gr_bucket_bits(e->nodes.as<Node>(), d_bnb, nb, e->acc.as<uint64_t>(), e->codes.as<uint64_t>(), d_skip,
+                          e->bucket_bits.as<uint64_t>(), s);
+    if (batch) launch_batch_scan_u64(e->bucket_bits.as<uint64_t>(), d_req, (uint32_t)R, e->pos_acc.as<uint64_t>(), s);
+    else launch_scan_u64(e->bucket_bits.as<uint64_t>(), nb, e->pos_acc.as<uint64_t>(), s);
+    CU(cudaMemcpyAsync(pos, e->pos_acc.p, acc_bytes, cudaMemcpyDeviceToHost, s));
+    CU(cudaMemcpyAsync(hmisc, misc, sizeof(Misc), cudaMemcpyDeviceToHost, s));
     CU(cudaStreamSynchronize(s));
+    const uint32_t err = hmisc->err;
     if (err && blk) {
         cudaStreamSynchronize(e->stream2);
         release_all(blk);
@@ -747,14 +785,16 @@ shg_status build_batch(shg_engine *e, const shg_params *p, const uint64_t *d_fir
     }
     CU(e->words.ensure(wbase[R] * 8));
     CU(cudaMemsetAsync(e->words.p, 0, wbase[R] * 8, s));
-    for (size_t r = 0; r < R; r++) {
-        unsigned long long *w = e->words.as<unsigned long long>() + wbase[r];
-        launch_gr_write(e->nodes.as<Node>(), e->fixed_off.as<uint16_t>(), d_bnb + boff[r], nbr[r],
-                        e->acc.as<uint64_t>() + boff[r], e->pos_acc.as<uint64_t>() + boff[r] + r, e->codes.as<uint64_t>(),
-                        d_skip, w, s);
-        launch_set_bit(w, total[r], s);
-        launches += 4;
+    uint64_t *d_woff = nullptr;
+    if (batch) {
+        d_woff = (uint64_t *)(e->breq.as<BatchReq>() + R);
+        for (size_t r = 0; r < R; r++) hwoff[r] = wbase[r];
+        CU(cudaMemcpyAsync(d_woff, hwoff, R * 8, cudaMemcpyHostToDevice, s));
     }
+    launch_gr_write(e->nodes.as<Node>(), e->fixed_off.as<uint16_t>(), d_bnb, nb, e->acc.as<uint64_t>(),
+                    e->pos_acc.as<uint64_t>(), e->codes.as<uint64_t>(), d_skip, e->words.as<unsigned long long>(), d_req, d_woff,
+                    (uint32_t)R, s);
+    launches += 3;
     CU(cudaGetLastError());
     CU(cudaEventRecord(e->ev[5], s));
 
@@ -762,9 +802,7 @@ shg_status build_batch(shg_engine *e, const shg_params *p, const uint64_t *d_fir
     // each result holding a reference); the retrieval input is compacted on the device first.
     bool keys_done = early_keys || stream_out, bits_done = stream_out;
     if (early_keys || stream_out) {
-        bool fits = true;
-        for (size_t r = 0; r < R; r++) fits = fits && words[r] <= wcap[r];
-        if (!fits) {  // descriptor stream longer than the bound: a new block, keys (and bits) copied again
+        if (wbase[R] > wcap) {  // descriptor stream longer than the bound: a new block, keys (and bits) copied again
             CU(cudaStreamSynchronize(e->stream2));
             release_all(blk);
             blk = nullptr;
@@ -772,45 +810,35 @@ shg_status build_batch(shg_engine *e, const shg_params *p, const uint64_t *d_fir
         }
     }
     if (!blk) {
-        for (size_t r = 0; r < R; r++) wcap[r] = words[r];
-        layout();
-        blk = acquire_pinned(e, roff[R], (int)R);
+        blk = acquire_pinned(e, o_desc + wbase[R] * 8, (int)R);
         if (!blk) return fail(SHG_ERR_OOM, "pinned host allocation failed");
     }
     const uint64_t *src_keys = is_sh1(p->variant) ? e->rib_keys.as<uint64_t>() : e->keys.as<uint64_t>();
+    uint8_t *const hp = (uint8_t *)blk->p;
+    if (!bits_done)
+        launch_compact_ribbon(src_keys, e->rib_bits.as<uint8_t>(), n, e->singles.as<uint64_t>(), nsingles, 0,
+                              keys_done ? nullptr : e->ckeys.as<uint64_t>(), e->cbits.as<uint8_t>(), s);
+    CU(cudaMemcpyAsync(hp + o_desc, e->words.p, wbase[R] * 8, cudaMemcpyDeviceToHost, s));
+    if (rn_all && !keys_done) CU(cudaMemcpyAsync(hp + o_keys, e->ckeys.p, rn_all * 8, cudaMemcpyDeviceToHost, s));
+    if (rn_all && !bits_done) CU(cudaMemcpyAsync(hp + o_bits, e->cbits.p, rn_all, cudaMemcpyDeviceToHost, s));
+    if (keys_done && early_keys) CU(cudaStreamWaitEvent(s, e->join_ev, 0));  // the keys copied during the leaves
+    CU(cudaEventRecord(e->ev[6], s));
+    memcpy(hp + acc_bytes, pos, acc_bytes);  // next to the copies
     for (size_t r = 0; r < R; r++) {
         shg_result *out = &outs[r];
-        const uint64_t ns = soff[r + 1] - soff[r], rn = rnv[r];
-        if (!bits_done)
-            launch_compact_ribbon(src_keys + off[r], e->rib_bits.as<uint8_t>() + off[r], nr[r], e->singles.as<uint64_t>() + soff[r],
-                                  ns, off[r], keys_done ? nullptr : e->ckeys.as<uint64_t>() + off[r],
-                                  e->cbits.as<uint8_t>() + off[r], s);
-        const size_t acc_bytes = (nbr[r] + 1) * 8;
-        uint8_t *hp = (uint8_t *)blk->p + roff[r];
         out->owner = blk;
-        out->bucket_size_acc = (uint64_t *)hp;
-        out->bucket_pos_acc = (uint64_t *)(hp + acc_bytes);
-        out->ribbon_keys = (uint64_t *)(hp + 2 * acc_bytes);
-        out->ribbon_bits = hp + 2 * acc_bytes + rn * 8;
-        out->descriptors = (uint64_t *)(hp + ((2 * acc_bytes + rn * 9 + 7) & ~(size_t)7));
+        out->bucket_size_acc = (uint64_t *)hp + boff[r] + r;
+        out->bucket_pos_acc = (uint64_t *)(hp + acc_bytes) + boff[r] + r;
+        out->ribbon_keys = (uint64_t *)(hp + o_keys) + (off[r] - soff[r]);
+        out->ribbon_bits = hp + o_bits + (off[r] - soff[r]);
+        out->descriptors = (uint64_t *)(hp + o_desc) + wbase[r];
         for (uint64_t b = 0; b <= nbr[r]; b++) out->bucket_size_acc[b] = acc[boff[r] + b] - acc[boff[r]];
-        CU(cudaMemcpyAsync(out->bucket_pos_acc, e->pos_acc.as<uint64_t>() + boff[r] + r, acc_bytes, cudaMemcpyDeviceToHost, s));
-        CU(cudaMemcpyAsync(out->descriptors, e->words.as<uint64_t>() + wbase[r], words[r] * 8, cudaMemcpyDeviceToHost, s));
-        if (rn) {
-            if (!keys_done)
-                CU(cudaMemcpyAsync(out->ribbon_keys, e->ckeys.as<uint64_t>() + off[r], rn * 8, cudaMemcpyDeviceToHost, s));
-            if (!bits_done)
-                CU(cudaMemcpyAsync(out->ribbon_bits, e->cbits.as<uint8_t>() + off[r], rn, cudaMemcpyDeviceToHost, s));
-        }
         out->desc_words = words[r];
         out->desc_bits = total[r] + 1;
-        out->ribbon_n = rn;
+        out->ribbon_n = rnv[r];
     }
-    if (keys_done && early_keys) CU(cudaStreamWaitEvent(s, e->join_ev, 0));  // the keys copied during the leaves
-    unsigned long long work[8];
-    CU(cudaMemcpyAsync(work, misc->work, sizeof(work), cudaMemcpyDeviceToHost, s));
-    CU(cudaMemcpyAsync(e->split_kind, misc->split_kind, sizeof(e->split_kind), cudaMemcpyDeviceToHost, s));
-    CU(cudaEventRecord(e->ev[6], s));
+    const unsigned long long *const work = hmisc->work;  // final since the encoding's copy
+    memcpy(e->split_kind, hmisc->split_kind, sizeof(e->split_kind));
     CU(cudaStreamSynchronize(s));
     e->split_launches = 0;
     for (int lv = 0; lv < nlevels; lv++) e->split_launches += level_count[lv] ? 1 : 0;
@@ -831,11 +859,10 @@ shg_status build_batch(shg_engine *e, const shg_params *p, const uint64_t *d_fir
         out->work[5] = nleaves;
         out->work[6] = nn - nleaves;
         // kernels of this build: hashing (when the keys were hashed on the device), partition
-        // (count and scatter per request, one scan, one sort), plan (offset scan and expansion),
-        // split levels and leaves, Golomb-Rice encoding (4 per request, counted above), retrieval
-        // compaction (keys and bits together, or keys before the leaves and bits after them)
-        out->work[7] = (hash_ms > 0.f ? 1 : 0) + 2 * R + 2 + plan_launches + launches +
-                      R * ((early_keys ? 1 : 0) + (bits_done ? 0 : 1));
+        // (count, scan, scatter, sort), plan (offset scan and expansion), split levels and leaves,
+        // Golomb-Rice encoding (3, counted above), retrieval compaction (keys and bits together, or keys
+        // before the leaves and bits after them)
+        out->work[7] = (hash_ms > 0.f ? 1 : 0) + 4 + plan_launches + launches + (early_keys ? 1 : 0) + (bits_done ? 0 : 1);
     }
     return SHG_OK;
 }

@@ -31,8 +31,8 @@ __global__ void k_gr_bucket_bits(const Node *__restrict__ nodes, const uint32_t 
     }
 }
 
-// Exclusive scan of n u64 values into out[0..n] (out[n] = total), one block.
-__global__ void k_scan_u64(const uint64_t *__restrict__ in, uint64_t n, uint64_t *__restrict__ out) {
+// Exclusive scan of n u64 values into out[0..n] (out[n] = total) by one block.
+__device__ __forceinline__ void scan_u64(const uint64_t *__restrict__ in, uint64_t n, uint64_t *__restrict__ out) {
     __shared__ uint64_t warp_sums[32];
     __shared__ uint64_t carry;
     if (threadIdx.x == 0) carry = 0;
@@ -67,6 +67,12 @@ __global__ void k_scan_u64(const uint64_t *__restrict__ in, uint64_t n, uint64_t
     }
     if (threadIdx.x == 0) out[n] = carry;
 }
+__global__ void k_scan_u64(const uint64_t *__restrict__ in, uint64_t n, uint64_t *__restrict__ out) { scan_u64(in, n, out); }
+// The same for each request of a batch, one block per request.
+__global__ void k_batch_scan_u64(const uint64_t *__restrict__ in, const BatchReq *__restrict__ req, uint64_t *__restrict__ pos) {
+    const BatchReq q = req[blockIdx.x];
+    scan_u64(in + q.b_first, q.nb, pos + q.b_first + blockIdx.x);
+}
 
 __device__ __forceinline__ void or_bits(unsigned long long *words, uint64_t pos, uint64_t v, int len) {
     if (len == 0) return;
@@ -83,14 +89,29 @@ __device__ __forceinline__ void or_bits(unsigned long long *words, uint64_t pos,
 __global__ void k_gr_write(const Node *__restrict__ nodes, const uint16_t *__restrict__ fixed_off,
                            const uint32_t *__restrict__ bnb, uint64_t nb, const uint64_t *__restrict__ acc,
                            const uint64_t *__restrict__ pos_acc, const uint64_t *__restrict__ codes,
-                           const uint32_t *__restrict__ skip_bits, unsigned long long *__restrict__ words) {
+                           const uint32_t *__restrict__ skip_bits, unsigned long long *__restrict__ stream,
+                           const BatchReq *__restrict__ req, const uint64_t *__restrict__ word_off, uint32_t nreq) {
     const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
     for (uint64_t b = warp; b < nb; b += nwarps) {
         const uint32_t n0 = bnb[b], n1 = bnb[b + 1];
+        uint32_t r = 0;
+        uint64_t end = nb;  // the request of bucket b and its last bucket's successor
+        if (req) {
+            for (uint32_t hi = nreq; hi - r > 1;) {
+                const uint32_t mid = (r + hi) >> 1;
+                if (req[mid].b_first <= b) r = mid; else hi = mid;
+            }
+            end = req[r].b_first + req[r].nb;
+        }
+        unsigned long long *const words = stream + (req ? word_off[r] : 0);
+        const uint64_t pos = pos_acc[b + r];
+        if (b + 1 == end && lane == 0) {  // the sentinel after the request's last code
+            const uint64_t bit = pos_acc[end + r];
+            atomicOr(&words[bit >> 6], 1ull << (bit & 63));
+        }
         if (n0 == n1) continue;
-        const uint64_t pos = pos_acc[b];
         const uint32_t m = (uint32_t)(acc[b + 1] - acc[b]);
         const uint64_t unary0 = pos + skip_bits[m];
         uint64_t carry = 0;
@@ -119,8 +140,6 @@ __global__ void k_gr_write(const Node *__restrict__ nodes, const uint16_t *__res
     }
 }
 
-__global__ void k_set_bit(unsigned long long *words, uint64_t bit) { atomicOr(&words[bit >> 6], 1ull << (bit & 63)); }
-
 void launch_gr_bucket_bits(const Node *nodes, const uint32_t *bnb, uint64_t nb, const uint64_t *acc, const uint64_t *codes,
                            const uint32_t *skip_bits, uint64_t *bucket_bits, cudaStream_t s) {
     const uint64_t blocks = (nb * 32 + 255) / 256;
@@ -130,11 +149,13 @@ void launch_gr_bucket_bits(const Node *nodes, const uint32_t *bnb, uint64_t nb, 
 void launch_scan_u64(const uint64_t *in, uint64_t n, uint64_t *out, cudaStream_t s) { k_scan_u64<<<1, 1024, 0, s>>>(in, n, out); }
 void launch_gr_write(const Node *nodes, const uint16_t *fixed_off, const uint32_t *bnb, uint64_t nb, const uint64_t *acc,
                      const uint64_t *pos_acc, const uint64_t *codes, const uint32_t *skip_bits, unsigned long long *words,
-                     cudaStream_t s) {
+                     const BatchReq *req, const uint64_t *word_off, uint32_t nreq, cudaStream_t s) {
     const uint64_t blocks = (nb * 32 + 255) / 256;
     k_gr_write<<<(int)(blocks < 148 * 16 ? blocks : 148 * 16), 256, 0, s>>>(nodes, fixed_off, bnb, nb, acc, pos_acc, codes,
-                                                                            skip_bits, words);
+                                                                            skip_bits, words, req, word_off, nreq);
 }
-void launch_set_bit(unsigned long long *words, uint64_t bit, cudaStream_t s) { k_set_bit<<<1, 1, 0, s>>>(words, bit); }
+void launch_batch_scan_u64(const uint64_t *in, const BatchReq *req, uint32_t nreq, uint64_t *pos, cudaStream_t s) {
+    k_batch_scan_u64<<<nreq, 1024, 0, s>>>(in, req, pos);
+}
 
 } // namespace shg

@@ -214,14 +214,28 @@ void launch_tree_queue(const Node *nodes, const uint32_t *ids, const uint32_t *s
                        uint64_t max_trials, uint32_t *err, unsigned long long *work, unsigned long long *kind_work,
                        unsigned int *ctr, uint32_t nleaf_tail, const uint64_t *acc, const uint64_t *singles,
                        const QueueOut *out, uint32_t nreq, uint32_t max_m, const SplitTuning &t, int grid, cudaStream_t s);
+// One request of a batched build: its keys are [key_off, key_off + n) of the batch's arrays and its buckets
+// [b_first, b_first + nb), which hold buckets b0, b0 + 1, ... of a structure with nb_map buckets.
+struct BatchReq {
+    uint64_t key_off, n, b_first, nb, nb_map, b0;
+};
+// Bucket counts (zeroed by the caller) and scatter of all requests' keys, nreq requests in one launch.
+void launch_batch_count(const uint64_t *first, const BatchReq *req, uint32_t nreq, uint32_t *counts, uint32_t *err,
+                        cudaStream_t s);
+void launch_batch_scatter(const uint64_t *first, const BatchReq *req, uint32_t nreq, uint32_t *cursor, uint64_t *sfirst,
+                          uint32_t *sidx, cudaStream_t s);
+// Each request's bucket lengths scanned into pos + b_first + r: nb + 1 positions per request r.
+void launch_batch_scan_u64(const uint64_t *in, const BatchReq *req, uint32_t nreq, uint64_t *pos, cudaStream_t s);
 void launch_gr_bucket_bits(const Node *nodes, const uint32_t *bnb, uint64_t nb, const uint64_t *acc,
                            const uint64_t *codes, const uint32_t *memo_skip_bits, uint64_t *bucket_bits,
                            cudaStream_t s);
 void launch_scan_u64(const uint64_t *in, uint64_t n, uint64_t *out_excl_plus_total, cudaStream_t s);
+// The descriptor words of all buckets and each request's sentinel: request r's stream starts at word
+// word_off[r], its bucket positions at pos_acc + b_first + r. One request: req and word_off null.
 void launch_gr_write(const Node *nodes, const uint16_t *fixed_off, const uint32_t *bnb, uint64_t nb,
                      const uint64_t *acc, const uint64_t *pos_acc, const uint64_t *codes,
-                     const uint32_t *memo_skip_bits, unsigned long long *words, cudaStream_t s);
-void launch_set_bit(unsigned long long *words, uint64_t bit, cudaStream_t s);
+                     const uint32_t *memo_skip_bits, unsigned long long *words, const BatchReq *req,
+                     const uint64_t *word_off, uint32_t nreq, cudaStream_t s);
 void launch_compact_ribbon(const uint64_t *keys, const uint8_t *bits, uint64_t n, const uint64_t *singles,
                            uint64_t nsingles, uint64_t single_base, uint64_t *out_keys, uint8_t *out_bits,
                            cudaStream_t s);

@@ -463,6 +463,40 @@ void launch_bucket_count(const uint64_t *first, uint64_t n, uint64_t nb, uint64_
         k_bucket_count<<<grid_for(n, 256), 256, 0, s>>>(first, n, nb, nb_map, b0, counts, err);
     }
 }
+// The partition's counts and scatter for a batch of key sets: kBatchBlocks blocks per request, in one launch
+// (a launch per request of 20,000 keys took about 5 and 7 us each, and its host time).
+constexpr uint32_t kBatchBlocks = 16;
+__global__ void k_batch_count(const uint64_t *__restrict__ first, const BatchReq *__restrict__ req,
+                              uint32_t *__restrict__ counts, uint32_t *__restrict__ err) {
+    const BatchReq q = req[blockIdx.x / kBatchBlocks];
+    for (uint64_t i = (blockIdx.x % kBatchBlocks) * (uint64_t)blockDim.x + threadIdx.x; i < q.n;
+         i += kBatchBlocks * (uint64_t)blockDim.x) {
+        const uint64_t b = remap128(first[q.key_off + i], q.nb_map) - q.b0;
+        if (b >= q.nb) atomicOr(err, kErrArg);
+        else atomicAdd(&counts[q.b_first + b], 1u);
+    }
+}
+__global__ void k_batch_scatter(const uint64_t *__restrict__ first, const BatchReq *__restrict__ req,
+                                uint32_t *__restrict__ cursor, uint64_t *__restrict__ sfirst, uint32_t *__restrict__ sidx) {
+    const BatchReq q = req[blockIdx.x / kBatchBlocks];
+    for (uint64_t i = (blockIdx.x % kBatchBlocks) * (uint64_t)blockDim.x + threadIdx.x; i < q.n;
+         i += kBatchBlocks * (uint64_t)blockDim.x) {
+        const uint64_t f = first[q.key_off + i];
+        const uint64_t b = remap128(f, q.nb_map) - q.b0;
+        if (b >= q.nb) continue;  // reported by k_batch_count
+        const uint32_t pos = atomicAdd(&cursor[q.b_first + b], 1u);
+        sfirst[pos] = f;
+        sidx[pos] = (uint32_t)(q.key_off + i);
+    }
+}
+void launch_batch_count(const uint64_t *first, const BatchReq *req, uint32_t nreq, uint32_t *counts, uint32_t *err,
+                        cudaStream_t s) {
+    k_batch_count<<<nreq * kBatchBlocks, 512, 0, s>>>(first, req, counts, err);
+}
+void launch_batch_scatter(const uint64_t *first, const BatchReq *req, uint32_t nreq, uint32_t *cursor, uint64_t *sfirst,
+                          uint32_t *sidx, cudaStream_t s) {
+    k_batch_scatter<<<nreq * kBatchBlocks, 512, 0, s>>>(first, req, cursor, sfirst, sidx);
+}
 void launch_scan_counts(const uint32_t *counts, uint64_t nb, uint64_t *acc, uint32_t *cursor, uint32_t *maxsz,
                         cudaStream_t s) {
     cudaMemsetAsync(maxsz, 0, sizeof(uint32_t), s);
