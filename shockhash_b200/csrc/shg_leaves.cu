@@ -116,9 +116,19 @@ struct Sh1WarpSmem {
     uint8_t xr[64];
 };
 
-// Rotation of the low l bits of v by r (ShockHash.h:299-301).
-__device__ __forceinline__ uint64_t rot_bits(uint64_t v, uint32_t r, uint32_t l) {
-    return r ? ((v << r) | (v >> (l - r))) & ((1ull << l) - 1) : v;
+// Rotation of the low l bits of v by r < l (ShockHash.h:299-301).
+template <class M> __device__ __forceinline__ M rot_bits(M v, uint32_t r, uint32_t l, M all) {
+    return r ? ((v << r) | (v >> (l - r))) & all : v;
+}
+
+// The cells of a staged key under seed offset t (sh1_cells).
+__device__ __forceinline__ void sh1_staged_cells(const SeedKey &k, uint32_t t, uint32_t m, uint32_t &c1, uint32_t &c2) {
+    uint32_t l2, h2;
+    seed_mid(k, t, l2, h2);
+    const uint64_t p = (uint64_t)l2 * kM2Lo;
+    const uint32_t lo = (uint32_t)p, hi = (uint32_t)(p >> 32) + l2 * kM2Hi + h2 * kM2Lo;
+    c1 = fastrange32(lo ^ funnel_r(lo, hi, 31), m / 2);
+    c2 = fastrange32(hi ^ (hi >> 31), (m + 1) / 2) + m / 2;
 }
 
 // ShockHash<L, true>: a leaf of exactly L keys with rotation fitting (ShockHash.h:316-399). Keys
@@ -126,8 +136,14 @@ __device__ __forceinline__ uint64_t rot_bits(uint64_t v, uint32_t r, uint32_t l)
 // hashes with x & ~mask (mask 7 when L > 32, so eight seeds share set A's cells) and set B with x.
 // For r = 0..L-1 the candidate is set B's cells rotated by r: it passes when A's cells and B's
 // rotated cells cover all L cells and the cuckoo graph is a pseudoforest. The answer is the
-// smallest x, then the smallest r (lanes take consecutive x, each lane tries its r in order);
-// the stored code is (x - start_seed) * L + r.
+// smallest x, then the smallest r; the stored code is (x - start_seed) * L + r.
+//
+// Lanes take consecutive x. What bounds a round is the pseudoforest tests: about a third of the seeds
+// have a rotation that covers, and one in thirty of those rotations passes. So the covering pairs (x, r) of
+// a round are put in order first and then tested 32 at a time, one per lane, instead of each lane
+// testing its own while the others wait (ShockHash<30, true>, 2M keys: leaf stage 4.8 -> 1.6 ms). M: 32-bit
+// masks for L <= 32.
+template <class M>
 __device__ bool rotation_leaf(Sh1WarpSmem &sm, uint16_t *cells, LaneUF &uf, int lane, uint32_t m, uint64_t seed0,
                               uint64_t cap_x, uint64_t &code) {
     const unsigned below = (1u << lane) - 1;
@@ -142,73 +158,98 @@ __device__ bool rotation_leaf(Sh1WarpSmem &sm, uint16_t *cells, LaneUF &uf, int 
         nB += __popc(bo);
     }
     __syncwarp();
-    const uint64_t gmask = m > 32 ? 7 : 0;
-    const uint64_t all = (1ull << m) - 1;
-    // cells[k * 32 + lane] = c1 | c2 << 8 of key k under the lane's seed, written by the coverage
-    // pass; with gmask a set-A key's cells sit in the slot of the group lane that hashed it
-    auto pseudoforest = [&](uint32_t r) {
-        uf.init(m);
-        bool ok = true;
-        for (uint32_t k = 0; k < m && ok; k++) {
-            uint32_t c1, c2;
-            if (k < nA) {
-                const uint32_t w = cells[k * 32 + (gmask ? ((lane & ~7) | (k & 7)) : lane)];
-                c1 = w & 0xFF;
-                c2 = w >> 8;
-            } else {
-                const uint32_t w = cells[k * 32 + lane];
-                c1 = ((w & 0xFF) + r) % m;
-                c2 = ((w >> 8) + r) % m;
-            }
-            ok = uf.add(c1, c2);
-        }
-        return ok;
-    };
+    const uint32_t gmask = m > 32 ? 7 : 0;
+    const M all = (M)~(M)0 >> (8 * sizeof(M) - m);
     // Rounds of 32 seeds start at a multiple of 8 (seeds below seed0 in the first round take no
     // part), so with gmask = 7 each aligned group of 8 lanes shares set A's seed: its lanes hash
     // every eighth set-A key and OR their masks together.
-    const uint64_t x_lo = seed0 & ~7ull;
-    for (uint64_t off = 0; off < cap_x + (seed0 - x_lo); off += 32) {
-        const uint64_t x = x_lo + off + lane, xa = x & ~gmask;
+    const uint64_t x_lo = seed0 & ~7ull, end = cap_x + (seed0 - x_lo);
+    auto stage = [&](uint64_t at) {  // the keys for seeds x_lo + at, + at + 1, ...; how many they are good for
+        uint32_t room = kSeedSpan;
+        for (uint32_t k = lane; k < m; k += 32) {
+            const uint64_t z = sm.fkeys[k] + x_lo + at;
+            sm.staged[k] = seed_key(z);
+            room = min(room, seed_room(z));
+        }
+        room = __reduce_min_sync(0xffffffffu, room);
+        __syncwarp();
+        return room;
+    };
+    uint64_t base0 = 0;
+    uint32_t room = stage(0);
+    uint16_t *const win = reinterpret_cast<uint16_t *>(sm.q);  // 32 covering pairs: lane << 8 | r
+    for (uint64_t off = 0; off < end; off += 32) {
+        const bool plain = off - base0 + 32 > room;  // some key's low bits run over in this round
+        const uint32_t t = (uint32_t)(off - base0) + lane;
+        const uint64_t x = x_lo + off + lane;
         const bool live = x >= seed0 && x - seed0 < cap_x;
-        uint64_t a = 0, b = 0;
+        // cells[k * 32 + lane] = c1 | c2 << 8 of key k under the lane's seed; with gmask a set-A key's cells sit
+        // in the slot of the group lane that hashed it
+        auto hash = [&](uint32_t k, uint32_t mask) -> M {
+            uint32_t c1, c2;
+            if (plain) sh1_cells(sm.fkeys[k], x & ~(uint64_t)mask, m, c1, c2);
+            else sh1_staged_cells(sm.staged[k], t & ~mask, m, c1, c2);
+            cells[k * 32 + lane] = (uint16_t)(c1 | c2 << 8);
+            return (M)1 << c1 | (M)1 << c2;
+        };
+        M a = 0, b = 0;
         if (gmask) {
-            for (uint32_t k = lane & 7; k < nA; k += 8) {
-                uint32_t c1, c2;
-                sh1_cells(sm.fkeys[k], xa, m, c1, c2);
-                a |= (1ull << c1) | (1ull << c2);
-                cells[k * 32 + lane] = (uint16_t)(c1 | c2 << 8);
-            }
+            for (uint32_t k = lane & 7; k < nA; k += 8) a |= hash(k, gmask);
             a |= __shfl_xor_sync(0xffffffffu, a, 1);
             a |= __shfl_xor_sync(0xffffffffu, a, 2);
             a |= __shfl_xor_sync(0xffffffffu, a, 4);
         } else {
-            for (uint32_t k = 0; k < nA; k++) {
-                uint32_t c1, c2;
-                sh1_cells(sm.fkeys[k], xa, m, c1, c2);
-                a |= (1ull << c1) | (1ull << c2);
-                cells[k * 32 + lane] = (uint16_t)(c1 | c2 << 8);
-            }
+            for (uint32_t k = 0; k < nA; k++) a |= hash(k, 0);
         }
-        for (uint32_t k = nA; k < m; k++) {
-            uint32_t c1, c2;
-            sh1_cells(sm.fkeys[k], x, m, c1, c2);
-            b |= (1ull << c1) | (1ull << c2);
-            cells[k * 32 + lane] = (uint16_t)(c1 | c2 << 8);
-        }
-        __syncwarp();
-        int rr = -1;
+        for (uint32_t k = nA; k < m; k++) b |= hash(k, 0);
+        M fits = 0;  // rotations with which the lane's seed covers all cells
         if (live)
             for (uint32_t r = 0; r < m; r++)
-                if ((a | rot_bits(b, r, m)) == all && pseudoforest(r)) {
-                    rr = (int)r;
-                    break;
+                if ((a | rot_bits(b, r, m, all)) == all) fits |= (M)1 << r;
+        const uint32_t mine = sizeof(M) == 8 ? __popcll(fits) : __popc((uint32_t)fits);
+        uint32_t incl = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+        uint32_t pos = incl - mine;  // of the lane's first pair still to be tested
+        int src = -1, fr = 0;
+        for (uint32_t q0 = 0; q0 < total && src < 0; q0 += 32) {
+            for (; fits && pos < q0 + 32; pos++) {
+                const uint32_t r = sizeof(M) == 8 ? __ffsll((long long)fits) - 1 : __ffs((int)fits) - 1;
+                fits &= fits - 1;
+                win[pos - q0] = (uint16_t)(lane << 8 | r);
+            }
+            __syncwarp();
+            bool ok = q0 + lane < total;
+            uint32_t from = 0, r = 0;
+            if (ok) {
+                from = win[lane] >> 8;
+                r = win[lane] & 0xFF;
+                uf.init(m);
+                for (uint32_t k = 0; k < m && ok; k++) {
+                    const uint32_t w = cells[k * 32 + (k < nA && gmask ? (from & ~7u) | (k & 7) : from)];
+                    uint32_t c1 = w & 0xFF, c2 = w >> 8;
+                    if (k >= nA) {
+                        c1 += r;
+                        c2 += r;
+                        if (c1 >= m) c1 -= m;
+                        if (c2 >= m) c2 -= m;
+                    }
+                    ok = uf.add(c1, c2);
                 }
-        const unsigned bal = __ballot_sync(0xffffffffu, rr >= 0);  // also orders the cell reads before the next round's writes
-        if (bal) {
-            const int src = __ffs(bal) - 1;
+            }
+            const unsigned bal = __ballot_sync(0xffffffffu, ok);  // also orders the window's reads before its next writes
+            if (bal) {
+                src = __shfl_sync(0xffffffffu, from, __ffs(bal) - 1);
+                fr = __shfl_sync(0xffffffffu, r, __ffs(bal) - 1);
+            }
+        }
+        __syncwarp();  // the cells are read before the next round's are written
+        if (src >= 0) {
             const uint64_t fx = x_lo + off + src - seed0;
-            const int fr = __shfl_sync(0xffffffffu, rr, src);
             if (fx >= cap_x) return false;
             code = fx * m + (uint64_t)fr;
             // orientation: the reference's ordered insertion in set order, then cell order
@@ -219,7 +260,7 @@ __device__ bool rotation_leaf(Sh1WarpSmem &sm, uint16_t *cells, LaneUF &uf, int 
                 for (uint32_t k = 0; k < m && okc; k++) {
                     uint32_t c1, c2;
                     if (k < nA) {
-                        sh1_cells(sm.fkeys[k], xf & ~gmask, m, c1, c2);
+                        sh1_cells(sm.fkeys[k], xf & ~(uint64_t)gmask, m, c1, c2);
                     } else {
                         sh1_cells(sm.fkeys[k], xf, m, c1, c2);
                         c1 = (c1 + fr) % m;
@@ -231,6 +272,10 @@ __device__ bool rotation_leaf(Sh1WarpSmem &sm, uint16_t *cells, LaneUF &uf, int 
             }
             code = __shfl_sync(0xffffffffu, code, 0);
             return code != ~0ull;
+        }
+        if (plain) {
+            base0 = off + 32;
+            room = stage(base0);
         }
     }
     return false;
@@ -290,7 +335,8 @@ __global__ void __launch_bounds__(kLeafWarps * 32) k_leaves_sh1(const Node *__re
             uint64_t cap_x = (1ull << min(nd.g + 10, 40)) / m + 1;
             if (max_trials && max_trials < cap_x) cap_x = max_trials;
             uint64_t code = 0;
-            const bool ok = rotation_leaf(sm, rot_cells + warp * 64 * 32, uf, lane, m, seed0, cap_x, code);
+            const bool ok = m <= 32 ? rotation_leaf<uint32_t>(sm, rot_cells + warp * 64 * 32, uf, lane, m, seed0, cap_x, code)
+                                    : rotation_leaf<uint64_t>(sm, rot_cells + warp * 64 * 32, uf, lane, m, seed0, cap_x, code);
             if (!ok) {
                 if (lane == 0) atomicOr(err, code == ~0ull ? kErrInternal : kErrTrialLimit);
                 continue;
