@@ -89,7 +89,9 @@ __device__ bool cuckoo_insert(int16_t *cell, uint8_t *xr, int e, uint32_t c1, ui
 // Seeds that pass a sieve queue up in seed order for the next one, so that each runs with its lanes
 // filled: the first sieve's survivors are tested for the full coverage 32 at a time (one per lane;
 // leaves of up to kSh1SmallLeaf keys, which expect fewer seeds than a round has, after every round),
-// and the full coverage's for the pseudoforest property side by side once kSh1Drain of them wait.
+// and the full coverage's for the pseudoforest property side by side once a few of them wait (drain_at:
+// four, two for leaves of more than 31 keys; two / four / eight, leaf stage at 1M keys: ShockHash<30> 3.5 / 3.3 / 3.4
+// ms, ShockHash<33> 7.6 / 8.1 / 9.8, ShockHash<40> 41.5 / 43.8 / 47.9).
 //
 // What bounds it: the integer pipes, in the first sieve, which sees every seed. It therefore works on
 // staged keys (SeedKey, shg_common.cuh), looks at one half of the cells only (one range reduction, shift
@@ -97,10 +99,7 @@ __device__ bool cuckoo_insert(int16_t *cell, uint8_t *xr, int e, uint32_t c1, ui
 // can change the lowest bit alone, so the cell is the same unless the product with the half's size
 // lies within one size of a multiple of 2^32. The smallest low word over the keys says whether one
 // does; such a seed (about 1 in 10^6) counts as passing, and the second sieve decides.
-#ifndef SHG_SH1_DRAIN
-#define SHG_SH1_DRAIN 4
-#endif
-constexpr uint32_t kSh1Drain = SHG_SH1_DRAIN;
+constexpr uint32_t kSh1Drain = 4;
 constexpr uint32_t kSh1SmallLeaf = 16;
 constexpr uint32_t kSh1Half = 31 + 64;        // waiting for the full coverage: at most 31, plus one round's 32 x SPL (SPL <= 2)
 constexpr uint32_t kSh1Queue = kSh1Drain + 32;  // fewer than kSh1Drain wait, plus one batch of 32
@@ -385,6 +384,7 @@ __global__ void __launch_bounds__(kLeafWarps * 32) k_leaves_sh1(const Node *__re
             __syncwarp();  // the queue's slots are read before the next round refills them
         };
         // the second sieve: the first n <= 32 waiting seeds, one per lane, against both halves
+        const uint32_t drain_at = m > 31 ? 2 : kSh1Drain;
         uint32_t nhalf = 0;
         auto cover = [&](uint32_t n) {
             const uint64_t off = (uint32_t)lane < n ? sm.half[lane] : 0;
@@ -407,7 +407,7 @@ __global__ void __launch_bounds__(kLeafWarps * 32) k_leaves_sh1(const Node *__re
             if ((uint32_t)lane + 32 < rest) sm.half[32 + lane] = v1;
             nhalf = rest;
             __syncwarp();
-            if (nq >= kSh1Drain) drain();
+            if (nq >= drain_at) drain();
         };
         // the keys staged for seeds seed0 + at, + at + 1, ...; how many such seeds they are good for
         auto stage = [&](uint64_t at) {
