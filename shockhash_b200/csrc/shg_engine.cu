@@ -140,6 +140,7 @@ static void release_pinned(PinnedBlock *b) {
 }
 
 constexpr int kStageThreads = 8;
+constexpr float kHashPending = -1.f;  // a build's hashing time is still to be read from the engine's hash_ev
 struct shg_engine {
     std::vector<PinnedBlock *> pool;
     int device = 0;
@@ -160,7 +161,7 @@ struct shg_engine {
     std::vector<Shapes *> shapes;
     DevBuf plan_offs, ret_scratch, qdone, qorder, split_best, breq;
     HostBuf small;
-    cudaEvent_t ev[8] = {};
+    cudaEvent_t ev[8] = {}, hash_ev[2] = {};
     cudaStream_t stream2 = nullptr;  // leaves of the pipelined mode
     static constexpr int kMaxChunks = 64;
     cudaEvent_t chunk_ev[kMaxChunks] = {};
@@ -218,6 +219,8 @@ struct shg_engine {
             pool.clear();
         }
         for (auto &e : ev)
+            if (e) cudaEventDestroy(e);
+        for (auto &e : hash_ev)
             if (e) cudaEventDestroy(e);
         for (auto &e : chunk_ev)
             if (e) cudaEventDestroy(e);
@@ -871,6 +874,7 @@ shg_status build_batch(shg_engine *e, const shg_params *p, const uint64_t *d_fir
     e->split_launches = 0;
     for (int lv = 0; lv < nlevels; lv++) e->split_launches += level_count[lv] ? 1 : 0;
     e->leaf_scan = work[5];  // the leaf kernel's candidate-scan count (the slot is reported as leaves below)
+    if (hash_ms == kHashPending) cudaEventElapsedTime(&hash_ms, e->hash_ev[0], e->hash_ev[1]);
     float ms[6] = {};
     cudaEventElapsedTime(&ms[0], e->ev[0], e->ev[1]);
     cudaEventElapsedTime(&ms[1], e->ev[1], e->ev[2]);
@@ -1366,20 +1370,22 @@ void shg_engine_destroy(shg_engine *e) {
     delete e;
 }
 
+// A failed build returns only when the copies from the caller's memory that it has queued are done.
+static shg_status settle(shg_engine *e, shg_status st) {
+    if (st != SHG_OK) cudaStreamSynchronize(e->stream);
+    return st;
+}
+
 static shg_status timed_hash_u64(shg_engine *e, const uint64_t *d_keys, uint64_t n, float &ms) {
     CU(e->first.ensure(std::max<uint64_t>(n, 1) * 8));
     CU(e->second.ensure(std::max<uint64_t>(n, 1) * 8));
-    cudaEvent_t a, b;
-    cudaEventCreate(&a);
-    cudaEventCreate(&b);
-    cudaEventRecord(a, e->stream);
+    for (auto &ev : e->hash_ev)
+        if (!ev) CU(cudaEventCreate(&ev));
+    CU(cudaEventRecord(e->hash_ev[0], e->stream));
     launch_spooky_u64(d_keys, n, e->first.as<uint64_t>(), e->second.as<uint64_t>(), e->stream);
-    cudaEventRecord(b, e->stream);
-    cudaEventSynchronize(b);
-    cudaEventElapsedTime(&ms, a, b);
-    cudaEventDestroy(a);
-    cudaEventDestroy(b);
     CU(cudaGetLastError());
+    CU(cudaEventRecord(e->hash_ev[1], e->stream));
+    ms = kHashPending;
     return SHG_OK;
 }
 
@@ -1679,8 +1685,8 @@ shg_status shg_build_u64_device(shg_engine *e, const shg_params *p, const uint64
     CU(cudaSetDevice(e->device));
     float ms = 0;
     st = timed_hash_u64(e, d_keys, n, ms);
-    if (st) return st;
-    return build_core(e, p, e->first.as<uint64_t>(), e->second.as<uint64_t>(), n, out, ms);
+    if (st) return settle(e, st);
+    return settle(e, build_core(e, p, e->first.as<uint64_t>(), e->second.as<uint64_t>(), n, out, ms));
 }
 
 shg_status shg_build_u64(shg_engine *e, const shg_params *p, const uint64_t *keys, uint64_t n, shg_result *out) {
@@ -1692,8 +1698,8 @@ shg_status shg_build_u64(shg_engine *e, const shg_params *p, const uint64_t *key
     if (shg_status cs = h2d_from_host(e, e->in_keys.p, keys, n * 8, e->stream)) return cs;
     float ms = 0;
     st = timed_hash_u64(e, e->in_keys.as<uint64_t>(), n, ms);
-    if (st) return st;
-    return build_core(e, p, e->first.as<uint64_t>(), e->second.as<uint64_t>(), n, out, ms);
+    if (st) return settle(e, st);
+    return settle(e, build_core(e, p, e->first.as<uint64_t>(), e->second.as<uint64_t>(), n, out, ms));
 }
 
 shg_status shg_build_batch_u64(shg_engine *e, const shg_params *p, const uint64_t *const *keys, const uint64_t *n,
@@ -1713,8 +1719,9 @@ shg_status shg_build_batch_u64(shg_engine *e, const shg_params *p, const uint64_
     if (shg_status cs = h2d_segments(e, e->in_keys.p, segs, e->stream)) return cs;
     float ms = 0;
     st = timed_hash_u64(e, e->in_keys.as<uint64_t>(), total, ms);
-    if (st) return st;
-    return build_batch(e, p, e->first.as<uint64_t>(), e->second.as<uint64_t>(), std::vector<uint64_t>(n, n + nreq), outs, ms);
+    if (st) return settle(e, st);
+    return settle(e, build_batch(e, p, e->first.as<uint64_t>(), e->second.as<uint64_t>(), std::vector<uint64_t>(n, n + nreq), outs,
+                                 ms));
 }
 
 static shg_status hash_strings_dev(shg_engine *e, const char *bytes, const uint64_t *offsets, uint64_t n, float &ms) {
@@ -1729,18 +1736,14 @@ shg_status hash_strings_into(shg_engine *e, const char *bytes, const uint64_t *o
     CU(e->second.ensure(std::max<uint64_t>(n, 1) * 8));
     if (shg_status cs = h2d_from_host(e, e->in_bytes.p, bytes, nbytes, e->stream)) return cs;
     if (shg_status cs = h2d_from_host(e, e->in_offsets.p, offsets, (n + 1) * 8, e->stream)) return cs;
-    cudaEvent_t a, b;
-    cudaEventCreate(&a);
-    cudaEventCreate(&b);
-    cudaEventRecord(a, e->stream);
+    for (auto &ev : e->hash_ev)
+        if (!ev) CU(cudaEventCreate(&ev));
+    CU(cudaEventRecord(e->hash_ev[0], e->stream));
     launch_spooky_strings(e->in_bytes.as<uint8_t>(), e->in_offsets.as<uint64_t>(), n, e->first.as<uint64_t>(),
                           e->second.as<uint64_t>(), e->stream);
-    cudaEventRecord(b, e->stream);
-    cudaEventSynchronize(b);
-    cudaEventElapsedTime(&ms, a, b);
-    cudaEventDestroy(a);
-    cudaEventDestroy(b);
     CU(cudaGetLastError());
+    CU(cudaEventRecord(e->hash_ev[1], e->stream));
+    ms = kHashPending;
     return SHG_OK;
 }
 
@@ -1753,8 +1756,8 @@ shg_status shg_build_strings(shg_engine *e, const shg_params *p, const char *byt
     CU(cudaSetDevice(e->device));
     float ms = 0;
     st = hash_strings_dev(e, bytes, offsets, n, ms);
-    if (st) return st;
-    return build_core(e, p, e->first.as<uint64_t>(), e->second.as<uint64_t>(), n, out, ms);
+    if (st) return settle(e, st);
+    return settle(e, build_core(e, p, e->first.as<uint64_t>(), e->second.as<uint64_t>(), n, out, ms));
 }
 
 shg_status shg_hash_strings(shg_engine *e, const char *bytes, const uint64_t *offsets, uint64_t n, uint64_t *first,
