@@ -132,6 +132,14 @@ SHG_HD uint32_t seed_hi_product(const SeedKey &k, uint32_t t) {
     seed_mid(k, t, l2, h2);
     return mulhi32(l2, kM2Lo) + l2 * kM2Hi + h2 * kM2Lo;
 }
+// The low word of remix(z + t).
+SHG_HD uint32_t seed_lo(const SeedKey &k, uint32_t t) {
+    uint32_t l2, h2;
+    seed_mid(k, t, l2, h2);
+    const uint64_t p = (uint64_t)l2 * kM2Lo;
+    const uint32_t lo = (uint32_t)p, hi = (uint32_t)(p >> 32) + l2 * kM2Hi + h2 * kM2Lo;
+    return lo ^ funnel_r(lo, hi, 31);
+}
 // The low 16 bits of remix(z + t) at bits 15..30, other bits below and 0 above.
 SHG_HD uint32_t seed_low16_at30(const SeedKey &k, uint32_t t) {
     uint32_t l2, h2;

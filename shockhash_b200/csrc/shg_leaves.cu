@@ -87,7 +87,7 @@ __device__ bool cuckoo_insert(int16_t *cell, uint8_t *xr, int e, uint32_t c1, ui
 
 // ------------------------------------------------------------------ original ShockHash leaves
 // Seeds that pass a sieve queue up in seed order for the next one, so that each runs with its lanes
-// filled: the first sieve's survivors are tested for the full coverage 32 at a time (one per lane;
+// filled: the first sieve's survivors are tested for the other half's coverage 32 at a time (one per lane;
 // leaves of up to kSh1SmallLeaf keys, which expect fewer seeds than a round has, after every round),
 // and the full coverage's for the pseudoforest property side by side once a few of them wait (drain_at:
 // four, two for leaves of more than 31 keys; two / four / eight, leaf stage at 1M keys: ShockHash<30> 3.5 / 3.3 / 3.4
@@ -101,6 +101,7 @@ __device__ bool cuckoo_insert(int16_t *cell, uint8_t *xr, int e, uint32_t c1, ui
 // does; such a seed (about 1 in 10^6) counts as passing, and the second sieve decides.
 constexpr uint32_t kSh1Drain = 4;
 constexpr uint32_t kSh1SmallLeaf = 16;
+constexpr uint64_t kSh1Unsure = 1ull << 63;  // on a waiting seed offset (below 2^41): the second half is to be checked
 constexpr uint32_t kSh1Half = 31 + 64;        // waiting for the full coverage: at most 31, plus one round's 32 x SPL (SPL <= 2)
 constexpr uint32_t kSh1Queue = kSh1Drain + 32;  // fewer than kSh1Drain wait, plus one batch of 32
 
@@ -383,18 +384,32 @@ __global__ void __launch_bounds__(kLeafWarps * 32) k_leaves_sh1(const Node *__re
             nq = 0;
             __syncwarp();  // the queue's slots are read before the next round refills them
         };
-        // the second sieve: the first n <= 32 waiting seeds, one per lane, against both halves
+        // the second sieve: the first n <= 32 waiting seeds, one per lane, against the first half's cells (and,
+        // where the first sieve was not sure, the second half's). Waiting seeds are within the staged keys'
+        // span, but for those of a round hashed in plain form.
         const uint32_t drain_at = m > 31 ? 2 : kSh1Drain;
         uint32_t nhalf = 0;
-        auto cover = [&](uint32_t n) {
-            const uint64_t off = (uint32_t)lane < n ? sm.half[lane] : 0;
-            uint32_t c1m = 0, c2m = 0;
-            for (uint32_t k = 0; k < m; k++) {
-                const uint64_t r = remix(sm.keys[k] + seed0 + off);
-                c1m |= 1u << fastrange32((uint32_t)r, h1);
-                c2m |= 1u << fastrange32((uint32_t)(r >> 32), h2);
+        uint64_t base0 = 0;  // the keys are staged for seed0 + base0 and the seeds after it
+        auto cover = [&](uint32_t n, bool plain) {
+            const uint64_t entry = (uint32_t)lane < n ? sm.half[lane] : base0, off = entry & ~kSh1Unsure;
+            uint32_t c1m = 0;
+            if (!plain) {
+                const uint32_t t = (uint32_t)(off - base0);
+#pragma unroll 4
+                for (uint32_t k = 0; k < m; k++) c1m |= 1u << fastrange32(seed_lo(sm.staged[k], t), h1);
             }
-            const bool ok = (uint32_t)lane < n && c1m == all1 && c2m == all2;
+            bool ok = (uint32_t)lane < n && (plain || c1m == all1);
+            if (ok && (plain || (entry & kSh1Unsure))) {
+                uint32_t c2m = 0;
+                c1m = 0;
+                for (uint32_t k = 0; k < m; k++) {
+                    const uint64_t r = remix(sm.keys[k] + seed0 + off);
+                    c1m |= 1u << fastrange32((uint32_t)r, h1);
+                    c2m |= 1u << fastrange32((uint32_t)(r >> 32), h2);
+                }
+                ok = c1m == all1 && c2m == all2;
+            }
+            __syncwarp();
             const unsigned bal = __ballot_sync(0xffffffffu, ok);
             if (ok) sm.q[nq + __popc(bal & below)] = off;
             nq += __popc(bal);
@@ -421,7 +436,6 @@ __global__ void __launch_bounds__(kLeafWarps * 32) k_leaves_sh1(const Node *__re
             __syncwarp();
             return room;
         };
-        uint64_t base0 = 0;
         uint32_t room = stage(0);
         const uint32_t batch = m <= kSh1SmallLeaf ? 1 : 32;
         // SPL seeds per lane (x, x + 32, ...): one shared-memory key read feeds SPL evaluations.
@@ -439,21 +453,22 @@ __global__ void __launch_bounds__(kLeafWarps * 32) k_leaves_sh1(const Node *__re
 #pragma unroll
                     for (int t = 0; t < SPL; t++)
                         mask[t] |= 1u << fastrange32((uint32_t)(remix(sm.keys[k] + seed0 + base + lane + 32 * t) >> 32), h2);
-                base0 = base + kStep;
-                __syncwarp();
-                room = stage(base0);
             }
 #pragma unroll
             for (int t = 0; t < SPL; t++) {  // seeds in order: all lanes' x + 32 t before x + 32 (t + 1)
-                const bool ok = sh1_half_passes(mask[t], low[t], all2, h2);
+                const bool sure = (mask[t] & all2) == all2 && low[t] >= 2 * h2, ok = sh1_half_passes(mask[t], low[t], all2, h2);
                 const unsigned bal = __ballot_sync(0xffffffffu, ok);
-                if (ok) sm.half[nhalf + __popc(bal & below)] = base + 32 * t + lane;
+                if (ok) sm.half[nhalf + __popc(bal & below)] = (base + 32 * t + lane) | (sure ? 0 : kSh1Unsure);
                 nhalf += __popc(bal);
             }
             __syncwarp();
-            while (found == ~0ull && nhalf >= batch) cover(min(nhalf, 32u));
+            while (found == ~0ull && nhalf >= (plain ? 1 : batch)) cover(min(nhalf, 32u), plain);
+            if (plain) {
+                base0 = base + kStep;
+                room = stage(base0);
+            }
         }
-        while (found == ~0ull && nhalf) cover(min(nhalf, 32u));  // what still waits (the trial limit, or BLOCK)
+        while (found == ~0ull && nhalf) cover(min(nhalf, 32u), false);  // what still waits (the trial limit, or BLOCK)
         if (found == ~0ull && nq) drain();
         if constexpr (BLOCK) {
             if (lane == 0 && found != ~0ull) atomicMin(&block_best, (unsigned long long)found);

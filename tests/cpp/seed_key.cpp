@@ -44,7 +44,8 @@ int main() {
     for (int i = 0; i < 200000; i++) {  // the high word of the second product
         const uint64_t z = rng();
         const uint32_t t = (uint32_t)(rng() % seed_room(z)), hi = seed_hi_product(seed_key(z), t);
-        if ((hi ^ (hi >> 31)) != (uint32_t)(remix(z + t) >> 32)) return printf("hi z %llx\n", (unsigned long long)z), 1;
+        if ((hi ^ (hi >> 31)) != (uint32_t)(remix(z + t) >> 32) || seed_lo(seed_key(z), t) != (uint32_t)remix(z + t))
+            return printf("words z %llx\n", (unsigned long long)z), 1;
     }
     printf("ok\n");
     return 0;
