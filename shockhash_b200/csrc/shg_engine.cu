@@ -598,7 +598,7 @@ shg_status build_batch(shg_engine *e, const shg_params *p, const uint64_t *d_fir
     // The work-queue schedule: bipartite leaves of up to 64 keys (other builds take the level schedule). By
     // default only in the middle of the range, where it hides the ends of the level launches without
     // filling the chip many times: level / queue, 1,000 keys 0.55 / 1.39 ms, 300,000 keys 2.7 / 3.1, 1M
-    // keys 6.4 / 6.1, 10M keys 44.6 / 47.2, 20M keys 87.4 / 93.4. Its blocks hold the leaf search's shared
+    // keys 6.1 / 5.8, 10M keys 43.5 / 45.7, 20M keys 86.8 / 92. Its blocks hold the leaf search's shared
     // memory and registers, 24 warps per SM, during the splits too, and the two codes share the
     // instruction cache.
     const bool queue = p->variant == SHG_SHOCKHASH2 && p->leaf_size <= 64 &&
