@@ -16,6 +16,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <new>
 #include <string>
 #include <thread>
 #include <vector>
@@ -272,20 +273,19 @@ struct HostSeg {
     const void *src;
     size_t bytes;
 };
-shg_status h2d_segments(shg_engine *e, void *dst, const std::vector<HostSeg> &segs, cudaStream_t s) {
-    std::vector<size_t> start(segs.size() + 1, 0);
-    for (size_t i = 0; i < segs.size(); i++) start[i + 1] = start[i] + segs[i].bytes;
-    const size_t bytes = start.back();
+// segs[0 .. nseg) back to back at dst; start[i]: the bytes before segment i, start[nseg] all of them.
+shg_status h2d_segments(shg_engine *e, void *dst, const HostSeg *segs, const size_t *start, size_t nseg, cudaStream_t s) {
+    const size_t bytes = start[nseg];
     if (!bytes) return SHG_OK;
-    bool stage = segs.size() > 1 ? bytes >= (64u << 10) : bytes >= kStageMin;
-    for (size_t i = 0; i < segs.size() && stage; i++) stage = !segs[i].bytes || !is_pinned(segs[i].src);
+    bool stage = nseg > 1 ? bytes >= (64u << 10) : bytes >= kStageMin;
+    for (size_t i = 0; i < nseg && stage; i++) stage = !segs[i].bytes || !is_pinned(segs[i].src);
     if (stage && !e->stage && cudaHostAlloc(&e->stage, kStageThreads * 2 * kStagePiece, cudaHostAllocDefault) != cudaSuccess) {
         e->stage = nullptr;  // no pinned memory to spare: copy directly
         cudaGetLastError();
         stage = false;
     }
     if (!stage) {
-        for (size_t i = 0; i < segs.size(); i++)
+        for (size_t i = 0; i < nseg; i++)
             if (segs[i].bytes) CU(cudaMemcpyAsync((char *)dst + start[i], segs[i].src, segs[i].bytes, cudaMemcpyHostToDevice, s));
         return SHG_OK;
     }
@@ -304,7 +304,7 @@ shg_status h2d_segments(shg_engine *e, void *dst, const std::vector<HostSeg> &se
             char *const buf = (char *)e->stage + b * kStagePiece;
             if ((st = cudaEventSynchronize(e->stage_ev[b])) != cudaSuccess) break;  // the copy that last read this buffer
             const size_t lo = piece * kStagePiece, hi = std::min(bytes, lo + kStagePiece);
-            size_t i = std::upper_bound(start.begin(), start.end(), lo) - start.begin() - 1;
+            size_t i = std::upper_bound(start, start + nseg + 1, lo) - start - 1;
             for (size_t at = lo; at < hi; i++) {
                 const size_t end = std::min(hi, start[i + 1]);
                 if (end > at) memcpy(buf + (at - lo), (const char *)segs[i].src + (at - start[i]), end - at);
@@ -320,7 +320,9 @@ shg_status h2d_segments(shg_engine *e, void *dst, const std::vector<HostSeg> &se
     return SHG_OK;
 }
 shg_status h2d_from_host(shg_engine *e, void *dst, const void *src, size_t bytes, cudaStream_t s) {
-    return h2d_segments(e, dst, std::vector<HostSeg>{{src, bytes}}, s);
+    const HostSeg seg{src, bytes};
+    const size_t start[2] = {0, bytes};
+    return h2d_segments(e, dst, &seg, start, 1, s);
 }
 
 PinnedBlock *acquire_pinned(shg_engine *e, size_t bytes, int refs = 1) {
@@ -1714,9 +1716,17 @@ shg_status shg_build_batch_u64(shg_engine *e, const shg_params *p, const uint64_
     if (st) return st;
     CU(cudaSetDevice(e->device));
     CU(e->in_keys.ensure(std::max<uint64_t>(total, 1) * 8));
-    std::vector<HostSeg> segs(nreq);
-    for (uint64_t r = 0; r < nreq; r++) segs[r] = HostSeg{keys[r], n[r] * 8};
-    if (shg_status cs = h2d_segments(e, e->in_keys.p, segs, e->stream)) return cs;
+    try {
+        std::vector<HostSeg> segs(nreq);
+        std::vector<size_t> start(nreq + 1, 0);
+        for (uint64_t r = 0; r < nreq; r++) {
+            segs[r] = HostSeg{keys[r], n[r] * 8};
+            start[r + 1] = start[r] + segs[r].bytes;
+        }
+        if (shg_status cs = h2d_segments(e, e->in_keys.p, segs.data(), start.data(), nreq, e->stream)) return cs;
+    } catch (const std::bad_alloc &) {
+        return fail(SHG_ERR_OOM, "host allocation failed");
+    }
     float ms = 0;
     st = timed_hash_u64(e, e->in_keys.as<uint64_t>(), total, ms);
     if (st) return settle(e, st);
