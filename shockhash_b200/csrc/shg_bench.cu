@@ -55,22 +55,26 @@ template <bool SIMD> void launch_peak_split(int nt, int blocks, uint64_t iters, 
 }
 
 // The original leaf search's first sieve as the leaf kernel runs it, alone: a leaf of h1 + h2 staged keys
-// in shared memory, lanes on consecutive seeds, two seeds per lane per key read, the masks compared after
-// each round; no later sieves. `iters` key reads per thread, rounded up to whole rounds (the caller counts
-// the rounded number).
+// in shared memory, two pairs of consecutive seeds per lane, the masks compared after each round; no later
+// sieves. `iters` pairs of evaluations per thread, rounded up to whole rounds (the caller counts the rounded
+// number).
 __global__ void __launch_bounds__(kPeakThreads) k_int_peak_sh1(uint64_t iters, uint32_t h1, uint32_t h2,
                                                                unsigned long long *sink) {
     __shared__ shg::SeedKey keys[64];
-    for (int i = threadIdx.x; i < 64; i += blockDim.x)
+    __shared__ uint2 delta[64];
+    for (int i = threadIdx.x; i < 64; i += blockDim.x) {  // every key even
         keys[i] = shg::seed_key(shg::remix(0x9E3779B97F4A7C15ULL * (i + 1) + blockIdx.x) & ~(uint64_t)(shg::kSeedSpan - 1));
+        const uint64_t d = keys[i].fold & 1 ? 0ull - shg::kRemixM1 : shg::kRemixM1;
+        delta[i] = make_uint2((uint32_t)d, (uint32_t)(d >> 32));
+    }
     __syncthreads();
     const uint32_t m = h1 + h2, all2 = (1u << h2) - 1;
-    uint32_t at = (threadIdx.x >> 5) * 64 + (threadIdx.x & 31), hits = 0;
-    for (uint64_t done = 0; done < iters; done += m, at = (at + 512) & (shg::kSeedSpan / 2 - 1)) {
-        uint32_t mask[2] = {0, 0}, low[2] = {~0u, ~0u};
-        shg::sh1_half_masks<2>(keys, m, h2, at, mask, low);
+    uint32_t at = (threadIdx.x >> 5) * 128, hits = 0;
+    for (uint64_t done = 0; done < iters; done += 2 * m, at = (at + 1024) & (shg::kSeedSpan / 2 - 1)) {
+        uint32_t mask[4], low[4];
+        shg::sh1_half_pairs<2>(keys, delta, m, m, h2, at, mask, low);
 #pragma unroll
-        for (int t = 0; t < 2; t++) hits += shg::sh1_half_passes(mask[t], low[t], all2, h2);
+        for (int t = 0; t < 4; t++) hits += shg::sh1_half_passes(mask[t], low[t], all2, h2);
     }
     sink[blockIdx.x * (uint64_t)blockDim.x + threadIdx.x] = hits;
 }
@@ -208,7 +212,7 @@ int shg_int_peak_kind(int device, int kind, uint64_t iters, double *evals_per_s,
     } else if (kind == 20) {
         per_iter = shg::sh2_op_peak_per_iter(6);
     } else if (kind == 1) {
-        timed_iters = (iters + 39) / 40 * 40;  // whole rounds of the 40-key leaf
+        timed_iters = (iters + 79) / 80 * 80;  // whole rounds of the 40-key leaf, two pairs of seeds each
     } else if (kind == 2) {
         timed_iters = (iters + 63) / 64 * 64;  // whole rounds of the 64-key leaf
     } else {

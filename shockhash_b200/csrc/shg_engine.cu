@@ -31,7 +31,7 @@ uint64_t sh2_scratch_bytes(uint32_t smax, uint32_t cmax, int max_leaf);
 void launch_leaves_sh1_ctr(const Node *nodes, const uint32_t *ids, uint32_t count, const uint64_t *keys, uint64_t *codes,
                            uint64_t *rib_keys, uint8_t *rib_bits, uint64_t max_trials, uint32_t *err,
                            unsigned long long *work, unsigned int *ctr, int grid, cudaStream_t s, uint32_t rot_leaf = 0,
-                           int spl = 2, bool block = false);
+                           int spl = 2, bool block = false, int leaf = 0);
 void launch_leaves_sh2_ctr(const Node *nodes, const uint32_t *ids, uint32_t count, const uint64_t *keys, uint64_t *codes,
                            uint8_t *rib_bits, uint8_t *scratch, uint64_t scratch_per_warp, uint32_t smax, uint32_t cmax,
                            uint32_t *err, unsigned long long *work, unsigned int *ctr, int grid, cudaStream_t s,
@@ -697,7 +697,7 @@ shg_status build_batch(shg_engine *e, const shg_params *p, const uint64_t *d_fir
             launch_leaves_sh1_ctr(e->nodes.as<Node>(), d_ids + leaf_off + a, (uint32_t)(b - a), e->keys.as<uint64_t>(),
                                   e->codes.as<uint64_t>(), e->rib_keys.as<uint64_t>(), e->rib_bits.as<uint8_t>(), p->max_trials,
                                   &misc->err, misc->work, &misc->leaf_ctr, grid, st,
-                                  is_rotation(p->variant) ? (uint32_t)p->leaf_size : 0, tun.sh1_spl, sh1_block);
+                                  is_rotation(p->variant) ? (uint32_t)p->leaf_size : 0, tun.sh1_spl, sh1_block, p->leaf_size);
         launches++;
     };
     if (queue) {

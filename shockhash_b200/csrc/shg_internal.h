@@ -162,7 +162,7 @@ struct Tuning {
     SplitTuning split;
     int leaf_bps = 0;    // leaf grid in blocks per SM (0: as many as shared memory allows, at most 8)
     int leaf_minb = 6;   // bipartite leaves of up to 64 keys: launch bound of 4, 6 or 8 blocks per SM
-    int sh1_spl = 2;     // original leaves: seeds per lane, 1 or 2
+    int sh1_spl = 2;     // original leaves: seeds (or pairs of them) per lane, 1 or 2
     int queue_lag = 8;   // work-queue item order: lag between a bucket's levels in rounds of the grid
                          // (0: none, the levels one after another and the leaves last; 1..64)
 };

@@ -1,8 +1,7 @@
 // ShockHash leaf searches, one warp per leaf, leaves pulled from a device counter.
 //
-// Original ShockHash (ShockHash.h:404-434): lanes take consecutive seeds x (SPL per lane, x, x + 32,
-// ..., per round of 32 * SPL); a lane's seed passes
-// when the two candidate cells of all m keys cover all m cells and the cuckoo graph
+// Original ShockHash (ShockHash.h:404-434): lanes take consecutive seeds x, or pairs of them; a lane's seed
+// passes when the two candidate cells of all m keys cover all m cells and the cuckoo graph
 // (cells = vertices, keys = edges) is a pseudoforest. Seeds go through three sieves in seed order:
 // the second-half cells of all keys cover their half (one key in 8 to 20 does, for leaves of 30 to 40
 // keys), both halves are covered, pseudoforest. The pseudoforest test is a per-lane
@@ -102,15 +101,18 @@ __device__ bool cuckoo_insert(int16_t *cell, uint8_t *xr, int e, uint32_t c1, ui
 constexpr uint32_t kSh1Drain = 4;
 constexpr uint32_t kSh1SmallLeaf = 16;
 constexpr uint64_t kSh1Unsure = 1ull << 63;  // on a waiting seed offset (below 2^41): the second half is to be checked
-constexpr uint32_t kSh1Half = 31 + 64;        // waiting for the full coverage: at most 31, plus one round's 32 x SPL (SPL <= 2)
+constexpr uint32_t kSh1Half = 31 + 128;       // waiting for the full coverage: at most 31, plus one round's (at most 128)
 constexpr uint32_t kSh1Queue = kSh1Drain + 32;  // fewer than kSh1Drain wait, plus one batch of 32
 
 struct Sh1WarpSmem {
-    SeedKey staged[64];     // the keys under the first seed of the current span
+    SeedKey staged[64];     // the keys under the first seed of the current span (PAIRS: even ones first)
     uint64_t half[kSh1Half];  // seed offsets that cover the second half, ascending
     uint64_t q[kSh1Queue];  // coverage-passing seed offsets, ascending
     uint64_t keys[64];
-    uint64_t fkeys[64];  // rotation fitting: even keys in order, odd keys from the back
+    union {
+        uint64_t fkeys[64];  // rotation fitting: even keys in order, odd keys from the back
+        uint2 delta[64];     // PAIRS: what a key's first product changes by from an even seed to the next
+    };
     uint8_t uf[64 * 32];
     int16_t cell[64];
     uint8_t xr[64];
@@ -281,12 +283,14 @@ __device__ bool rotation_leaf(Sh1WarpSmem &sm, uint16_t *cells, LaneUF &uf, int 
     return false;
 }
 
-// SPL: seeds per lane and round (1 or 2; a tuning parameter, the same seed is found either way).
+// SPL: seeds per lane and round, or pairs of them with PAIRS (1 or 2; a tuning parameter, the same seed is found
+// either way).
+// PAIRS (sh1_pairs, below): the first sieve takes a key under two consecutive seeds at a time (sh1_half_pairs).
 // BLOCK: the block's warps search a leaf together (not with rotation fitting): warp w takes the rounds w,
 // w + kLeafWarps, ..., on its own, and goes on until its next round begins past the smallest passing seed
 // any of them has found, so every smaller seed has been tried. One leaf then takes a quarter of the time,
 // and with it the launch's tail, in which the last leaves run alone.
-template <int SPL, bool BLOCK>
+template <int SPL, bool BLOCK, bool PAIRS>
 __global__ void __launch_bounds__(kLeafWarps * 32) k_leaves_sh1(const Node *__restrict__ nodes, const uint32_t *__restrict__ ids,
                                                                 uint32_t count, const uint64_t *__restrict__ keys,
                                                                 uint64_t *__restrict__ codes, uint64_t *__restrict__ rib_keys,
@@ -413,24 +417,46 @@ __global__ void __launch_bounds__(kLeafWarps * 32) k_leaves_sh1(const Node *__re
             const unsigned bal = __ballot_sync(0xffffffffu, ok);
             if (ok) sm.q[nq + __popc(bal & below)] = off;
             nq += __popc(bal);
-            // the rest moves up (at most 63 entries)
+            // the rest moves up
             const uint32_t rest = nhalf - n;
-            const uint64_t v0 = (uint32_t)lane < rest ? sm.half[n + lane] : 0;
-            const uint64_t v1 = (uint32_t)lane + 32 < rest ? sm.half[n + 32 + lane] : 0;
-            __syncwarp();
-            if ((uint32_t)lane < rest) sm.half[lane] = v0;
-            if ((uint32_t)lane + 32 < rest) sm.half[32 + lane] = v1;
+            for (uint32_t i = 0; i < rest; i += 32) {
+                const uint64_t v = i + lane < rest ? sm.half[n + i + lane] : 0;
+                __syncwarp();
+                if (i + lane < rest) sm.half[i + lane] = v;
+                __syncwarp();
+            }
             nhalf = rest;
-            __syncwarp();
             if (nq >= drain_at) drain();
         };
         // the keys staged for seeds seed0 + at, + at + 1, ...; how many such seeds they are good for
+        uint32_t evens = 0;
         auto stage = [&](uint64_t at) {
-            uint32_t room = kSeedSpan;
-            for (uint32_t k = lane; k < m; k += 32) {
-                const uint64_t z = sm.keys[k] + seed0 + at;
-                sm.staged[k] = seed_key(z);
-                room = min(room, seed_room(z));
+            uint32_t room = kSeedSpan, odds = 0;
+            if constexpr (!PAIRS) {
+                for (uint32_t k = lane; k < m; k += 32) {
+                    const uint64_t z = sm.keys[k] + seed0 + at;
+                    sm.staged[k] = seed_key(z);
+                    room = min(room, seed_room(z));
+                }
+                room = __reduce_min_sync(0xffffffffu, room);
+                __syncwarp();
+                return room;
+            }
+            evens = 0;
+            for (uint32_t k0 = 0; k0 < m; k0 += 32) {
+                const uint32_t k = k0 + lane;
+                const uint64_t z = k < m ? sm.keys[k] + seed0 + at : 0;
+                const unsigned be = __ballot_sync(0xffffffffu, k < m && !(z & 1)), bo = __ballot_sync(0xffffffffu, k < m && (z & 1));
+                if (k < m) {
+                    const uint32_t slot = z & 1 ? m - 1 - (odds + __popc(bo & below)) : evens + __popc(be & below);
+                    const SeedKey key = seed_key(z);
+                    const uint64_t d = key.fold & 1 ? 0ull - kRemixM1 : kRemixM1;
+                    sm.staged[slot] = key;
+                    sm.delta[slot] = make_uint2((uint32_t)d, (uint32_t)(d >> 32));
+                    room = min(room, seed_room(z));
+                }
+                evens += __popc(be);
+                odds += __popc(bo);
             }
             room = __reduce_min_sync(0xffffffffu, room);
             __syncwarp();
@@ -438,28 +464,44 @@ __global__ void __launch_bounds__(kLeafWarps * 32) k_leaves_sh1(const Node *__re
         };
         uint32_t room = stage(0);
         const uint32_t batch = m <= kSh1SmallLeaf ? 1 : 32;
-        // SPL seeds per lane (x, x + 32, ...): one shared-memory key read feeds SPL evaluations.
-        constexpr uint32_t kStep = 32 * SPL * (BLOCK ? kLeafWarps : 1);
-        for (uint64_t base = BLOCK ? 32 * SPL * warp : 0; base < cap && found == ~0ull; base += kStep) {
+        // one shared-memory key read feeds the evaluations of all the lane's seeds
+        constexpr int kIn = PAIRS ? 2 : 1, kLane = SPL * kIn;
+        constexpr uint32_t kSeeds = PAIRS ? sh1_pair_seeds(SPL) : 32 * SPL, kStep = kSeeds * (BLOCK ? kLeafWarps : 1);
+        for (uint64_t base = BLOCK ? kSeeds * warp : 0; base < cap && found == ~0ull; base += kStep) {
             if (BLOCK && base > *(volatile unsigned long long *)&block_best) break;
-            uint32_t mask[SPL], low[SPL];
+            uint32_t mask[kLane], low[kLane];
 #pragma unroll
-            for (int t = 0; t < SPL; t++) mask[t] = 0, low[t] = ~0u;
-            const bool plain = base - base0 + 32 * SPL > room;
+            for (int i = 0; i < kLane; i++) mask[i] = 0, low[i] = ~0u;
+            const bool plain = base - base0 + 32 * kLane > room;
             if (!plain) {
-                sh1_half_masks<SPL>(sm.staged, m, h2, (uint32_t)(base - base0) + lane, mask, low);
+                if constexpr (!PAIRS) sh1_half_masks<SPL>(sm.staged, m, h2, (uint32_t)(base - base0) + lane, mask, low);
+                else sh1_half_pairs<SPL>(sm.staged, sm.delta, evens, m, h2, (uint32_t)(base - base0), mask, low);
             } else {  // some key's low bits run over in this round
                 for (uint32_t k = 0; k < m; k++)
 #pragma unroll
-                    for (int t = 0; t < SPL; t++)
-                        mask[t] |= 1u << fastrange32((uint32_t)(remix(sm.keys[k] + seed0 + base + lane + 32 * t) >> 32), h2);
+                    for (int i = 0; i < kLane; i++) {
+                        const uint64_t x = seed0 + base + 32 * kIn * (i / kIn) + kIn * lane + i % kIn;
+                        mask[i] |= 1u << fastrange32((uint32_t)(remix(sm.keys[k] + x) >> 32), h2);
+                    }
             }
 #pragma unroll
-            for (int t = 0; t < SPL; t++) {  // seeds in order: all lanes' x + 32 t before x + 32 (t + 1)
-                const bool sure = (mask[t] & all2) == all2 && low[t] >= 2 * h2, ok = sh1_half_passes(mask[t], low[t], all2, h2);
-                const unsigned bal = __ballot_sync(0xffffffffu, ok);
-                if (ok) sm.half[nhalf + __popc(bal & below)] = (base + 32 * t + lane) | (sure ? 0 : kSh1Unsure);
-                nhalf += __popc(bal);
+            for (int p = 0; p < SPL; p++) {  // seeds in order: all lanes' p-th seed or pair before the next
+                const uint32_t first = kIn * (32 * p + lane);
+                bool ok[kIn];
+                uint32_t pos = nhalf;
+#pragma unroll
+                for (int i = 0; i < kIn; i++) {
+                    ok[i] = first + i < kSeeds && sh1_half_passes(mask[kIn * p + i], low[kIn * p + i], all2, h2);
+                    const unsigned bal = __ballot_sync(0xffffffffu, ok[i]);
+                    pos += __popc(bal & below);
+                    nhalf += __popc(bal);
+                }
+#pragma unroll
+                for (int i = 0; i < kIn; i++)
+                    if (ok[i]) {
+                        const bool sure = (mask[kIn * p + i] & all2) == all2 && low[kIn * p + i] >= 2 * h2;
+                        sm.half[pos++] = (base + first + i) | (sure ? 0 : kSh1Unsure);
+                    }
             }
             __syncwarp();
             while (found == ~0ull && nhalf >= (plain ? 1 : batch)) cover(min(nhalf, 32u), plain);
@@ -508,16 +550,27 @@ __global__ void __launch_bounds__(kLeafWarps * 32) k_leaves_sh1(const Node *__re
 
 int leaves_sh1_warps_per_block() { return kLeafWarps; }
 
+// Whether the first sieve works on pairs of seeds: a seed costs it less, but a round has twice the seeds, and
+// a leaf's last round (last four with a block per leaf) is half wasted; staging costs more, too. It pays
+// where a leaf takes many rounds. Leaf stage, single seeds / pairs: a warp per leaf, leaves of 24 keys (2M
+// keys) 1.73 / 1.91 ms, 26 (4M) 4.76 / 4.92, 28 (4M) 7.04 / 7.02, 29 (4M) 8.81 / 8.65, 30 (1M) 3.23 / 3.14, 30 (4M)
+// 11.15 / 10.88, 33 (8M) 45.3 / 43.7; a block per leaf, 32 (1M) 6.18 / 6.72, 33 (1M) 7.63 / 7.88, 34 (1M) 9.35 / 9.15,
+// 35 (1M) 11.99 / 11.38, 40 (30,000 keys) 3.9 / 3.4, 40 (1M) 42.1 / 39.1, 48 (20,000) 30.4 / 26.5.
+static bool sh1_pairs(int leaf, bool block) { return block ? leaf >= 34 : leaf >= 29; }
+
 void launch_leaves_sh1_ctr(const Node *nodes, const uint32_t *ids, uint32_t count, const uint64_t *keys, uint64_t *codes,
                            uint64_t *rib_keys, uint8_t *rib_bits, uint64_t max_trials, uint32_t *err,
                            unsigned long long *work, unsigned int *ctr, int grid, cudaStream_t s, uint32_t rot_leaf,
-                           int spl, bool block) {
+                           int spl, bool block, int leaf) {
     if (!count) return;
     block = block && !rot_leaf;
     cudaMemsetAsync(ctr, 0, sizeof(unsigned int), s);
     const size_t dyn = rot_leaf ? (size_t)kLeafWarps * 64 * 32 * sizeof(uint16_t) : 0;  // 16 KB per block
-    auto kernel = block ? (spl == 1 ? k_leaves_sh1<1, true> : k_leaves_sh1<2, true>)
-                        : (spl == 1 ? k_leaves_sh1<1, false> : k_leaves_sh1<2, false>);
+    const bool pairs = !rot_leaf && sh1_pairs(leaf, block);
+    auto kernel = block ? (pairs ? (spl == 1 ? k_leaves_sh1<1, true, true> : k_leaves_sh1<2, true, true>)
+                                 : (spl == 1 ? k_leaves_sh1<1, true, false> : k_leaves_sh1<2, true, false>))
+                        : (pairs ? (spl == 1 ? k_leaves_sh1<1, false, true> : k_leaves_sh1<2, false, true>)
+                                 : (spl == 1 ? k_leaves_sh1<1, false, false> : k_leaves_sh1<2, false, false>));
     kernel<<<grid, kLeafWarps * 32, dyn, s>>>(nodes, ids, count, keys, codes, rib_keys, rib_bits, max_trials, err, work, ctr,
                                               rot_leaf);
 }

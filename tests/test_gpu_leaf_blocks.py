@@ -54,3 +54,42 @@ def test_original_block_and_warp_search_agree(engine, leaf, n):
     assert np.array_equal(part.bucket_size_acc, acc[:b1 + 1])
     k = len(part.ribbon_keys)
     assert np.array_equal(part.ribbon_keys, keys[:k]) and np.array_equal(part.ribbon_bits, bits[:k])
+
+
+def second_halves(rng, n, kind):
+    """Distinct second halves: all even, all odd, or short of where their low 30 bits run over under a
+    start seed of depths 0..3 (ShockHash.h:47-49)."""
+    if kind == "over":
+        start = np.array([0x106393c187cae21a, 0x6453cec3f7376937, 0x643e521ddbd2be98, 0x3740c6412f6572cb], dtype=np.uint64)
+        short = rng.integers(1, 3000, size=n).astype(np.uint64) + start[rng.integers(0, 4, size=n)]
+        out = (unique_u64(rng, n) & ~np.uint64(0x3fffffff)) - short
+    else:
+        out = (unique_u64(rng, n) & ~np.uint64(1)) | np.uint64(kind == "odd")
+    assert len(np.unique(out)) == n
+    return out
+
+
+@pytest.mark.parametrize("kind", ["even", "odd", "over"])
+@pytest.mark.parametrize("leaf", [34, 35, 40])
+def test_original_seed_pairs_block_search(engine, port, leaf, kind):
+    # leaves of 34 keys or more, a block per leaf: the first sieve takes seeds in pairs
+    rng = np.random.default_rng(leaf)
+    n = 1000 + leaf // 2
+    first, second = rng.integers(0, 2**64, size=n, dtype=np.uint64), second_halves(rng, n, kind)
+    r, p = engine.build_hash128(shg.SHOCKHASH, leaf, first, second, 500), port.build_hash(shg.SHOCKHASH, leaf, first, second, 500)
+    assert np.array_equal(r.descriptors, p.desc)
+    assert np.array_equal(r.ribbon_keys, p.ribbon_keys) and np.array_equal(r.ribbon_bits, p.ribbon_bits)
+
+
+@pytest.mark.parametrize("kind", ["even", "odd", "over"])
+def test_original_seed_pairs_warp_search(engine, kind):
+    # many leaves of 30 keys (a warp per leaf, seeds in pairs) against a few of them (a block, single seeds)
+    rng = np.random.default_rng(30)
+    n, nb, b1 = 400_000, 200, 3
+    first, second = rng.integers(0, 2**64, size=n, dtype=np.uint64), second_halves(rng, n, kind)
+    whole = engine.build_hash128(shg.SHOCKHASH, 30, first, second, 2000)
+    keys, bits = whole.ribbon_keys.copy(), whole.ribbon_bits.copy()
+    inside = np.array([(int(f) * nb) >> 64 < b1 for f in first])
+    part = engine.build_shard_hash128(shg.SHOCKHASH, 30, first[inside], second[inside], nb, 0, b1, 2000)
+    k = len(part.ribbon_keys)
+    assert np.array_equal(part.ribbon_keys, keys[:k]) and np.array_equal(part.ribbon_bits, bits[:k])
