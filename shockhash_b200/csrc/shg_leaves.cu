@@ -4,8 +4,8 @@
 // passes when the two candidate cells of all m keys cover all m cells and the cuckoo graph
 // (cells = vertices, keys = edges) is a pseudoforest. Seeds go through three sieves in seed order:
 // the second-half cells of all keys cover their half (one key in 8 to 20 does, for leaves of 30 to 40
-// keys), both halves are covered, pseudoforest. The pseudoforest test is a per-lane
-// union-find with a cycle flag per root; the reference inserts into a cuckoo table instead, and
+// keys), both halves are covered, pseudoforest. The pseudoforest test peels the graph (group_peel); the
+// reference inserts into a cuckoo table instead, and
 // ordered cuckoo insertion succeeds exactly when the graph is a pseudoforest, so both accept the
 // same seeds. The coverage mask is kept as two 32-bit halves (first-half and second-half cells).
 // The smallest accepted seed is kept (ballot + find-first-set), then lane 0 replays
@@ -21,46 +21,6 @@
 namespace shg {
 
 constexpr int kLeafWarps = 4;  // warps per block
-
-// ------------------------------------------------------------------ per-lane union-find
-// parent[v * 32 + lane] (bytes) in shared memory; cycle flags of roots in two 64-bit registers.
-struct LaneUF {
-    uint8_t *par;
-    int lane;
-    uint64_t cyc0 = 0, cyc1 = 0;
-    // Root of x with path halving.
-    __device__ __forceinline__ uint32_t find(uint32_t x) {
-        for (;;) {
-            const uint32_t p = par[x * 32 + lane];
-            if (p == x) return x;
-            const uint32_t gp = par[p * 32 + lane];
-            par[x * 32 + lane] = (uint8_t)gp;
-            x = gp;
-        }
-    }
-    __device__ __forceinline__ bool cyc(uint32_t r) const { return ((r < 64 ? cyc0 : cyc1) >> (r & 63)) & 1; }
-    __device__ __forceinline__ void set_cyc(uint32_t r) {
-        if (r < 64) cyc0 |= 1ull << r; else cyc1 |= 1ull << (r & 63);
-    }
-    __device__ __forceinline__ void init(uint32_t n) {
-        for (uint32_t v = 0; v < n; v++) par[v * 32 + lane] = (uint8_t)v;
-        cyc0 = cyc1 = 0;
-    }
-    // Adds edge (u, v); false when a component would get a second cycle.
-    __device__ __forceinline__ bool add(uint32_t u, uint32_t v) {
-        const uint32_t ru = find(u), rv = find(v);
-        if (ru == rv) {
-            if (cyc(ru)) return false;
-            set_cyc(ru);
-            return true;
-        }
-        const bool cu = cyc(ru), cv = cyc(rv);
-        if (cu && cv) return false;
-        par[ru * 32 + lane] = (uint8_t)rv;
-        if (cu) set_cyc(rv);
-        return true;
-    }
-};
 
 // Ordered cuckoo insertion with cycle detection (TinyBinaryCuckooHashTable.h:169-198), run by one
 // thread. cell[c] = key index or -1; xr[e] = c1 ^ c2 of key e. Returns false when the walk returns
@@ -88,9 +48,8 @@ __device__ bool cuckoo_insert(int16_t *cell, uint8_t *xr, int e, uint32_t c1, ui
 // Seeds that pass a sieve queue up in seed order for the next one, so that each runs with its lanes
 // filled: the first sieve's survivors are tested for the other half's coverage 32 at a time (one per lane;
 // leaves of up to kSh1SmallLeaf keys, which expect fewer seeds than a round has, after every round),
-// and the full coverage's for the pseudoforest property side by side once a few of them wait (drain_at:
-// four, two for leaves of more than 31 keys; two / four / eight, leaf stage at 1M keys: ShockHash<30> 3.5 / 3.3 / 3.4
-// ms, ShockHash<33> 7.6 / 8.1 / 9.8, ShockHash<40> 41.5 / 43.8 / 47.9).
+// and the full coverage's for the pseudoforest property four at a time, straight after that (waiting for two /
+// three / four of them: ShockHash<30>, 4M keys 9.0 -> 9.3 / 9.4 / 9.6 ms, ShockHash<40>, 1M 36.1 -> 36.4 / 37.2 / 38.0).
 //
 // What bounds it: the integer pipes, in the first sieve, which sees every seed. It therefore works on
 // staged keys (SeedKey, shg_common.cuh), looks at one half of the cells only (one range reduction, shift
@@ -98,25 +57,80 @@ __device__ bool cuckoo_insert(int16_t *cell, uint8_t *xr, int e, uint32_t c1, ui
 // can change the lowest bit alone, so the cell is the same unless the product with the half's size
 // lies within one size of a multiple of 2^32. The smallest low word over the keys says whether one
 // does; such a seed (about 1 in 10^6) counts as passing, and the second sieve decides.
-constexpr uint32_t kSh1Drain = 4;
 constexpr uint32_t kSh1SmallLeaf = 16;
 constexpr uint64_t kSh1Unsure = 1ull << 63;  // on a waiting seed offset (below 2^41): the second half is to be checked
 constexpr uint32_t kSh1Half = 31 + 128;       // waiting for the full coverage: at most 31, plus one round's (at most 128)
-constexpr uint32_t kSh1Queue = kSh1Drain + 32;  // fewer than kSh1Drain wait, plus one batch of 32
 
 struct Sh1WarpSmem {
     SeedKey staged[64];     // the keys under the first seed of the current span (PAIRS: even ones first)
     uint64_t half[kSh1Half];  // seed offsets that cover the second half, ascending
-    uint64_t q[kSh1Queue];  // coverage-passing seed offsets, ascending
+    uint64_t q[32];         // coverage-passing seed offsets of a batch, ascending
     uint64_t keys[64];
     union {
         uint64_t fkeys[64];  // rotation fitting: even keys in order, odd keys from the back
         uint2 delta[64];     // PAIRS: what a key's first product changes by from an even seed to the next
     };
-    uint8_t uf[64 * 32];
     int16_t cell[64];
     uint8_t xr[64];
 };
+
+// Whether the cuckoo graph of m keys over m cells, all of them covered, is a pseudoforest; a group of 8 lanes
+// tests one graph, the warp four (`live` false: no graph, and false for it). cells(k, c1, c2): the two cells of key
+// k of the group's graph. As there are as many edges as vertices, the graph is a pseudoforest exactly if no
+// component is a tree. So the vertices of degree one are taken off with their edges, all at a time, until there
+// are none: a tree ends in an edge between two of them or in a vertex whose edges all went. They are the
+// vertices seen once, but not twice, in the union of the lanes' edges.
+//
+// Against one lane per graph with a union-find in shared memory, of which few graphs at a time filled few lanes:
+// hashing takes an eighth of the steps, and a turn of the peeling (about five) has no dependent memory access.
+// Leaf stage: ShockHash<16>, 2M keys 0.70 -> 0.49 ms; ShockHash<30>, 4M 10.9 -> 9.0; ShockHash<40>, 1M 39.1 -> 35.4.
+// M: a word with more bits than cells (the top bit carries the lanes' verdicts). E: keys per lane.
+template <class M, int E, class Cells>
+__device__ __forceinline__ bool group_peel(uint32_t m, bool live, const Cells &cells) {
+    constexpr M kTree = (M)1 << (8 * sizeof(M) - 1);
+    M v[E];
+#pragma unroll
+    for (int e = 0; e < E; e++) {
+        const uint32_t k = 8 * e + (threadIdx.x & 7);
+        v[e] = 0;
+        if (live && k < m) {
+            uint32_t c1, c2;
+            cells(k, c1, c2);
+            v[e] = (M)1 << c1 | (M)1 << c2;
+        }
+    }
+    M left = ((M)1 << m) - 1, ones = 0;  // vertices not taken off; those of degree one
+    bool tree = !live;
+    for (;;) {
+        M once = 0, twice = 0;
+#pragma unroll
+        for (int e = 0; e < E; e++) {
+            const M x = v[e] & ones;
+            if (x) {
+                if (x == v[e]) once |= kTree;
+                v[e] = 0;
+            }
+            twice |= once & v[e];
+            once |= v[e];
+        }
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) {
+            const M xo = __shfl_xor_sync(0xffffffffu, once, o), xt = __shfl_xor_sync(0xffffffffu, twice, o);
+            twice |= xt | (once & xo);
+            once |= xo;
+        }
+        left &= ~ones;
+        tree = tree || (once & kTree) || (left & ~once);
+        ones = tree ? 0 : once & ~twice;
+        if (!__any_sync(0xffffffffu, ones != 0)) return !tree;
+    }
+}
+template <class Cells> __device__ __forceinline__ bool group_pseudoforest(uint32_t m, bool live, const Cells &cells) {
+    if (m == 1) return live;  // its two cells are one
+    if (m < 32) return group_peel<uint32_t, 4>(m, live, cells);
+    if (m <= 40) return group_peel<uint64_t, 5>(m, live, cells);
+    return group_peel<uint64_t, 8>(m, live, cells);
+}
 
 // Rotation of the low l bits of v by r < l (ShockHash.h:299-301).
 template <class M> __device__ __forceinline__ M rot_bits(M v, uint32_t r, uint32_t l, M all) {
@@ -142,11 +156,12 @@ __device__ __forceinline__ void sh1_staged_cells(const SeedKey &k, uint32_t t, u
 //
 // Lanes take consecutive x. What bounds a round is the pseudoforest tests: about a third of the seeds
 // have a rotation that covers, and one in thirty of those rotations passes. So the covering pairs (x, r) of
-// a round are put in order first and then tested 32 at a time, one per lane, instead of each lane
-// testing its own while the others wait (ShockHash<30, true>, 2M keys: leaf stage 4.8 -> 1.6 ms). M: 32-bit
+// a round are put in order first and then tested side by side, instead of each lane
+// testing its own while the others wait (ShockHash<30, true>, 2M keys: leaf stage 4.8 -> 1.6 ms), four graphs
+// peeled by groups of lanes (0.86 ms). M: 32-bit
 // masks for L <= 32.
 template <class M>
-__device__ bool rotation_leaf(Sh1WarpSmem &sm, uint16_t *cells, LaneUF &uf, int lane, uint32_t m, uint64_t seed0,
+__device__ bool rotation_leaf(Sh1WarpSmem &sm, uint16_t *cells, int lane, uint32_t m, uint64_t seed0,
                               uint64_t cap_x, uint64_t &code) {
     const unsigned below = (1u << lane) - 1;
     uint32_t nA = 0, nB = 0;
@@ -225,29 +240,27 @@ __device__ bool rotation_leaf(Sh1WarpSmem &sm, uint16_t *cells, LaneUF &uf, int 
                 win[pos - q0] = (uint16_t)(lane << 8 | r);
             }
             __syncwarp();
-            bool ok = q0 + lane < total;
-            uint32_t from = 0, r = 0;
-            if (ok) {
-                from = win[lane] >> 8;
-                r = win[lane] & 0xFF;
-                uf.init(m);
-                for (uint32_t k = 0; k < m && ok; k++) {
-                    const uint32_t w = cells[k * 32 + (k < nA && gmask ? (from & ~7u) | (k & 7) : from)];
-                    uint32_t c1 = w & 0xFF, c2 = w >> 8;
+            for (uint32_t q1 = 0; q1 < 32 && q0 + q1 < total && src < 0; q1 += 4) {
+                const bool live = q0 + q1 + lane / 8 < total;
+                const uint32_t w = live ? win[q1 + lane / 8] : 0, from = w >> 8, r = w & 0xFF;
+                const bool ok = group_pseudoforest(m, live, [&](uint32_t k, uint32_t &c1, uint32_t &c2) {
+                    const uint32_t c = cells[k * 32 + (k < nA && gmask ? (from & ~7u) | (k & 7) : from)];
+                    c1 = c & 0xFF;
+                    c2 = c >> 8;
                     if (k >= nA) {
                         c1 += r;
                         c2 += r;
                         if (c1 >= m) c1 -= m;
                         if (c2 >= m) c2 -= m;
                     }
-                    ok = uf.add(c1, c2);
+                });
+                const unsigned bal = __ballot_sync(0xffffffffu, ok);
+                if (bal) {
+                    src = __shfl_sync(0xffffffffu, from, __ffs(bal) - 1);
+                    fr = __shfl_sync(0xffffffffu, r, __ffs(bal) - 1);
                 }
             }
-            const unsigned bal = __ballot_sync(0xffffffffu, ok);  // also orders the window's reads before its next writes
-            if (bal) {
-                src = __shfl_sync(0xffffffffu, from, __ffs(bal) - 1);
-                fr = __shfl_sync(0xffffffffu, r, __ffs(bal) - 1);
-            }
+            __syncwarp();  // the window is read before it is written again
         }
         __syncwarp();  // the cells are read before the next round's are written
         if (src >= 0) {
@@ -290,8 +303,10 @@ __device__ bool rotation_leaf(Sh1WarpSmem &sm, uint16_t *cells, LaneUF &uf, int 
 // w + kLeafWarps, ..., on its own, and goes on until its next round begins past the smallest passing seed
 // any of them has found, so every smaller seed has been tried. One leaf then takes a quarter of the time,
 // and with it the launch's tail, in which the last leaves run alone.
+// Eight blocks per SM: 64 registers (72 without the bound: ShockHash<16>, 2M keys 0.53 instead of 0.49 ms; ten
+// blocks, 48 registers: ShockHash<30>, 4M 9.3 instead of 9.1).
 template <int SPL, bool BLOCK, bool PAIRS>
-__global__ void __launch_bounds__(kLeafWarps * 32) k_leaves_sh1(const Node *__restrict__ nodes, const uint32_t *__restrict__ ids,
+__global__ void __launch_bounds__(kLeafWarps * 32, 8) k_leaves_sh1(const Node *__restrict__ nodes, const uint32_t *__restrict__ ids,
                                                                 uint32_t count, const uint64_t *__restrict__ keys,
                                                                 uint64_t *__restrict__ codes, uint64_t *__restrict__ rib_keys,
                                                                 uint8_t *__restrict__ rib_bits, uint64_t max_trials,
@@ -333,14 +348,13 @@ __global__ void __launch_bounds__(kLeafWarps * 32) k_leaves_sh1(const Node *__re
         // ~2^(g+1) trials are expected; 2^(g+10) is only reached by duplicate keys.
         uint64_t cap = 1ull << min(nd.g + 10, 40);
         if (max_trials && max_trials < cap) cap = max_trials;
-        LaneUF uf{sm.uf, lane};
         if (!BLOCK && rot_leaf && m == rot_leaf) {
             // ~2^(g+1) codes x * L + r are expected; the cap counts seeds x
             uint64_t cap_x = (1ull << min(nd.g + 10, 40)) / m + 1;
             if (max_trials && max_trials < cap_x) cap_x = max_trials;
             uint64_t code = 0;
-            const bool ok = m <= 32 ? rotation_leaf<uint32_t>(sm, rot_cells + warp * 64 * 32, uf, lane, m, seed0, cap_x, code)
-                                    : rotation_leaf<uint64_t>(sm, rot_cells + warp * 64 * 32, uf, lane, m, seed0, cap_x, code);
+            const bool ok = m <= 32 ? rotation_leaf<uint32_t>(sm, rot_cells + warp * 64 * 32, lane, m, seed0, cap_x, code)
+                                    : rotation_leaf<uint64_t>(sm, rot_cells + warp * 64 * 32, lane, m, seed0, cap_x, code);
             if (!ok) {
                 if (lane == 0) atomicOr(err, code == ~0ull ? kErrInternal : kErrTrialLimit);
                 continue;
@@ -363,25 +377,16 @@ __global__ void __launch_bounds__(kLeafWarps * 32) k_leaves_sh1(const Node *__re
             continue;
         }
         uint64_t found = ~0ull;
-        // Pseudoforest test of one lane's seed (union-find with a cycle flag per root).
-        auto pseudoforest = [&](uint64_t x) {
-            uf.init(m);
-            bool ok = true;
-            for (uint32_t k = 0; k < m && ok; k++) {
-                uint32_t c1, c2;
-                sh1_cells(sm.keys[k], x, m, c1, c2);
-                ok = uf.add(c1, c2);
-            }
-            return ok;
-        };
-        // queued survivors, tested 32 at a time in queue (= seed) order: the first passing one is
+        // queued survivors, tested four at a time in queue (= seed) order: the first passing one is
         // the smallest passing seed, as every smaller seed failed coverage or an earlier test
         const unsigned below = (1u << lane) - 1;
         uint32_t nq = 0;
         auto drain = [&]() {
-            for (uint32_t q0 = 0; q0 < nq && found == ~0ull; q0 += 32) {
-                const uint64_t off = q0 + lane < nq ? sm.q[q0 + lane] : ~0ull;
-                const bool pass = off != ~0ull && pseudoforest(seed0 + off);
+            for (uint32_t q0 = 0; q0 < nq && found == ~0ull; q0 += 4) {
+                const bool live = q0 + lane / 8 < nq;
+                const uint64_t off = live ? sm.q[q0 + lane / 8] : 0;
+                const bool pass = group_pseudoforest(
+                    m, live, [&](uint32_t k, uint32_t &c1, uint32_t &c2) { sh1_cells(sm.keys[k], seed0 + off, m, c1, c2); });
                 const unsigned bal = __ballot_sync(0xffffffffu, pass);
                 if (bal) found = __shfl_sync(0xffffffffu, off, __ffs(bal) - 1);
             }
@@ -391,7 +396,6 @@ __global__ void __launch_bounds__(kLeafWarps * 32) k_leaves_sh1(const Node *__re
         // the second sieve: the first n <= 32 waiting seeds, one per lane, against the first half's cells (and,
         // where the first sieve was not sure, the second half's). Waiting seeds are within the staged keys'
         // span, but for those of a round hashed in plain form.
-        const uint32_t drain_at = m > 31 ? 2 : kSh1Drain;
         uint32_t nhalf = 0;
         uint64_t base0 = 0;  // the keys are staged for seed0 + base0 and the seeds after it
         auto cover = [&](uint32_t n, bool plain) {
@@ -426,7 +430,7 @@ __global__ void __launch_bounds__(kLeafWarps * 32) k_leaves_sh1(const Node *__re
                 __syncwarp();
             }
             nhalf = rest;
-            if (nq >= drain_at) drain();
+            if (nq) drain();
         };
         // the keys staged for seeds seed0 + at, + at + 1, ...; how many such seeds they are good for
         uint32_t evens = 0;

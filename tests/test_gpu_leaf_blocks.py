@@ -93,3 +93,23 @@ def test_original_seed_pairs_warp_search(engine, kind):
     part = engine.build_shard_hash128(shg.SHOCKHASH, 30, first[inside], second[inside], nb, 0, b1, 2000)
     k = len(part.ribbon_keys)
     assert np.array_equal(part.ribbon_keys, keys[:k]) and np.array_equal(part.ribbon_bits, bits[:k])
+
+
+@pytest.mark.parametrize("leaf,n", [(2, 90), (3, 91), (31, 700), (32, 700), (41, 300), (48, 200)])
+def test_original_pseudoforest_word_sizes(engine, port, leaf, n):
+    # the peeling's words and keys per lane change at 32 and 41 keys
+    rng = np.random.default_rng(leaf)
+    first, second = rng.integers(0, 2**64, size=n, dtype=np.uint64), unique_u64(rng, n)
+    r, p = engine.build_hash128(shg.SHOCKHASH, leaf, first, second, 200), port.build_hash(shg.SHOCKHASH, leaf, first, second, 200)
+    assert np.array_equal(r.descriptors, p.desc)
+    assert np.array_equal(r.ribbon_keys, p.ribbon_keys) and np.array_equal(r.ribbon_bits, p.ribbon_bits)
+
+
+@pytest.mark.parametrize("leaf", [2, 31, 32, 40, 41])
+def test_rotation_pseudoforest_word_sizes(engine, leaf):
+    # the oracle has no rotation fitting: the structure has to be a minimal perfect hash for its host query
+    rng = np.random.default_rng(leaf)
+    n = 40 * leaf + 3
+    first, second = rng.integers(0, 2**64, size=n, dtype=np.uint64), unique_u64(rng, n)
+    r = engine.build_hash128(shg.SHOCKHASH_ROTATION, leaf, first, second, 500, query=True)
+    assert np.array_equal(np.sort(r._mphf.query_hash(first, second)), np.arange(n, dtype=np.uint64))
