@@ -70,6 +70,8 @@ template <int SPL, int THREADS, bool SIMD> struct SplitSmem {
     uint64_t scan[kWarps];
     uint32_t best[2];   // smallest valid seed slot of a round, by the round's parity
     uint32_t stop[2];   // striped search: no smaller seed can come from this block's next rounds
+    uint32_t last;      // striped search: this block is the last of the node's to be done (not `stop`, which a late
+                        // warp may still have to read)
     uint64_t found;     // striped search, in the node's last block: the smallest seed of all its blocks
     uint32_t room;      // smallest seed_room of the staged keys
     SplitKey<SIMD> keys[kMaxBucket];  // last: a launch takes memory for the keys of its largest node only
@@ -373,11 +375,11 @@ __device__ __forceinline__ void split_node(SplitSmem<SPL, THREADS, SIMD> &sm, co
             __threadfence();  // the seed before the count of finished blocks
             const bool last = atomicAdd(&stripe.node->done, 1u) == stripe.count - 1;
             __threadfence();
-            sm.stop[0] = last;
+            sm.last = last;
             if (last) sm.found = ~atomicMax(&stripe.node->inv_best, 0ull);
         }
         __syncthreads();
-        if (!sm.stop[0]) return;
+        if (!sm.last) return;
         trial = sm.found;
     }
     if (trial == ~0ull) {
