@@ -421,6 +421,7 @@ __global__ void __launch_bounds__(kLeafWarps * 32, 8) k_leaves_sh1(const Node *_
             const unsigned bal = __ballot_sync(0xffffffffu, ok);
             if (ok) sm.q[nq + __popc(bal & below)] = off;
             nq += __popc(bal);
+            __syncwarp();  // the queue is written before other lanes read it
             // the rest moves up
             const uint32_t rest = nhalf - n;
             for (uint32_t i = 0; i < rest; i += 32) {

@@ -202,3 +202,9 @@ template <class T, class V> T atomicAdd(T *p, V v) { T o = *p; *p = o + (T)v; re
 template <class T, class V> T atomicMin(T *p, V v) { T o = *p; *p = std::min(o, (T)v); return o; }
 template <class T, class V> T atomicMax(T *p, V v) { T o = *p; *p = std::max(o, (T)v); return o; }
 template <class T, class V> T atomicOr(T *p, V v) { T o = *p; *p = o | (T)v; return o; }
+inline size_t __cvta_generic_to_shared(const void *p) { return (size_t)p; }
+// Static shared memory: one area per kernel instance, so a run of such a kernel has one block.
+#undef __shared__
+#define __shared__ static
+#undef __launch_bounds__
+#define __launch_bounds__(...)
