@@ -473,7 +473,8 @@ __global__ void __launch_bounds__(kLeafWarps * 32, 8) k_leaves_sh1(const Node *_
         constexpr int kIn = PAIRS ? 2 : 1, kLane = SPL * kIn;
         constexpr uint32_t kSeeds = PAIRS ? sh1_pair_seeds(SPL) : 32 * SPL, kStep = kSeeds * (BLOCK ? kLeafWarps : 1);
         for (uint64_t base = BLOCK ? kSeeds * warp : 0; base < cap && found == ~0ull; base += kStep) {
-            if (BLOCK && base > *(volatile unsigned long long *)&block_best) break;
+            // other warps lower block_best meanwhile, so lanes may read different values: the warp leaves as one
+            if (BLOCK && __any_sync(0xffffffffu, base > *(volatile unsigned long long *)&block_best)) break;
             uint32_t mask[kLane], low[kLane];
 #pragma unroll
             for (int i = 0; i < kLane; i++) mask[i] = 0, low[i] = ~0u;

@@ -1245,8 +1245,9 @@ __global__ void __launch_bounds__(kBlockLeafWarps<MAXM> * 32, 24 / kBlockLeafWar
                 __syncwarp();
             };
             for (uint64_t qb = qa; qb < qz && !done; qb += 32) {
-                // a pair that comes before this warp's next one has passed already
-                if (*(volatile unsigned long long *)&sm.best < ((unsigned long long)jb << 32 | ib)) break;
+                // a pair that comes before this warp's next one has passed already (other warps lower `best`
+                // meanwhile, so lanes may read different values: the warp leaves as one)
+                if (__any_sync(0xffffffffu, *(volatile unsigned long long *)&sm.best < ((unsigned long long)jb << 32 | ib))) break;
                 uint32_t j = jb, i = ib + lane;
                 while (i >= j) {
                     i -= j;

@@ -64,6 +64,12 @@ template <int M> void bipartite(const std::vector<Leaf> &leaves, uint64_t order)
               k_leaves_sh2_v2<M, NodeLeaves, 4>(NodeLeaves{nodes, ids, codes}, n, keys, bits, base, slice, smax, cmax, err, work,
                                                 next, kQuadMinRecSplit);
           });
+    check("bipartite, block", leaves, order, 32 * kBlockLeafWarps<M>, sizeof(Sh2BlockSmem<M>),
+          [=](const Node *nodes, const uint32_t *ids, uint32_t n, const uint64_t *keys, uint64_t *codes, uint64_t *, uint8_t *bits,
+              uint32_t *err, unsigned long long *work, unsigned *next) {
+              k_leaves_sh2_block<M, NodeLeaves>(NodeLeaves{nodes, ids, codes}, n, keys, bits, base, slice, smax, cmax, err, work,
+                                                next, kQuadMinRecSplit);
+          });
 }
 
 int main(int, char **argv) {
@@ -90,6 +96,8 @@ int main(int, char **argv) {
                     };
                 };
                 const unsigned th = 32 * kLeafWarps;
+                check("original, block", leaves, order, th, 0, sh1(k_leaves_sh1<1, true, false>));
+                check("original, block, pairs", leaves, order, th, 0, sh1(k_leaves_sh1<2, true, true>));
                 check("original, warp", leaves, order, th, 0, sh1(k_leaves_sh1<2, false, false>));
                 check("original, warp, pairs", leaves, order, th, 0, sh1(k_leaves_sh1<1, false, true>));
             } else {
