@@ -440,7 +440,7 @@ void launch_plan_expand(const uint64_t *acc, uint64_t nb, uint32_t rows, const u
 // the global-atomic kernels were measured faster on B200 (partition of 4M / 10M / 16M keys:
 // 0.33 / 0.92 / 1.80 ms with these kernels, 0.56 / 1.04 / 1.46 ms without).
 static int partition_smem_blocks(uint64_t n, uint64_t nb, size_t &smem) {
-    constexpr uint64_t kMaxSmem = 6144 * sizeof(uint32_t);
+    constexpr uint64_t kMaxSmem = 6144 * sizeof(uint32_t);  // within the 48 KB that a launch may ask for without more ado
     smem = (size_t)nb * sizeof(uint32_t);
     if (nb == 0 || smem > kMaxSmem) return 0;
     int dev = 0, sms = 148;
@@ -456,8 +456,6 @@ void launch_bucket_count(const uint64_t *first, uint64_t n, uint64_t nb, uint64_
     size_t smem = 0;
     const int blocks = partition_smem_blocks(n, nb, smem);
     if (blocks) {
-        // the shared-memory limit is an attribute of the kernel on the current device: set it on every launch
-        cudaFuncSetAttribute(k_bucket_count_smem, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         k_bucket_count_smem<<<blocks, 1024, smem, s>>>(first, n, nb, nb_map, b0, counts, err);
     } else {
         k_bucket_count<<<grid_for(n, 256), 256, 0, s>>>(first, n, nb, nb_map, b0, counts, err);
@@ -508,7 +506,6 @@ void launch_bucket_scatter(const uint64_t *first, uint64_t n, uint64_t nb, uint6
     size_t smem = 0;
     const int blocks = partition_smem_blocks(n, nb, smem);
     if (blocks) {
-        cudaFuncSetAttribute(k_bucket_scatter_smem, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         k_bucket_scatter_smem<<<blocks, 1024, smem, s>>>(first, n, nb, nb_map, b0, cursor, sfirst, sidx, idx_base);
     } else {
         k_bucket_scatter<<<grid_for(n, 256), 256, 0, s>>>(first, n, nb, nb_map, b0, cursor, sfirst, sidx, idx_base);

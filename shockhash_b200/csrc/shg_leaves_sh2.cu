@@ -1560,7 +1560,8 @@ void launch_queue_t(const Node *nodes, const uint32_t *ids, const uint32_t *seq,
                     unsigned int *ctr, uint32_t nleaf_tail, const uint64_t *acc, const uint64_t *singles,
                     const QueueOut *out, uint32_t nreq, uint32_t max_m, int round_div, int grid, cudaStream_t s) {
     const size_t smem = tree_queue_smem_per_block(SPL, max_m);
-    cudaFuncSetAttribute(k_tree_queue<SPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // the limit is shared by all engines' threads: the same value on every launch, room for any node
+    cudaFuncSetAttribute(k_tree_queue<SPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, tree_queue_smem_per_block(SPL, kMaxBucket));
     k_tree_queue<SPL><<<grid, kQueueThreads, smem, s>>>(nodes, ids, seq, nitems, nsplit, offs, stride, nlevels, done, keys,
                                                         codes, rib_bits, scratch, per_warp, smax, cmax, max_trials, err, work,
                                                         kind_work, ctr, nleaf_tail, acc, singles, out, nreq, round_div);

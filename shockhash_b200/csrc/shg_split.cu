@@ -23,9 +23,11 @@ template <int SPL, int THREADS, bool SIMD>
 static void launch_split_t(const Node *nodes, const uint32_t *ids, uint32_t count, uint64_t *keys, uint64_t *codes,
                            uint64_t max_trials, uint32_t *err, unsigned long long *work, unsigned long long *kind_work,
                            uint32_t max_m, int round_div, uint32_t stripes, SplitBest *best, cudaStream_t s) {
+    // A launch takes memory for its largest node. The limit, though, is an attribute of the kernel on the device,
+    // and engines in other threads launch the same kernel: every launch sets the same value, room for any node.
     const size_t smem = split_smem_bytes<SPL, THREADS, SIMD>(max_m);
     auto kernel = stripes > 1 ? k_split<SPL, THREADS, SIMD, true> : k_split<SPL, THREADS, SIMD, false>;
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SplitSmem<SPL, THREADS, SIMD>));
     kernel<<<count * stripes, THREADS, smem, s>>>(nodes, ids, keys, codes, max_trials, err, work, kind_work, round_div, stripes,
                                                   best);
 }
