@@ -473,8 +473,17 @@ shg_status build_batch(shg_engine *e, const shg_params *p, const uint64_t *d_fir
     // a batch's requests go through the partition and the encoding together, from this table
     const bool batch = R > 1;
     const BatchReq *d_req = nullptr;
+    uint64_t part_chunk = 0, part_blocks = 0;  // the partition's shared launch: keys per block, blocks
+    uint64_t alone = 0;                        // requests with launches of their own
     if (batch) {
-        for (size_t r = 0; r < R; r++) hreq[r] = BatchReq{off[r], nr[r], boff[r], nbr[r], nb_map[r], b0[r]};
+        uint64_t shared = 0;
+        for (size_t r = 0; r < R; r++) shared += nr[r] < kBatchAlone ? nr[r] : 0;
+        part_chunk = std::max<uint64_t>(kBatchChunk, shared / kBatchBlocks);
+        for (size_t r = 0; r < R; r++) {
+            hreq[r] = BatchReq{off[r], nr[r], boff[r], nbr[r], nb_map[r], b0[r], part_blocks};
+            if (nr[r] < kBatchAlone) part_blocks += (nr[r] + part_chunk - 1) / part_chunk;
+            else alone++;
+        }
         CU(e->breq.ensure(R * (sizeof(BatchReq) + 8)));
         CU(cudaMemcpyAsync(e->breq.p, hreq, R * sizeof(BatchReq), cudaMemcpyHostToDevice, s));
         d_req = e->breq.as<BatchReq>();
@@ -504,7 +513,11 @@ shg_status build_batch(shg_engine *e, const shg_params *p, const uint64_t *d_fir
     CU(cudaEventRecord(e->ev[0], s));
     if (batch) {
         CU(cudaMemsetAsync(e->counts.p, 0, nb * 4, s));
-        launch_batch_count(d_first, d_req, (uint32_t)R, e->counts.as<uint32_t>(), &misc->err, s);
+        for (size_t r = 0; r < R; r++)
+            if (nr[r] >= kBatchAlone)
+                launch_bucket_count(d_first + off[r], nr[r], nbr[r], nb_map[r], b0[r], e->counts.as<uint32_t>() + boff[r],
+                                    &misc->err, s);
+        launch_batch_count(d_first, d_req, (uint32_t)R, part_chunk, (uint32_t)part_blocks, e->counts.as<uint32_t>(), &misc->err, s);
     } else {
         launch_bucket_count(d_first, n, nb, nb_map[0], b0[0], e->counts.as<uint32_t>(), &misc->err, s);
     }
@@ -528,10 +541,14 @@ shg_status build_batch(shg_engine *e, const shg_params *p, const uint64_t *d_fir
         CU(cudaStreamSynchronize(s));
     }
     const ShapeTables &tab = shp->host;
-    if (batch)
-        launch_batch_scatter(d_first, d_req, (uint32_t)R, e->cursor.as<uint32_t>(), e->sfirst.as<uint64_t>(),
-                             e->sidx.as<uint32_t>(), s);
-    else
+    if (batch) {
+        for (size_t r = 0; r < R; r++)
+            if (nr[r] >= kBatchAlone)
+                launch_bucket_scatter(d_first + off[r], nr[r], nbr[r], nb_map[r], b0[r], e->cursor.as<uint32_t>() + boff[r],
+                                      e->sfirst.as<uint64_t>(), e->sidx.as<uint32_t>(), off[r], s);
+        launch_batch_scatter(d_first, d_req, (uint32_t)R, part_chunk, (uint32_t)part_blocks, e->cursor.as<uint32_t>(),
+                             e->sfirst.as<uint64_t>(), e->sidx.as<uint32_t>(), s);
+    } else
         launch_bucket_scatter(d_first, n, nb, nb_map[0], b0[0], e->cursor.as<uint32_t>(), e->sfirst.as<uint64_t>(),
                               e->sidx.as<uint32_t>(), 0, s);
     launch_bucket_sort(e->acc.as<uint64_t>(), nb, e->sfirst.as<uint64_t>(), e->sidx.as<uint32_t>(), d_second,
@@ -893,10 +910,12 @@ shg_status build_batch(shg_engine *e, const shg_params *p, const uint64_t *d_fir
         out->work[5] = nleaves;
         out->work[6] = nn - nleaves;
         // kernels of this build: hashing (when the keys were hashed on the device), partition
-        // (count, scan, scatter, sort), plan (offset scan and expansion), split levels and leaves,
+        // (scan, sort, counts and scatters), plan (offset scan and expansion), split levels and leaves,
         // Golomb-Rice encoding (3, counted above), retrieval compaction (keys and bits together, or keys
         // before the leaves and bits after them)
-        out->work[7] = (hash_ms > 0.f ? 1 : 0) + 4 + plan_launches + launches + (early_keys ? 1 : 0) + (bits_done ? 0 : 1);
+        const uint64_t partitions = batch ? alone + (part_blocks ? 1 : 0) : 1;
+        out->work[7] = (hash_ms > 0.f ? 1 : 0) + 2 + 2 * partitions + plan_launches + launches + (early_keys ? 1 : 0) +
+                       (bits_done ? 0 : 1);
     }
     return SHG_OK;
 }

@@ -215,15 +215,23 @@ void launch_tree_queue(const Node *nodes, const uint32_t *ids, const uint32_t *s
                        unsigned int *ctr, uint32_t nleaf_tail, const uint64_t *acc, const uint64_t *singles,
                        const QueueOut *out, uint32_t nreq, uint32_t max_m, const SplitTuning &t, int grid, cudaStream_t s);
 // One request of a batched build: its keys are [key_off, key_off + n) of the batch's arrays and its buckets
-// [b_first, b_first + nb), which hold buckets b0, b0 + 1, ... of a structure with nb_map buckets.
+// [b_first, b_first + nb), which hold buckets b0, b0 + 1, ... of a structure with nb_map buckets. The partition's
+// blocks for it begin at blk_first.
+//
+// Requests share the partition's launches, about kBatchBlocks blocks (all resident) in proportion to their keys,
+// but at least kBatchChunk keys a block; those of kBatchAlone keys or more have launches of their own, whose blocks count in
+// shared memory. Partition stage, shared / own launches: 48 requests of 20,000 keys 0.20 / 0.70 ms, 32 of 100,000 0.31 / 0.61,
+// 16 of 250,000 0.40 / 0.45, 8 of 1M 0.75 / 0.57, one of 4M among small ones 0.54 / 0.34, 2 of 10M 1.67 / 1.75. Twice the
+// blocks: 32 of 100,000 0.43, 8 of 1M 0.93. (Sixteen blocks for any request: 8 of 1M 0.82, 4M among small ones 0.84, 2 of 10M 2.83.)
+constexpr uint64_t kBatchBlocks = 4 * 148, kBatchChunk = 1280, kBatchAlone = 500000;
 struct BatchReq {
-    uint64_t key_off, n, b_first, nb, nb_map, b0;
+    uint64_t key_off, n, b_first, nb, nb_map, b0, blk_first;
 };
-// Bucket counts (zeroed by the caller) and scatter of all requests' keys, nreq requests in one launch.
-void launch_batch_count(const uint64_t *first, const BatchReq *req, uint32_t nreq, uint32_t *counts, uint32_t *err,
-                        cudaStream_t s);
-void launch_batch_scatter(const uint64_t *first, const BatchReq *req, uint32_t nreq, uint32_t *cursor, uint64_t *sfirst,
-                          uint32_t *sidx, cudaStream_t s);
+// Bucket counts (zeroed by the caller) and scatter of all requests' keys in one launch of `blocks` blocks.
+void launch_batch_count(const uint64_t *first, const BatchReq *req, uint32_t nreq, uint64_t chunk, uint32_t blocks, uint32_t *counts,
+                        uint32_t *err, cudaStream_t s);
+void launch_batch_scatter(const uint64_t *first, const BatchReq *req, uint32_t nreq, uint64_t chunk, uint32_t blocks, uint32_t *cursor,
+                          uint64_t *sfirst, uint32_t *sidx, cudaStream_t s);
 // Each request's bucket lengths scanned into pos + b_first + r: nb + 1 positions per request r.
 void launch_batch_scan_u64(const uint64_t *in, const BatchReq *req, uint32_t nreq, uint64_t *pos, cudaStream_t s);
 void launch_gr_bucket_bits(const Node *nodes, const uint32_t *bnb, uint64_t nb, const uint64_t *acc,

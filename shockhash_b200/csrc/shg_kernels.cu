@@ -461,24 +461,34 @@ void launch_bucket_count(const uint64_t *first, uint64_t n, uint64_t nb, uint64_
         k_bucket_count<<<grid_for(n, 256), 256, 0, s>>>(first, n, nb, nb_map, b0, counts, err);
     }
 }
-// The partition's counts and scatter for a batch of key sets: kBatchBlocks blocks per request, in one launch
-// (a launch per request of 20,000 keys took about 5 and 7 us each, and its host time).
-constexpr uint32_t kBatchBlocks = 16;
-__global__ void k_batch_count(const uint64_t *__restrict__ first, const BatchReq *__restrict__ req,
-                              uint32_t *__restrict__ counts, uint32_t *__restrict__ err) {
-    const BatchReq q = req[blockIdx.x / kBatchBlocks];
-    for (uint64_t i = (blockIdx.x % kBatchBlocks) * (uint64_t)blockDim.x + threadIdx.x; i < q.n;
-         i += kBatchBlocks * (uint64_t)blockDim.x) {
+// The partition's counts and scatter for a batch of key sets in one launch (a launch per request of 20,000 keys
+// took about 5 and 7 us each, and its host time): a block per `chunk` keys of a request, the request found from the
+// requests' first blocks.
+__device__ __forceinline__ uint32_t batch_request(const BatchReq *__restrict__ req, uint32_t nreq) {
+    uint32_t r = 0;
+    for (uint32_t hi = nreq; hi - r > 1;) {
+        const uint32_t mid = (r + hi) >> 1;
+        if (req[mid].blk_first <= blockIdx.x) r = mid; else hi = mid;
+    }
+    return r;
+}
+__global__ void __launch_bounds__(512) k_batch_count(const uint64_t *__restrict__ first, const BatchReq *__restrict__ req,
+                                                     uint32_t nreq, uint64_t chunk, uint32_t *__restrict__ counts,
+                                                     uint32_t *__restrict__ err) {
+    const BatchReq q = req[batch_request(req, nreq)];
+    const uint64_t lo = (blockIdx.x - q.blk_first) * chunk, hi = min(q.n, lo + chunk);
+    for (uint64_t i = lo + threadIdx.x; i < hi; i += blockDim.x) {
         const uint64_t b = remap128(first[q.key_off + i], q.nb_map) - q.b0;
         if (b >= q.nb) atomicOr(err, kErrArg);
         else atomicAdd(&counts[q.b_first + b], 1u);
     }
 }
-__global__ void k_batch_scatter(const uint64_t *__restrict__ first, const BatchReq *__restrict__ req,
-                                uint32_t *__restrict__ cursor, uint64_t *__restrict__ sfirst, uint32_t *__restrict__ sidx) {
-    const BatchReq q = req[blockIdx.x / kBatchBlocks];
-    for (uint64_t i = (blockIdx.x % kBatchBlocks) * (uint64_t)blockDim.x + threadIdx.x; i < q.n;
-         i += kBatchBlocks * (uint64_t)blockDim.x) {
+__global__ void __launch_bounds__(512) k_batch_scatter(const uint64_t *__restrict__ first, const BatchReq *__restrict__ req,
+                                                       uint32_t nreq, uint64_t chunk, uint32_t *__restrict__ cursor,
+                                                       uint64_t *__restrict__ sfirst, uint32_t *__restrict__ sidx) {
+    const BatchReq q = req[batch_request(req, nreq)];
+    const uint64_t lo = (blockIdx.x - q.blk_first) * chunk, hi = min(q.n, lo + chunk);
+    for (uint64_t i = lo + threadIdx.x; i < hi; i += blockDim.x) {
         const uint64_t f = first[q.key_off + i];
         const uint64_t b = remap128(f, q.nb_map) - q.b0;
         if (b >= q.nb) continue;  // reported by k_batch_count
@@ -487,13 +497,13 @@ __global__ void k_batch_scatter(const uint64_t *__restrict__ first, const BatchR
         sidx[pos] = (uint32_t)(q.key_off + i);
     }
 }
-void launch_batch_count(const uint64_t *first, const BatchReq *req, uint32_t nreq, uint32_t *counts, uint32_t *err,
-                        cudaStream_t s) {
-    k_batch_count<<<nreq * kBatchBlocks, 512, 0, s>>>(first, req, counts, err);
+void launch_batch_count(const uint64_t *first, const BatchReq *req, uint32_t nreq, uint64_t chunk, uint32_t blocks, uint32_t *counts,
+                        uint32_t *err, cudaStream_t s) {
+    if (blocks) k_batch_count<<<blocks, 512, 0, s>>>(first, req, nreq, chunk, counts, err);
 }
-void launch_batch_scatter(const uint64_t *first, const BatchReq *req, uint32_t nreq, uint32_t *cursor, uint64_t *sfirst,
-                          uint32_t *sidx, cudaStream_t s) {
-    k_batch_scatter<<<nreq * kBatchBlocks, 512, 0, s>>>(first, req, cursor, sfirst, sidx);
+void launch_batch_scatter(const uint64_t *first, const BatchReq *req, uint32_t nreq, uint64_t chunk, uint32_t blocks, uint32_t *cursor,
+                          uint64_t *sfirst, uint32_t *sidx, cudaStream_t s) {
+    if (blocks) k_batch_scatter<<<blocks, 512, 0, s>>>(first, req, nreq, chunk, cursor, sfirst, sidx);
 }
 void launch_scan_counts(const uint32_t *counts, uint64_t nb, uint64_t *acc, uint32_t *cursor, uint32_t *maxsz,
                         cudaStream_t s) {
