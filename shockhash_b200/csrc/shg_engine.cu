@@ -255,11 +255,13 @@ template <class F> void run_parts(unsigned nt, F &fn) {
     for (auto &th : pool) th.join();
 }
 
-bool is_pinned(const void *p) {
+// Whether p is plain host memory, which a copy has to stage: not pinned, managed or device memory, which the copy
+// engine reads (or refuses) by itself and the host may be unable to.
+bool is_pageable(const void *p) {
     cudaPointerAttributes attr{};
-    const bool pinned = cudaPointerGetAttributes(&attr, p) == cudaSuccess && attr.type == cudaMemoryTypeHost;
+    const bool pageable = cudaPointerGetAttributes(&attr, p) != cudaSuccess || attr.type == cudaMemoryTypeUnregistered;
     cudaGetLastError();  // a pageable pointer may leave an error behind on some drivers
-    return pinned;
+    return pageable;
 }
 
 // Host-to-device copies from pageable memory. A copy straight from there runs at about 11 GB/s (the driver
@@ -278,7 +280,7 @@ shg_status h2d_segments(shg_engine *e, void *dst, const HostSeg *segs, const siz
     const size_t bytes = start[nseg];
     if (!bytes) return SHG_OK;
     bool stage = nseg > 1 ? bytes >= (64u << 10) : bytes >= kStageMin;
-    for (size_t i = 0; i < nseg && stage; i++) stage = !segs[i].bytes || !is_pinned(segs[i].src);
+    for (size_t i = 0; i < nseg && stage; i++) stage = !segs[i].bytes || is_pageable(segs[i].src);
     if (stage && !e->stage && cudaHostAlloc(&e->stage, kStageThreads * 2 * kStagePiece, cudaHostAllocDefault) != cudaSuccess) {
         e->stage = nullptr;  // no pinned memory to spare: copy directly
         cudaGetLastError();
