@@ -47,6 +47,8 @@ using namespace shg;
 static thread_local std::string g_last_error;
 
 static shg_status fail(shg_status st, const std::string &msg) {
+    // the failed call's error is reported by this one: the next call's checks must not find it again
+    if (st == SHG_ERR_CUDA || st == SHG_ERR_OOM) cudaGetLastError();
     g_last_error = msg;
     return st;
 }
