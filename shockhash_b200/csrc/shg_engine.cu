@@ -435,9 +435,8 @@ struct ShardSpec {
     uint64_t nb_global, b0, b1;
 };
 
-shg_status build_batch(shg_engine *e, const shg_params *p, const uint64_t *d_first, const uint64_t *d_second,
-                       const std::vector<uint64_t> &nr, shg_result *outs, float hash_ms,
-                       const ShardSpec *shards = nullptr) {
+shg_status queue_batch(shg_engine *e, const shg_params *p, const uint64_t *d_first, const uint64_t *d_second,
+                       const std::vector<uint64_t> &nr, shg_result *outs, float hash_ms, const ShardSpec *shards) {
     const Config &cfg = config_of(p->variant, p->leaf_size);
     cudaStream_t s = e->stream;
     const size_t R = nr.size();
@@ -924,6 +923,21 @@ shg_status build_batch(shg_engine *e, const shg_params *p, const uint64_t *d_fir
     return SHG_OK;
 }
 
+// A failed build returns only when the copies it has queued are done: those from the caller's memory, and those from
+// and to the engine's pinned host buffers, which the next build fills or gives back.
+shg_status settle(shg_engine *e, shg_status st) {
+    if (st != SHG_OK) {
+        cudaStreamSynchronize(e->stream);
+        cudaStreamSynchronize(e->stream2);
+    }
+    return st;
+}
+
+shg_status build_batch(shg_engine *e, const shg_params *p, const uint64_t *d_first, const uint64_t *d_second,
+                       const std::vector<uint64_t> &nr, shg_result *outs, float hash_ms, const ShardSpec *shards = nullptr) {
+    return settle(e, queue_batch(e, p, d_first, d_second, nr, outs, hash_ms, shards));
+}
+
 shg_status build_core(shg_engine *e, const shg_params *p, const uint64_t *d_first, const uint64_t *d_second, uint64_t n,
                       shg_result *out, float hash_ms) {
     return build_batch(e, p, d_first, d_second, std::vector<uint64_t>{n}, out, hash_ms);
@@ -1395,12 +1409,6 @@ void shg_engine_destroy(shg_engine *e) {
     delete e;
 }
 
-// A failed build returns only when the copies from the caller's memory that it has queued are done.
-static shg_status settle(shg_engine *e, shg_status st) {
-    if (st != SHG_OK) cudaStreamSynchronize(e->stream);
-    return st;
-}
-
 static shg_status timed_hash_u64(shg_engine *e, const uint64_t *d_keys, uint64_t n, float &ms) {
     CU(e->first.ensure(std::max<uint64_t>(n, 1) * 8));
     CU(e->second.ensure(std::max<uint64_t>(n, 1) * 8));
@@ -1711,7 +1719,7 @@ shg_status shg_build_u64_device(shg_engine *e, const shg_params *p, const uint64
     float ms = 0;
     st = timed_hash_u64(e, d_keys, n, ms);
     if (st) return settle(e, st);
-    return settle(e, build_core(e, p, e->first.as<uint64_t>(), e->second.as<uint64_t>(), n, out, ms));
+    return build_core(e, p, e->first.as<uint64_t>(), e->second.as<uint64_t>(), n, out, ms);
 }
 
 shg_status shg_build_u64(shg_engine *e, const shg_params *p, const uint64_t *keys, uint64_t n, shg_result *out) {
@@ -1724,7 +1732,7 @@ shg_status shg_build_u64(shg_engine *e, const shg_params *p, const uint64_t *key
     float ms = 0;
     st = timed_hash_u64(e, e->in_keys.as<uint64_t>(), n, ms);
     if (st) return settle(e, st);
-    return settle(e, build_core(e, p, e->first.as<uint64_t>(), e->second.as<uint64_t>(), n, out, ms));
+    return build_core(e, p, e->first.as<uint64_t>(), e->second.as<uint64_t>(), n, out, ms);
 }
 
 shg_status shg_build_batch_u64(shg_engine *e, const shg_params *p, const uint64_t *const *keys, const uint64_t *n,
@@ -1753,8 +1761,7 @@ shg_status shg_build_batch_u64(shg_engine *e, const shg_params *p, const uint64_
     float ms = 0;
     st = timed_hash_u64(e, e->in_keys.as<uint64_t>(), total, ms);
     if (st) return settle(e, st);
-    return settle(e, build_batch(e, p, e->first.as<uint64_t>(), e->second.as<uint64_t>(), std::vector<uint64_t>(n, n + nreq), outs,
-                                 ms));
+    return build_batch(e, p, e->first.as<uint64_t>(), e->second.as<uint64_t>(), std::vector<uint64_t>(n, n + nreq), outs, ms);
 }
 
 static shg_status hash_strings_dev(shg_engine *e, const char *bytes, const uint64_t *offsets, uint64_t n, float &ms) {
@@ -1790,7 +1797,7 @@ shg_status shg_build_strings(shg_engine *e, const shg_params *p, const char *byt
     float ms = 0;
     st = hash_strings_dev(e, bytes, offsets, n, ms);
     if (st) return settle(e, st);
-    return settle(e, build_core(e, p, e->first.as<uint64_t>(), e->second.as<uint64_t>(), n, out, ms));
+    return build_core(e, p, e->first.as<uint64_t>(), e->second.as<uint64_t>(), n, out, ms);
 }
 
 shg_status shg_hash_strings(shg_engine *e, const char *bytes, const uint64_t *offsets, uint64_t n, uint64_t *first,

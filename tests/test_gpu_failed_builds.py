@@ -39,3 +39,17 @@ def test_engine_goes_on_after_failed_builds():
     for k, w in zip(sets, want):
         assert products(eng.build_u64(shg.SHOCKHASH2, 24, k, 100)) == w
     eng.close()
+
+
+@pytest.mark.parametrize("mode", [shg.MODE_LEVELS, shg.MODE_QUEUE, shg.MODE_PIPELINED])
+def test_larger_build_follows_a_failed_one(mode):
+    # the engine's pinned buffers grow (and are given back) right after builds that stopped half way
+    eng, other = shg.Engine(0), shg.Engine(0)
+    for i, n in enumerate((500, 20_000, 200_000)):
+        first, second = (shg.keys_mt19937_64(80 + 2 * i + j, n) for j in (0, 1))
+        with pytest.raises(shg.ShgError):
+            eng.build_hash128(shg.SHOCKHASH2, 24, first, second, 100, mode=mode, max_trials=1)
+        keys = shg.keys_mt19937_64(90 + i, 4 * n)
+        assert products(eng.build_u64(shg.SHOCKHASH2, 24, keys, 100, mode=mode)) == products(other.build_u64(shg.SHOCKHASH2, 24, keys, 100))
+    eng.close()
+    other.close()
