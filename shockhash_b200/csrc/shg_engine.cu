@@ -690,19 +690,24 @@ shg_status queue_batch(shg_engine *e, const shg_params *p, const uint64_t *d_fir
     // a few thousand still ends with its longest searches alone (trial counts are geometric). Split
     // levels, one block per node / striped: 1,000 keys 0.61 / 0.10 ms, 30,000 keys 1.47 / 0.40, 300,000 keys
     // 2.76 / 1.80, 1M keys 5.07 / 4.70; with four grids 1M takes 5.17, with 32 grids 3M 12.3 instead of 11.3.
-    auto stripes_of = [&](uint64_t count) -> uint32_t {
-        const uint64_t want = 12ull * 5 * e->sms;
-        return (uint32_t)std::min<uint64_t>(32, std::max<uint64_t>(1, want / std::max<uint64_t>(count, 1)));
+    // And no more than two of the smallest rounds per block for the level's longest search: blocks
+    // that find nothing to do still cost the launch.
+    auto stripes_of = [&](size_t lv, uint64_t count) -> uint32_t {
+        const uint64_t want = 12ull * 5 * e->sms, rounds = (uint64_t)(tab.level_trials[lv] / (2 * 32 * tun.split.spl));
+        return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>({32, want / std::max<uint64_t>(count, 1), rounds}));
     };
     if (!queue && leaf_off) {
-        CU(e->split_best.ensure(leaf_off * sizeof(SplitBest)));
-        CU(cudaMemsetAsync(e->split_best.p, 0, leaf_off * sizeof(SplitBest), s));
+        uint64_t striped = 0;  // nodes of the levels down to the last striped one
+        for (int lv = 0; lv < nlevels; lv++)
+            if (level_count[lv] && (pipelined || stripes_of(lv, level_count[lv]) > 1)) striped = level_off[lv] + level_count[lv];
+        CU(e->split_best.ensure(std::max<uint64_t>(striped, 1) * sizeof(SplitBest)));
+        if (striped) CU(cudaMemsetAsync(e->split_best.p, 0, striped * sizeof(SplitBest), s));
     }
     auto split_range = [&](size_t lv, uint64_t a, uint64_t b, cudaStream_t st) {
         if (b <= a) return;
         launch_split_level(e->nodes.as<Node>(), d_ids + level_off[lv] + a, (uint32_t)(b - a), e->keys.as<uint64_t>(),
                            e->codes.as<uint64_t>(), p->max_trials, &misc->err, &misc->work[0], misc->split_kind,
-                           std::min<uint32_t>(maxsz, tab.level_max[lv]), tun.split, stripes_of(b - a),
+                           std::min<uint32_t>(maxsz, tab.level_max[lv]), tun.split, stripes_of(lv, b - a),
                            e->split_best.as<SplitBest>() + level_off[lv] + a, st);
         launches++;
     };

@@ -96,7 +96,8 @@ struct ShapeTables {
     std::vector<uint32_t> node_off;  // [rows + 1]
     std::vector<uint16_t> singles;
     std::vector<uint32_t> single_off;  // [rows + 1]
-    uint16_t level_max[kMaxLevels] = {};  // keys of the largest split node of each level
+    uint16_t level_max[kMaxLevels] = {};    // keys of the largest split node of each level
+    double level_trials[kMaxLevels] = {};  // largest number of seeds that a split node of the level is expected to take
 };
 void make_shape_tables(const Config &c, uint32_t rows, ShapeTables &t);
 

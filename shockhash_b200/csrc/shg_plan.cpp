@@ -140,6 +140,18 @@ const Shape &shape_of(const Config &c, uint32_t m, std::vector<Shape> &cache, st
     return cache[m];
 }
 
+// Seeds that a split node is expected to take: 1 / p, p the probability that a multinomial split of its keys has
+// exactly the parts' sizes (by Stirling's formula; the split kernel sizes its rounds by the same number).
+static double split_trials(const TNode &t) {
+    double sp = 1;
+    if (t.kind == kSplit2) sp = std::sqrt((double)t.unit) * std::sqrt((double)(t.m - t.unit));
+    else {
+        for (int i = 1; i < t.fanout; i++) sp *= std::sqrt((double)t.unit);
+        sp *= std::sqrt((double)(t.m - (t.fanout - 1) * t.unit));
+    }
+    return std::pow(2 * M_PI, (t.fanout - 1) / 2.0) * sp / std::sqrt((double)t.m);
+}
+
 void make_shape_tables(const Config &c, uint32_t rows, ShapeTables &t) {
     if (rows > (uint32_t)kMaxBucket) throw std::runtime_error("bucket size beyond MAX_BUCKET_SIZE");
     // shapes depend only on the configuration and the bucket size: reuse them across builds
@@ -153,6 +165,8 @@ void make_shape_tables(const Config &c, uint32_t rows, ShapeTables &t) {
     t.nodes.clear();
     t.singles.clear();
     std::fill(t.level_max, t.level_max + kMaxLevels, (uint16_t)0);
+    std::fill(t.level_trials, t.level_trials + kMaxLevels, 0.0);
+    std::vector<double> trials(rows, 0.0);  // of a split node, which its number of keys alone determines
     t.node_off.assign(rows + 1, 0);
     t.single_off.assign(rows + 1, 0);
     for (uint32_t m = 0; m < rows; m++) {
@@ -171,7 +185,11 @@ void make_shape_tables(const Config &c, uint32_t rows, ShapeTables &t) {
             n.unit = tn.unit;
             n.fixed_off = tn.fixed_off;
             n.seed = tn.seed;
-            if (tn.kind != kLeaf) t.level_max[tn.level] = std::max(t.level_max[tn.level], tn.m);
+            if (tn.kind != kLeaf) {
+                if (trials[tn.m] == 0.0) trials[tn.m] = split_trials(tn);
+                t.level_max[tn.level] = std::max(t.level_max[tn.level], tn.m);
+                t.level_trials[tn.level] = std::max(t.level_trials[tn.level], trials[tn.m]);
+            }
             const int col = tn.kind == kLeaf ? kColLeaves : kColLevel0 + tn.level;
             n.rank = (uint16_t)row[col]++;
             t.nodes.push_back(n);

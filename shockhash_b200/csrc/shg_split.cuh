@@ -306,18 +306,21 @@ __device__ __forceinline__ void split_node(SplitSmem<SPL, THREADS, SIMD> &sm, co
     constexpr int kWarps = THREADS / 32, kSeedsPerWarp = 32 * SPL;
     const uint32_t m = nd.m;
     const uint64_t seed0 = start_seed(nd.level);
-    if (threadIdx.x == 0) {
-        sm.best[0] = sm.best[1] = 0xffffffffu;
-        sm.room = kSeedSpan;
-    }
-    __syncthreads();
-    uint32_t room = kSeedSpan;
-    for (uint32_t i = threadIdx.x; i < m; i += THREADS) {
-        const uint64_t z = (L2 ? __ldcg(&keys[nd.start + i]) : keys[nd.start + i]) + seed0;
-        sm.keys[i] = SplitKey<SIMD>::make(z);
-        room = min(room, seed_room(z));
-    }
-    merge_room(sm, room);
+    auto stage = [&]() {
+        if (threadIdx.x == 0) {
+            sm.best[0] = sm.best[1] = 0xffffffffu;
+            sm.room = kSeedSpan;
+        }
+        __syncthreads();
+        uint32_t room = kSeedSpan;
+        for (uint32_t i = threadIdx.x; i < m; i += THREADS) {
+            const uint64_t z = (L2 ? __ldcg(&keys[nd.start + i]) : keys[nd.start + i]) + seed0;
+            sm.keys[i] = SplitKey<SIMD>::make(z);
+            room = min(room, seed_room(z));
+        }
+        merge_room(sm, room);
+    };
+    if constexpr (!STRIPED) stage();  // a stripe first finds out whether it takes part
 
     // Part boundaries as thresholds on the low 16 bits of remix (see header).
     uint32_t T[3] = {65536u, 65536u, 65536u}, need[3] = {m, m, m};
@@ -349,6 +352,7 @@ __device__ __forceinline__ void split_node(SplitSmem<SPL, THREADS, SIMD> &sm, co
         if (stripe.index >= stripe.count) return;
         expect /= stripe.count;
     }
+    if constexpr (STRIPED) stage();
     int G = 1;
     while (G < kWarps && (double)(kSeedsPerWarp * G * 2) * (double)round_div <= expect) G <<= 1;
     __syncthreads();
