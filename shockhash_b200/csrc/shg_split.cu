@@ -43,6 +43,14 @@ void launch_split_level(const Node *nodes, const uint32_t *ids, uint32_t count, 
                         uint32_t max_m, const SplitTuning &t, uint32_t stripes, SplitBest *best, cudaStream_t s) {
     if (!count) return;
     const bool simd = t.arith == kSplitArithSimd;
+    // Nodes of at most 128 keys: half the threads (unless the table asks for another number), at least one for each
+    // key. Their blocks spend their time on the prologue, two or three rounds and the partition, so what counts is how many
+    // nodes an SM holds. Splits stage, 256 / 128 threads: ShockHash<2>, b = 200, 1M keys 3.24 / 1.95 ms, ShockHash<8>, b = 1000, 1M 1.21 / 0.88,
+    // ShockHash<16>, b = 400, 1M 0.66 / 0.56, ShockHash2<64>, 4M 14.3 / 14.2. Up to 256 keys: ShockHash2<64>, 1M 4.85 instead of
+    // 4.67; up to 512: ShockHash2<16>, 30,000 keys 0.18 instead of 0.15.
+    if (t.threads == SplitTuning().threads && max_m <= 128)
+        return launch_split_level(nodes, ids, count, keys, codes, max_trials, err, work, kind_work, max_m,
+                                  SplitTuning{t.spl, 128, t.round_div, t.arith}, stripes, best, s);
 #define SHG_SPLIT_CASE(SPL, TH)                                                                                      \
     if (t.spl == SPL && t.threads == TH)                                                                            \
         return simd ? launch_split_t<SPL, TH, true>(nodes, ids, count, keys, codes, max_trials, err, work, kind_work, \

@@ -1,5 +1,5 @@
-"""Trees of small nodes: split levels whose searches expect too few seeds for several blocks per node (level by level,
-around the sizes where that changes), against the oracle."""
+"""Trees of small nodes: split levels whose searches expect too few seeds for several blocks per node, and levels of up to
+128 keys per node, which take blocks of half the threads (around the sizes where that changes), against the oracle."""
 import numpy as np
 import pytest
 
