@@ -54,7 +54,8 @@ typedef enum shg_variant {
 /* How the search stages are scheduled on the device. All modes give identical results. */
 typedef enum shg_mode {
     SHG_MODE_DEFAULT = 0,     /* the fastest measured schedule for the build's size: SHG_MODE_LEVELS, or
-                                 SHG_MODE_QUEUE for ShockHash2 builds of 0.6 to 2.5 million keys */
+                                 SHG_MODE_QUEUE for ShockHash2 builds of 0.6 to 2.5 million keys with leaves of 25 to
+                                 64 keys (fewer keys for small leaves) in buckets of eight leaves or more */
     SHG_MODE_LEVELS = 1,      /* one launch per RecSplit level (a block per split node, several while the level
                                  has few nodes), then one persistent leaf launch whose warps drain all leaves from a device counter */
     SHG_MODE_PER_LEAF = 2,    /* comparison form: per-level split launches and one launch per leaf */

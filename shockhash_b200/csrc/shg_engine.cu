@@ -619,12 +619,22 @@ shg_status queue_batch(shg_engine *e, const shg_params *p, const uint64_t *d_fir
     // practice) takes a new block after encoding.
     // The work-queue schedule: bipartite leaves of up to 64 keys (other builds take the level schedule). By
     // default only in the middle of the range, where it hides the ends of the level launches without
-    // filling the chip many times: level / queue, 1,000 keys 0.55 / 1.39 ms, 300,000 keys 2.7 / 3.1, 1M
-    // keys 6.1 / 5.8, 10M keys 43.5 / 45.7, 20M keys 86.8 / 92. Its blocks hold the leaf search's shared
-    // memory and registers, 24 warps per SM, during the splits too, and the two codes share the
-    // instruction cache.
+    // filling the chip many times, and only in trees whose searches are long enough for that. Its blocks hold the
+    // leaf search's shared memory and registers, 24 warps per SM, during the splits too, and the two codes share the
+    // instruction cache. Levels / queue, b = 2000, ms:
+    //   leaf      300,000 keys    600,000       1M          1.6M          2.5M          4M
+    //   8         0.72 / 1.11   1.11 / 1.75   1.60 / 2.60   2.41 / 3.87   3.52 / 5.84   5.43 / 9.12
+    //   24        1.18 / 1.30   1.82 / 1.80   2.65 / 2.71   3.84 / 4.28   5.66 / 6.75   8.72 / 10.9
+    //   33        1.38 / 1.36   2.18 / 2.03   3.11 / 2.90   4.52 / 4.42   6.62 / 6.77   9.96 / 10.6
+    //   48        1.60 / 1.65   2.65 / 2.50   3.90 / 3.78   5.63 / 5.43   8.38 / 8.29   12.9 / 13.0
+    //   64        2.40 / 2.79   3.95 / 3.73   6.07 / 5.71   8.48 / 8.14   12.5 / 12.1   18.3 / 18.6
+    // and for 1M keys in buckets of 400 / 100 keys: leaf 33 2.84 / 2.59 and 1.85 / 2.32, leaf 48 3.08 / 3.07 and 1.23 / 2.51,
+    // leaf 64 3.87 / 4.25 and 1.59 / 4.61 (few split levels to hide, and most of the work in the leaves).
+    const uint64_t leaf_keys = (uint64_t)p->leaf_size;
+    const bool by_size = leaf_keys > 24 && p->bucket_size >= 8 * leaf_keys && n >= 600000 &&
+                         n < std::min<uint64_t>(2500000, 50000 * leaf_keys);
     const bool queue = p->variant == SHG_SHOCKHASH2 && p->leaf_size <= 64 &&
-                       (p->mode == SHG_MODE_QUEUE || (p->mode == SHG_MODE_DEFAULT && n >= 600000 && n < 2500000));
+                       (p->mode == SHG_MODE_QUEUE || (p->mode == SHG_MODE_DEFAULT && by_size));
     const Tuning tun = e->tuning_of(p->variant, p->leaf_size);
     // with per-bucket leaf groups, the queue kernel writes each bucket's retrieval keys and bits
     // straight into the pinned result block as the bucket's leaves finish
