@@ -402,7 +402,8 @@ shg_status shg_engine_last_work(const shg_engine *e, uint64_t *out, int n);
 /* Launch parameters of the search kernels per configuration (no counterpart in the reference; they
  * change speed only, never a result). variant is an shg_variant (SHG_SHOCKHASH_ROTATION shares
  * SHG_SHOCKHASH's entry) or 4 for ShockHash2Flat<k> with leaf_size = k. Names and ranges:
- *   split_seeds_per_lane 1, 2, 4; split_threads 128, 256, 512; split_round_div 1..64 (a round of
+ *   split_seeds_per_lane 1, 2, 4; split_threads 128, 256, 512 (256, the default: 128 for levels whose
+ *   nodes have at most 128 keys); split_round_div 1..64 (a round of
  *   seeds aims at 1/round_div of a split node's expected trials); split_arith 0, 1 (the same
  *   arithmetic; kept for tables that set it);
  *   leaf_blocks_per_sm 0..16 (0 =

@@ -72,6 +72,50 @@ template <int M> void bipartite(const std::vector<Leaf> &leaves, uint64_t order)
           });
 }
 
+// Candidate capacities at which a leaf's round no longer fits: both forms list the same prefix of the candidates, so they
+// find the seed, or report that the capacity is exceeded, at the same capacities.
+template <int M> void capacities(const Leaf &leaf, uint64_t order) {
+    int found = 0, full = 0;
+    for (uint32_t cmax = 2; cmax <= 512; cmax += cmax < 32 ? 2 : 32) {
+        const uint32_t smax = 4096;
+        Sh2Global<M> g;
+        g.carve(nullptr, smax, cmax);
+        const size_t slice = ((size_t)(g.raw + (uint64_t)g.rawcap * (M / 8)) + 255) & ~(size_t)255;
+        std::vector<uint64_t> scratch(4 * slice / 8 + 2);
+        uint8_t *const base = (uint8_t *)(((uintptr_t)scratch.data() + 15) & ~(uintptr_t)15);
+        Node nd{};
+        nd.m = (uint16_t)leaf.keys.size();
+        const uint32_t id = 0;
+        uint64_t code[2] = {~0ull, ~0ull};
+        uint32_t err[2] = {};
+        const char *e[2];
+        for (int form = 0; form < 2; form++) {
+            std::vector<uint8_t> bits(leaf.keys.size());
+            unsigned long long work[8] = {};
+            unsigned next = 0;
+            const NodeLeaves src{&nd, &id, &code[form]};
+            if (form == 0)
+                e[0] = emu::run(1, 32, 4 * sizeof(Sh2Smem<M>), order, [&]() {
+                    k_leaves_sh2_v2<M, NodeLeaves, 4>(src, 1, leaf.keys.data(), bits.data(), base, slice, smax, cmax, &err[0], work,
+                                                      &next, kQuadMinRecSplit);
+                });
+            else
+                e[1] = emu::run(1, 32 * kBlockLeafWarps<M>, sizeof(Sh2BlockSmem<M>), order, [&]() {
+                    k_leaves_sh2_block<M, NodeLeaves>(src, 1, leaf.keys.data(), bits.data(), base, slice, smax, cmax, &err[1], work,
+                                                      &next, kQuadMinRecSplit);
+                });
+        }
+        const bool ok = code[0] == leaf.seed ? err[0] == 0 : code[0] == ~0ull && err[0] == kErrScratch;
+        if (e[0] || e[1] || !ok || code[0] != code[1] || err[0] != err[1]) {
+            bad++;
+            printf("capacity %u, %zu keys: %s %s, err %u %u, seed %" PRIu64 " %" PRIu64 " want %" PRIu64 "\n", cmax, leaf.keys.size(),
+                   e[0] ? e[0] : "", e[1] ? e[1] : "", err[0], err[1], code[0], code[1], leaf.seed);
+        }
+        (code[1] == leaf.seed ? found : full)++;
+    }
+    if (!found || !full) bad++, printf("capacities of %zu keys: found %d, exceeded %d\n", leaf.keys.size(), found, full);
+}
+
 int main(int, char **argv) {
     FILE *f = fopen(argv[1], "r");
     int kind = 0;
@@ -101,6 +145,7 @@ int main(int, char **argv) {
                 check("original, warp", leaves, order, th, 0, sh1(k_leaves_sh1<2, false, false>));
                 check("original, warp, pairs", leaves, order, th, 0, sh1(k_leaves_sh1<1, false, true>));
             } else {
+                if (leaves.size() == 1 && leaves[0].keys.size() == 64 && order == 10 * set) capacities<64>(leaves[0], order);
                 if (leaves[0].keys.size() <= 64) bipartite<64>(leaves, order);
                 else bipartite<128>(leaves, order);
             }
