@@ -49,12 +49,12 @@ CONFIG_NAME = "ShockHash2<64> b=2000, 10M uint64 keys (mt19937_64 seed 7) hashed
 MODES = ["default (by size: levels or queue)", "levels", "per_leaf",
          "pipelined", "queue"]
 # DRAM bytes (read + write) per key of one launch, from one ncu capture of the 1M-key case
-# (profiles/k_tree_queue_sh2_l64.md, profiles/k_split_sh2_l64.md) scaled by keys: the work-queue
+# (profiles/kernels_staged_seeds.md) scaled by keys: the work-queue
 # kernel (the whole search: node keys read, retrieval bits and spilled leaf scratch written) and a
 # quarter-split level launch of the level schedule (node keys read once; the partition's writes
 # stay in L2).
-QUEUE_DRAM_BYTES_PER_KEY = (13_114_880 + 81_113_856) / 1_000_000
-SPLIT_DRAM_BYTES_PER_KEY = (6_560_256 + 512) / 1_000_000
+QUEUE_DRAM_BYTES_PER_KEY = (14_646_784 + 87_149_056) / 1_000_000
+SPLIT_DRAM_BYTES_PER_KEY = (6_621_952 + 59_392) / 1_000_000
 
 
 def _workload(args):

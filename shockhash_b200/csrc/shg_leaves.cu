@@ -125,6 +125,10 @@ __device__ __forceinline__ bool group_peel(uint32_t m, bool live, const Cells &c
         if (!__any_sync(0xffffffffu, ones != 0)) return !tree;
     }
 }
+// Words and keys per lane by the number of cells: 32 bits hold up to 31 of them, and five keys for each of the eight
+// lanes are enough up to 40. Leaf stage at 1M keys, five keys / eight: ShockHash<32> 4.86 / 4.96 ms, <40> 34.9 / 35.0, rotation
+// fitting <40> 5.82 / 5.96. (Six keys up to 48 against eight: ShockHash<44>, 50,000 keys 11.6-11.9 / 12.0-12.2 ms, <48>, 20,000 30.4-31.0 /
+// 29.7-30.3: within what runs differ by.)
 template <class Cells> __device__ __forceinline__ bool group_pseudoforest(uint32_t m, bool live, const Cells &cells) {
     if (m == 1) return live;  // its two cells are one
     if (m < 32) return group_peel<uint32_t, 4>(m, live, cells);
