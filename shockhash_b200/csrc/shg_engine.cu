@@ -278,7 +278,7 @@ struct HostSeg {
     size_t bytes;
 };
 // segs[0 .. nseg) back to back at dst; start[i]: the bytes before segment i, start[nseg] all of them.
-shg_status h2d_segments(shg_engine *e, void *dst, const HostSeg *segs, const size_t *start, size_t nseg, cudaStream_t s) {
+shg_status queue_segments(shg_engine *e, void *dst, const HostSeg *segs, const size_t *start, size_t nseg, cudaStream_t s) {
     const size_t bytes = start[nseg];
     if (!bytes) return SHG_OK;
     bool stage = nseg > 1 ? bytes >= (64u << 10) : bytes >= kStageMin;
@@ -322,6 +322,12 @@ shg_status h2d_segments(shg_engine *e, void *dst, const HostSeg *segs, const siz
     run_parts(nt, work);
     CU((cudaError_t)error.load());
     return SHG_OK;
+}
+// The same; after a failure no copy is still reading the caller's memory.
+shg_status h2d_segments(shg_engine *e, void *dst, const HostSeg *segs, const size_t *start, size_t nseg, cudaStream_t s) {
+    const shg_status st = queue_segments(e, dst, segs, start, nseg, s);
+    if (st != SHG_OK) cudaStreamSynchronize(s);
+    return st;
 }
 shg_status h2d_from_host(shg_engine *e, void *dst, const void *src, size_t bytes, cudaStream_t s) {
     const HostSeg seg{src, bytes};
@@ -1509,28 +1515,33 @@ shg_status shg_build_batch_items(shg_engine *e, const shg_params *p, const shg_b
     if (st) return st;
     CU(cudaSetDevice(e->device));
     cudaStream_t s = e->stream;
-    CU(e->first.ensure(std::max<uint64_t>(total, 1) * 8));
-    CU(e->second.ensure(std::max<uint64_t>(total, 1) * 8));
-    CU(e->in_keys.ensure(std::max<uint64_t>(nkeys, 1) * 8));
-    CU(cudaEventRecord(e->ev[7], s));
-    uint64_t off = 0, koff = 0;
-    for (uint64_t r = 0; r < nitems; r++) {
-        const shg_batch_item &it = items[r];
-        if (!it.n) continue;
-        if (it.keys) {  // uint64 keys, hashed on the device as 8-byte strings
-            CU(cudaMemcpyAsync(e->in_keys.as<uint64_t>() + koff, it.keys, it.n * 8, cudaMemcpyHostToDevice, s));
-            launch_spooky_u64(e->in_keys.as<uint64_t>() + koff, it.n, e->first.as<uint64_t>() + off,
-                              e->second.as<uint64_t>() + off, s);
-            koff += it.n;
-        } else {
-            CU(cudaMemcpyAsync(e->first.as<uint64_t>() + off, it.first, it.n * 8, cudaMemcpyHostToDevice, s));
-            CU(cudaMemcpyAsync(e->second.as<uint64_t>() + off, it.second, it.n * 8, cudaMemcpyHostToDevice, s));
+    auto queue_inputs = [&]() -> shg_status {
+        CU(e->first.ensure(std::max<uint64_t>(total, 1) * 8));
+        CU(e->second.ensure(std::max<uint64_t>(total, 1) * 8));
+        CU(e->in_keys.ensure(std::max<uint64_t>(nkeys, 1) * 8));
+        CU(cudaEventRecord(e->ev[7], s));
+        uint64_t off = 0, koff = 0;
+        for (uint64_t r = 0; r < nitems; r++) {
+            const shg_batch_item &it = items[r];
+            if (!it.n) continue;
+            if (it.keys) {  // uint64 keys, hashed on the device as 8-byte strings
+                CU(cudaMemcpyAsync(e->in_keys.as<uint64_t>() + koff, it.keys, it.n * 8, cudaMemcpyHostToDevice, s));
+                launch_spooky_u64(e->in_keys.as<uint64_t>() + koff, it.n, e->first.as<uint64_t>() + off,
+                                  e->second.as<uint64_t>() + off, s);
+                koff += it.n;
+            } else {
+                CU(cudaMemcpyAsync(e->first.as<uint64_t>() + off, it.first, it.n * 8, cudaMemcpyHostToDevice, s));
+                CU(cudaMemcpyAsync(e->second.as<uint64_t>() + off, it.second, it.n * 8, cudaMemcpyHostToDevice, s));
+            }
+            off += it.n;
         }
-        off += it.n;
-    }
-    CU(cudaGetLastError());
-    CU(cudaEventRecord(e->ev[0], s));
-    CU(cudaEventSynchronize(e->ev[0]));
+        CU(cudaGetLastError());
+        CU(cudaEventRecord(e->ev[0], s));
+        CU(cudaEventSynchronize(e->ev[0]));
+        return SHG_OK;
+    };
+    st = queue_inputs();
+    if (st) return settle(e, st);
     float ms = 0;
     cudaEventElapsedTime(&ms, e->ev[7], e->ev[0]);
     return build_batch(e, p, e->first.as<uint64_t>(), e->second.as<uint64_t>(), nr, outs, ms, specs.data());
